@@ -24,6 +24,14 @@
 //
 // All state lives in a per-warp slot of device memory; the warp's pointers
 // and scalars live in shared memory.  Each phase is one non-inlined function.
+//
+// A refinement step is a chain of dependent loads, so what bounds the kernel is
+// the latency of one warp and, for the many-warp search, how many warps' state
+// fits in shared memory.  Positions and vertices are 16-bit (n <= 65536), and a
+// cell's level is not kept (see the log of cell starts): 6.4 bytes per vertex
+// where 32-bit arrays with in_level took 16.4.  With both changes a batch of
+// mixed graphs up to 256 vertices took 430 instead of 478 ms, a 4096-vertex
+// cubic graph 85 instead of 91 ms (12 instead of 3 warps of shared memory).
 #pragma once
 #include <cstdint>
 
@@ -46,12 +54,13 @@ struct SpTc {
 // Byte layout of one slot for graphs with at most n vertices and m2 CSR
 // entries, `pool` per-level representative arrays and `cap` ring slots.
 struct SpLayout {
-  uint64_t u32n[26];  // offsets of the n-sized u32 arrays
+  uint64_t u32n[23];  // offsets of the n-sized u32 arrays
+  uint64_t elem, pos;
   uint64_t fcode, ccode, pool_owner;
   uint64_t stb, sts, act, acts, tcb, tcbs;
   uint64_t fcert, bcert, ccert;
-  uint64_t tc, reps, auts, ulog, fixst;
-  uint32_t ulog_cap, fixcap;
+  uint64_t tc, reps, auts, fixst;
+  uint32_t fixcap;
   uint64_t bytes;
   uint32_t nw, nsw;
   uint32_t stride;  // elements per representative array / ring entry
@@ -69,7 +78,9 @@ __host__ __device__ inline SpLayout sp_layout(uint32_t n, uint64_t m2, uint32_t 
   };
   const uint64_t N1 = (uint64_t)n + 2;
   L.stride = (uint32_t)N1;
-  for (int i = 0; i < 26; ++i) L.u32n[i] = take(4 * N1);
+  for (int i = 0; i < 23; ++i) L.u32n[i] = take(4 * N1);
+  L.elem = take(2 * N1);
+  L.pos = take(2 * N1);
   L.fcode = take(4 * (N1 + 1));
   L.ccode = take(4 * (N1 + 1));
   L.pool_owner = take(4 * ((uint64_t)pool + 1));
@@ -87,8 +98,6 @@ __host__ __device__ inline SpLayout sp_layout(uint32_t n, uint64_t m2, uint32_t 
   L.tc = take(sizeof(SpTc) * N1);
   L.reps = take(4ull * pool * N1);
   L.auts = take(2ull * cap * N1);
-  L.ulog_cap = 5 * n + 64;
-  L.ulog = take(8ull * L.ulog_cap);
   L.fixcap = fixcap;
   L.fixst = take(8ull * fixcap);
   L.bytes = o;
@@ -96,21 +105,22 @@ __host__ __device__ inline SpLayout sp_layout(uint32_t n, uint64_t m2, uint32_t 
 }
 
 // Shared-memory staging: the arrays every refinement step touches (elem,
-// pos, in_level, the list of non-singleton cells and the start / active /
-// touched-cell bitmaps with their summaries) live in the warp's
-// shared-memory region when they fit.
+// pos, the list of non-singleton cells and the start / active / touched-cell
+// bitmaps with their summaries) live in the warp's shared-memory region when
+// they fit.
 __host__ __device__ inline uint64_t sp_smem_bytes(uint32_t n) {
   const uint64_t nw = (n + 63) / 64 + 1, nsw = (nw + 63) / 64 + 1;
-  const uint64_t a = ((uint64_t)n + 2) * 4u;
-  return 4 * ((a + 15) & ~15ull) + 3 * 8 * (nw + nsw);
+  const uint64_t a = ((uint64_t)n + 2) * 2u;
+  return 3 * ((a + 15) & ~15ull) + 3 * 8 * (nw + nsw);
 }
 
 struct SpWarp {
-  uint32_t *elem, *pos, *inlev, *cnt, *T, *Tc, *cellcnt, *off, *fill, *G, *tmp, *lst1, *lst2;
-  uint32_t *seq, *fseq, *bseq, *flabel, *blabel, *dsu, *hist, *pre, *fpos, *bpos, *nsl;
+  uint16_t *elem, *pos;  // position -> vertex, vertex -> position (n <= 65536)
+  uint32_t *slog, *cnt, *T, *Tc, *cellcnt, *off, *fill, *G, *tmp, *lst1, *lst2;
+  uint32_t *seq, *fseq, *bseq, *flabel, *blabel, *dsu, *hist, *pre, *fpos;
+  uint16_t* nsl;
   int32_t *fcode, *ccode, *pool_owner, *pathcode;
-  uint32_t *umark;  // per level: undo-log size when the level's child was made
-  uint2* ulog;      // undo log: {position | kStartFlag, previous in_level}
+  uint32_t *umark;  // per level: start-log size when the level's child was made
   uint2* fixst;     // per stored automorphism: {prefix of seq it fixes, first
                     // position of seq it moves or kNone}, valid for the path
   uint64_t *stb, *sts, *act, *acts, *tcb, *tcbs;
@@ -122,7 +132,7 @@ struct SpWarp {
   uint32_t n, nw, nsw, stride;  // stride: elements per pool / ring entry
   uint32_t ncells, nact, ntouched, nl1, nl2, npend;
   uint32_t pool_top, pool_cap, aut_cap, max_aut;
-  uint32_t utop, ulog_cap, ulog_bad;
+  uint32_t utop;  // entries of slog
   uint32_t fixcap;  // store entries whose fix state is kept (later ones are checked in full)
   // values the serial fold hands to the whole warp
   uint32_t lc, hint;
@@ -218,26 +228,21 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
   return m;
 }
 
-// ---- undo log of the partition's cell structure ----------------------------
-// Every change of a cell start or an in_level after the root refinement is
-// logged (by lane 0, in order), so backtracking undoes exactly the changes
-// made below the target level instead of rescanning the whole partition.
-// Vertex order inside cells is not restored: only cells as sets matter.
-constexpr uint32_t kStartFlag = 0x80000000u;
+// ---- log of the cell starts --------------------------------------------------
+// Every cell start made after the root refinement is logged in order of
+// creation, and umark[L] is the log's size when the node of level L got its
+// child, so a backtrack to level L clears exactly the starts logged from
+// there on.  That is reconstruct_at_level (partition_refinement.cpp:541-604):
+// it merges every maximal run of cells created below L with the cell that
+// follows it, and a split gives every fragment but the last the new level, so
+// the starts that survive are those made at or above L.  The in_level of a
+// cell has no other use.  A cell start is made once between two backtracks
+// past it, so the log holds at most n entries.  Vertex order inside cells is
+// not restored: only cells as sets matter.
 
-__device__ __forceinline__ void ulog_push(SpWarp& W, uint32_t x, uint32_t old) {
-  if (W.utop < W.ulog_cap)
-    W.ulog[W.utop++] = make_uint2(x, old);
-  else
-    W.ulog_bad = 1;  // full: backtracks rescan the partition
-}
-// lane 0: in_level write / new cell start, logged
-__device__ __forceinline__ void set_inlev(SpWarp& W, uint32_t p, uint32_t v) {
-  ulog_push(W, p, W.inlev[p]);
-  W.inlev[p] = v;
-}
+// lane 0: new cell start, logged
 __device__ __forceinline__ void add_start(SpWarp& W, uint32_t p) {
-  ulog_push(W, p | kStartFlag, 0u);
+  W.slog[W.utop++] = p;
   bm_set1(W.stb, W.sts, p);
 }
 
@@ -343,13 +348,12 @@ __device__ __noinline__ uint32_t sp_list_nonsingleton() {
 // fragment order; order inside a fragment is immaterial).  The hash then
 // folds every non-singleton cell in position order -- an untouched one
 // contributes its start, a touched one its fragments -- and lane 0 does the
-// bookkeeping of the splits (starts, in_level, active set, hint) in the same
-// order.  Nothing goes through the per-step scratch arrays of the general
+// bookkeeping of the splits (starts, active set, hint) in the same order.  Nothing goes through the per-step scratch arrays of the general
 // path.  Returns false, having changed nothing, when the splitter is too
 // large; `lc` and `hint` are the refinement's running hash and hint.
 // ---------------------------------------------------------------------------
-__device__ __noinline__ bool sp_refine_small(uint32_t s, uint32_t len, uint32_t lvl1,
-                                             uint32_t* lc_io, uint32_t* hint_io) {
+__device__ __noinline__ bool sp_refine_small(uint32_t s, uint32_t len, uint32_t* lc_io,
+                                             uint32_t* hint_io) {
   SpWarp& W = sp_w();
   const uint32_t lane = lane_id();
   if (len > 32) return false;
@@ -470,12 +474,10 @@ __device__ __noinline__ bool sp_refine_small(uint32_t s, uint32_t len, uint32_t 
       const uint32_t Lc = __shfl_sync(GCL_FULL, L, (int)src);
       const uint32_t kc = __shfl_sync(GCL_FULL, k, (int)src);
       const bool was = bm_test(W.act, cc);
-      const uint32_t oldlev = W.inlev[cc];
       __syncwarp();
-      uint32_t maxsz = 0, maxf = cc, lastf = cc;
+      uint32_t maxsz = 0, maxf = cc;
       if (Lc > kc) {  // the untouched fragment first
         lc = mash(lc, 0u + cc);
-        if (lane == 0) set_inlev(W, cc, lvl1);
         maxsz = Lc - kc;
       }
       // the touched fragments in ascending count (= ascending start)
@@ -490,34 +492,27 @@ __device__ __noinline__ bool sp_refine_small(uint32_t s, uint32_t len, uint32_t 
           pend |= 1u << s2;
           if (sz == 1) hint = fm;
         }
-        if (lane == 0) {
-          set_inlev(W, fm, lvl1);
-          if (fm != cc) {
-            W.ncells += 1;
-            if (!bm_test(W.act, fm)) {
-              bm_set1(W.act, W.acts, fm);
-              W.nact += 1;
-            }
+        if (lane == 0 && fm != cc) {
+          W.ncells += 1;
+          if (!bm_test(W.act, fm)) {
+            bm_set1(W.act, W.acts, fm);
+            W.nact += 1;
           }
         }
         if (sz > maxsz) {
           maxsz = sz;
           maxf = fm;
         }
-        lastf = fm;
       }
-      if (lane == 0) {
-        if (!was) {
-          if (!bm_test(W.act, cc)) {
-            bm_set1(W.act, W.acts, cc);
-            W.nact += 1;
-          }
-          if (bm_test(W.act, maxf)) {
-            bm_clear1(W.act, W.acts, maxf);
-            W.nact -= 1;
-          }
+      if (lane == 0 && !was) {
+        if (!bm_test(W.act, cc)) {
+          bm_set1(W.act, W.acts, cc);
+          W.nact += 1;
         }
-        set_inlev(W, lastf, oldlev);
+        if (bm_test(W.act, maxf)) {
+          bm_clear1(W.act, W.acts, maxf);
+          W.nact -= 1;
+        }
       }
       __syncwarp();
     }
@@ -544,28 +539,25 @@ __device__ __noinline__ bool sp_refine_small(uint32_t s, uint32_t len, uint32_t 
 // bitmap holds the initially active cells; returns the code (-1 on a failed
 // consistency check).  The caller increments the level.
 // ---------------------------------------------------------------------------
-__device__ __noinline__ int sp_refine(uint32_t level) {
+__device__ __noinline__ int sp_refine() {
   SpWarp& W = sp_w();
   const uint32_t lane = lane_id();
   const uint32_t n = W.n, nw = W.nw, nsw = W.nsw;
-  const uint32_t lvl1 = level + 1;
   uint32_t lc = W.ncells, hint = 0;
   uint64_t iters = 0;
   int ok = 1;
   // the arrays a step touches, in registers for the whole refinement (the
   // warp record's pointers would otherwise be reloaded after every store)
-  uint32_t* const elem = W.elem;
-  uint32_t* const pos = W.pos;
+  uint16_t* const elem = W.elem;
+  uint16_t* const pos = W.pos;
   uint64_t* const stb = W.stb;
   uint64_t* const sts = W.sts;
   uint64_t* const act = W.act;
   uint64_t* const acts = W.acts;
   const int32_t* const rp = W.rp;
   const int32_t* const col = W.col;
-  uint32_t* const inlev = W.inlev;
-  uint2* const ulog = W.ulog;
-  const uint32_t ucap = W.ulog_cap;
-  // the cell and active counts and the undo log's top, kept by every lane
+  uint32_t* const slog = W.slog;
+  // the cell and active counts and the start log's top, kept by every lane
   // alike during the singleton steps; the warp record holds them while the
   // other paths run (they update them there) and after the refinement
   uint32_t ncells = W.ncells, nact = W.nact, utop = W.utop;
@@ -644,7 +636,7 @@ __device__ __noinline__ int sp_refine(uint32_t level) {
         elem[p] = x;
         pos[x] = p;
       }
-      // split cells in position order: hash, in_level, starts, active set;
+      // split cells in position order: hash, starts, active set;
       // hint and hash are the same on every lane, lane 0 writes
       uint32_t leaders = __ballot_sync(GCL_FULL, lead);
       while (leaders) {
@@ -665,22 +657,11 @@ __device__ __noinline__ int sp_refine(uint32_t level) {
           if (nb == 1) hint = cmin;
         }
         if (lane == 0) {
-          // in_level of both fragments and the new start, logged in the
-          // order set_inlev / add_start would log them
-          const uint32_t oldc = inlev[cmin], oldp = inlev[pp];
-          if (utop + 3 <= ucap) {
-            ulog[utop] = make_uint2(pp, oldp);
-            ulog[utop + 1] = make_uint2(cmin, oldc);
-            ulog[utop + 2] = make_uint2(pp | kStartFlag, 0u);
-          } else {
-            W.ulog_bad = 1;  // full: backtracks rescan the partition
-          }
-          inlev[pp] = oldc;
-          inlev[cmin] = lvl1;
+          slog[utop] = pp;
           bm_set1(stb, sts, pp);
           bm_set1(act, acts, to_rest ? pp : cmin);
         }
-        if (utop + 3 <= ucap) utop += 3;
+        utop += 1;
         ncells += 1;
         nact += 1;
       }
@@ -697,7 +678,7 @@ __device__ __noinline__ int sp_refine(uint32_t level) {
     __syncwarp();
 
     // a small non-singleton splitter: warp-synchronous, no scratch arrays
-    if (len > 1 && sp_refine_small(s, len, lvl1, &lc, &hint)) {
+    if (len > 1 && sp_refine_small(s, len, &lc, &hint)) {
       ncells = W.ncells;
       nact = W.nact;
       utop = W.utop;
@@ -770,8 +751,6 @@ __device__ __noinline__ int sp_refine(uint32_t level) {
           lc = mash(lc, p - 1);
           const bool was = bm_test(W.act, c);
           if (lane == 0) {
-            set_inlev(W, p, W.inlev[c]);
-            set_inlev(W, c, lvl1);
             add_start(W, p);
             W.ncells += 1;
             const uint32_t nb = k, nn = L - k;
@@ -850,24 +829,20 @@ __device__ __noinline__ int sp_refine(uint32_t level) {
           __syncwarp();
           const uint32_t r0 = c + (L - k);
           sp_regroup(seg, k, r0, W.tmp);
-          // fragments: hash, starts, in_level, active (:326-465)
+          // fragments: hash, starts, active (:326-465)
           const bool was = bm_test(W.act, c);
-          const uint32_t oldlev = W.inlev[c];
           __syncwarp();
           if (lane == 0) {
-            uint32_t maxsz = 0, maxf = c, lastf = c, nfr = 0;
+            uint32_t maxsz = 0, maxf = c;
             if (L > k) {  // untouched fragment first
               lc = mash(lc, 0u + c);
-              set_inlev(W, c, lvl1);
               maxsz = L - k;
-              nfr = 1;
             }
             uint32_t f = r0;
             for (uint32_t i = 0; i < range; ++i) {
               const uint32_t sz = W.hist[i];
               if (!sz) continue;
               lc = mash(lc, mn + i + f);
-              set_inlev(W, f, lvl1);
               if (f != c) {
                 W.fpos[W.npend++] = f;  // set after the fold: the fold walks the old starts
                 W.ncells += 1;
@@ -881,9 +856,7 @@ __device__ __noinline__ int sp_refine(uint32_t level) {
                 maxsz = sz;
                 maxf = f;
               }
-              lastf = f;
               f += sz;
-              ++nfr;
             }
             if (!was) {
               if (!bm_test(W.act, c)) {
@@ -895,7 +868,6 @@ __device__ __noinline__ int sp_refine(uint32_t level) {
                 W.nact -= 1;
               }
             }
-            set_inlev(W, lastf, oldlev);
             W.lc = lc;
             W.hint = hint;
           }
@@ -956,8 +928,6 @@ __device__ __forceinline__ bool sp_individualize(uint32_t level, uint32_t v, uin
     W.pos[v] = t;
     add_start(W, t + 1);
     W.ncells += 1;
-    set_inlev(W, t + 1, W.inlev[t]);
-    set_inlev(W, t, level + 1);
     bm_set1(W.act, W.acts, t);
     W.nact = 1;
   }
@@ -965,189 +935,27 @@ __device__ __forceinline__ bool sp_individualize(uint32_t level, uint32_t v, uin
   return true;
 }
 
-// reconstruct_at_level (partition_refinement.cpp:541-604): a start survives
-// unless the cell before it was created after level Lv; a surviving start
-// whose own cell is that new takes the in_level of the first following cell
-// created at or before Lv.  Each lane handles a contiguous range of words;
-// prefix max / suffix min scans carry the neighbouring starts across lanes.
-__device__ __noinline__ bool sp_backtrack(uint32_t Lv) {
+// Backtrack to node level Lv (reconstruct_at_level,
+// partition_refinement.cpp:541-604): the starts logged since that node's child
+// was made go.  False if the log is inconsistent.
+__device__ __forceinline__ bool sp_backtrack(uint32_t Lv) {
   SpWarp& W = sp_w();
   const uint32_t lane = lane_id();
-  const uint32_t n = W.n, nw = (n + 63) / 64;
-  const uint32_t per = (nw + 31) / 32;
-  const uint32_t w0 = min(nw, lane * per), w1 = min(nw, w0 + per);
-  // chunk summary: last start (and whether it is "big"), first non-big start
-  uint32_t last = kNone, firstsmall = kNone;
-  bool lastbig = false;
-  for (uint32_t w = w0; w < w1; ++w) {
-    uint64_t b = W.stb[w];
-    while (b) {
-      const uint32_t p = w * 64 + ctz64(b);
-      b &= b - 1;
-      const bool big = W.inlev[p] > Lv;
-      last = p;
-      lastbig = big;
-      if (!big && firstsmall == kNone) firstsmall = p;
-    }
-  }
-  // previous start before this chunk: max over lower lanes of `last`
-  uint32_t prev_last = kNone;
-  bool prev_big = false;
-  {
-    // encode (position+1) so kNone sorts lowest
-    uint32_t key = last == kNone ? 0u : last + 1;
-    uint32_t bigbit = lastbig ? 1u : 0u;
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t k2 = __shfl_up_sync(GCL_FULL, key, o);
-      const uint32_t b2 = __shfl_up_sync(GCL_FULL, bigbit, o);
-      if (lane >= (uint32_t)o && k2 > key) {
-        key = k2;
-        bigbit = b2;
-      }
-    }
-    // exclusive: take the inclusive value of lane-1
-    const uint32_t kx = __shfl_up_sync(GCL_FULL, key, 1);
-    const uint32_t bx = __shfl_up_sync(GCL_FULL, bigbit, 1);
-    if (lane > 0 && kx) {
-      prev_last = kx - 1;
-      prev_big = bx != 0;
-    }
-  }
-  // first non-big start after this chunk: min over higher lanes
-  uint32_t next_small = kNone;
-  {
-    uint32_t key = firstsmall;
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t k2 = __shfl_down_sync(GCL_FULL, key, o);
-      if (lane + (uint32_t)o < 32 && k2 < key) key = k2;
-    }
-    const uint32_t kx = __shfl_down_sync(GCL_FULL, key, 1);
-    if (lane < 31) next_small = kx;
-  }
-  // decide survivors and new in_levels; remember the writes
-  bool bad = false;
-  __syncwarp();
-  {
-    bool pbig = prev_big;
-    const bool have_prev = prev_last != kNone;
-    bool first_in_chunk = true;
-    // the new in_level of a surviving big start: first non-big start after it
-    for (uint32_t w = w0; w < w1; ++w) {
-      uint64_t b = W.stb[w];
-      uint64_t keep = b;
-      uint64_t bb = b;
-      while (bb) {
-        const uint32_t p = w * 64 + ctz64(bb);
-        bb &= bb - 1;
-        const bool big = W.inlev[p] > Lv;
-        const bool has_prev = !first_in_chunk || have_prev;
-        const bool survive = !(has_prev && pbig);
-        if (!survive) keep &= ~bit64(p & 63);
-        if (survive && big) {
-          // closing cell: next non-big start after p
-          uint32_t j = kNone;
-          uint64_t rest = bb;
-          uint32_t ww = w;
-          while (true) {
-            while (rest) {
-              const uint32_t q = ww * 64 + ctz64(rest);
-              rest &= rest - 1;
-              if (W.inlev[q] <= Lv) {
-                j = q;
-                break;
-              }
-            }
-            if (j != kNone) break;
-            if (++ww >= w1) break;
-            rest = W.stb[ww];
-          }
-          if (j == kNone) j = next_small;
-          if (j == kNone) {
-            bad = true;
-          } else {
-            W.tmp[p] = W.inlev[j];  // staged new in_level
-          }
-        }
-        pbig = big;
-        first_in_chunk = false;
-      }
-      W.lst1[w] = (uint32_t)keep;          // staged word (low half)
-      W.lst2[w] = (uint32_t)(keep >> 32);  // staged word (high half)
-    }
-  }
-  if (__any_sync(GCL_FULL, bad)) return false;
-  __syncwarp();
-  // apply: in_levels of surviving big starts, then the start words
-  uint32_t removed = 0;
-  for (uint32_t w = w0; w < w1; ++w) {
-    const uint64_t old = W.stb[w];
-    const uint64_t keep = ((uint64_t)W.lst2[w] << 32) | W.lst1[w];
-    uint64_t sb = keep;
-    while (sb) {
-      const uint32_t p = w * 64 + ctz64(sb);
-      sb &= sb - 1;
-      if (W.inlev[p] > Lv) W.inlev[p] = W.tmp[p];
-    }
-    removed += popc64(old) - popc64(keep);
-    W.stb[w] = keep;
-  }
-  removed = __reduce_add_sync(GCL_FULL, removed);
-  __syncwarp();
-  bm_resummarize(W.stb, W.sts, nw, W.nsw);
-  if (lane == 0) W.ncells -= removed;
-  __syncwarp();
-  return true;
-}
-
-// Backtrack to node level Lv by undoing the logged changes made since that
-// node's child was created: the same cells as reconstruct_at_level.  Every
-// start created below Lv is cleared, and every in_level changed below Lv
-// returns to the value before its first change (entries are processed in
-// parallel: per position the earliest entry wins).
-__device__ __forceinline__ bool sp_backtrack_log(uint32_t Lv) {
-  SpWarp& W = sp_w();
-  const uint32_t lane = lane_id();
-  if (W.ulog_bad) {
-    const bool ok = sp_backtrack(Lv);
-    __syncwarp();
-    return ok;
-  }
   const uint32_t lo = W.umark[Lv], hi = W.utop;
   if (lo > hi) return false;
   for (uint32_t i = lo + lane; i < hi; i += 32) {
-    const uint2 e = W.ulog[i];
-    if (!(e.x & kStartFlag)) W.tmp[e.x] = 0xffffffffu;
+    const uint32_t p = W.slog[i];
+    atomicAnd((unsigned long long*)&W.stb[p >> 6], (unsigned long long)~bit64(p & 63));
   }
   __syncwarp();
   for (uint32_t i = lo + lane; i < hi; i += 32) {
-    const uint2 e = W.ulog[i];
-    if (!(e.x & kStartFlag)) atomicMin(&W.tmp[e.x], i);
+    const uint32_t w = W.slog[i] >> 6;
+    if (W.stb[w] == 0)
+      atomicAnd((unsigned long long*)&W.sts[w >> 6], (unsigned long long)~bit64(w & 63));
   }
-  __syncwarp();
-  uint32_t removed = 0;
-  for (uint32_t i = lo + lane; i < hi; i += 32) {
-    const uint2 e = W.ulog[i];
-    if (e.x & kStartFlag) {
-      const uint32_t p = e.x & ~kStartFlag;
-      atomicAnd((unsigned long long*)&W.stb[p >> 6], (unsigned long long)~bit64(p & 63));
-      ++removed;
-    } else if (W.tmp[e.x] == i) {
-      W.inlev[e.x] = e.y;
-    }
-  }
-  __syncwarp();
-  for (uint32_t i = lo + lane; i < hi; i += 32) {
-    const uint2 e = W.ulog[i];
-    if (e.x & kStartFlag) {
-      const uint32_t w = (e.x & ~kStartFlag) >> 6;
-      if (W.stb[w] == 0)
-        atomicAnd((unsigned long long*)&W.sts[w >> 6], (unsigned long long)~bit64(w & 63));
-    }
-  }
-  removed = __reduce_add_sync(GCL_FULL, removed);
   __syncwarp();
   if (lane == 0) {
-    W.ncells -= removed;
+    W.ncells -= hi - lo;
     W.utop = lo;
   }
   __syncwarp();
@@ -1224,7 +1032,8 @@ __device__ __forceinline__ int sp_cmp_leaf(const uint32_t* cur, const uint32_t* 
   return 0;
 }
 
-__device__ __forceinline__ void sp_copy_u32(uint32_t* dst, const uint32_t* src, uint32_t k) {
+template <typename T>
+__device__ __forceinline__ void sp_copy_u32(uint32_t* dst, const T* src, uint32_t k) {
   const uint32_t lane = lane_id();
   for (uint32_t i = lane; i < k; i += 32) dst[i] = src[i];
   __syncwarp();
@@ -1298,8 +1107,8 @@ __device__ __forceinline__ uint32_t sp_find(volatile uint32_t* d, uint32_t x, ui
 // one, then shortcut every member to its root, until a round changes
 // nothing (compute_orbits_fast's DSU, perm_group.cpp:60-116).  pm must map
 // the member set onto itself.  False if the rounds do not converge.
-template <bool kCg>
-__device__ __forceinline__ bool sp_dsu_apply(const uint16_t* pm, const uint32_t* members,
+template <bool kCg, typename T>
+__device__ __forceinline__ bool sp_dsu_apply(const uint16_t* pm, const T* members,
                                           uint32_t count, uint32_t n) {
   SpWarp& W = sp_w();
   const uint32_t lane = lane_id();
@@ -1343,7 +1152,7 @@ __device__ __forceinline__ bool sp_orbits(int idx, int num_aut, uint32_t seqlen)
   const int from = t.last == -1 ? 0 : t.last;
   volatile uint32_t* dsu = W.dsu;
   const uint32_t* reps = t.rslot >= 0 ? W.reps + (uint64_t)t.rslot * W.stride : nullptr;
-  const uint32_t* mem = W.elem + t.first;
+  const uint16_t* mem = W.elem + t.first;
   for (uint32_t i = lane; i < t.len; i += 32) {
     const uint32_t v = mem[i];
     dsu[v] = reps ? reps[v] : v;
@@ -1464,14 +1273,17 @@ __device__ __noinline__ void sp_init_partition(const int32_t* color) {
   SpWarp& W = sp_w();
   const uint32_t lane = lane_id();
   const uint32_t n = W.n;
-  for (uint32_t i = lane; i < n; i += 32) W.elem[i] = i;
+  for (uint32_t i = lane; i < n; i += 32) {
+    W.elem[i] = (uint16_t)i;
+    W.lst1[i] = i;
+  }
   __syncwarp();
   bool colored = false;
   if (color)
     for (uint32_t i = lane; i < n; i += 32) colored |= color[i] != 0;
   colored = __any_sync(GCL_FULL, colored);
   if (colored) {
-    uint32_t* a = W.elem;
+    uint32_t* a = W.lst1;
     uint32_t* b = W.tmp;
     for (int pass = 0; pass < 4; ++pass) {
       const int sh = pass * 8;
@@ -1501,7 +1313,9 @@ __device__ __noinline__ void sp_init_partition(const int32_t* color) {
       a = b;
       b = t;
     }
-    // four passes: the result is back in elem
+    // four passes: the result is back in lst1
+    for (uint32_t i = lane; i < n; i += 32) W.elem[i] = (uint16_t)W.lst1[i];
+    __syncwarp();
   }
   for (uint32_t i = lane; i < n; i += 32) W.pos[W.elem[i]] = i;
   for (uint32_t w = lane; w < W.nw; w += 32) {
@@ -1513,7 +1327,6 @@ __device__ __noinline__ void sp_init_partition(const int32_t* color) {
     W.cnt[i] = 0;
     W.cellcnt[i] = 0;
     W.fill[i] = 0;
-    W.inlev[i] = 0;
   }
   __syncwarp();
   // cell starts where the colour changes
@@ -1614,12 +1427,14 @@ __device__ __noinline__ void sp_bind(uint8_t* slot, const SpLayout& Lo, uint32_t
                                      uint32_t max_aut) {
   SpWarp& W = sp_w();
   if (lane_id() != 0) return;
+  W.elem = (uint16_t*)(slot + Lo.elem);
+  W.pos = (uint16_t*)(slot + Lo.pos);
   // the n-sized u32 arrays
-  uint32_t* base[26];
-  for (int i = 0; i < 26; ++i) base[i] = (uint32_t*)(slot + Lo.u32n[i]);
-  W.elem = base[0];
-  W.pos = base[1];
-  W.inlev = base[2];
+  uint32_t* base[23];
+  for (int i = 0; i < 23; ++i) base[i] = (uint32_t*)(slot + Lo.u32n[i]);
+  W.slog = base[0];
+  W.umark = base[1];
+  W.nsl = (uint16_t*)base[2];
   W.cnt = base[3];
   W.T = base[4];
   W.Tc = base[5];
@@ -1639,16 +1454,10 @@ __device__ __noinline__ void sp_bind(uint8_t* slot, const SpLayout& Lo, uint32_t
   W.hist = base[19];
   W.pre = base[20];
   W.fpos = base[21];
-  W.bpos = base[22];
-  W.nsl = base[23];
-  W.pathcode = (int32_t*)base[24];
-  W.umark = base[25];
-  W.ulog = (uint2*)(slot + Lo.ulog);
+  W.pathcode = (int32_t*)base[22];
   W.fixst = (uint2*)(slot + Lo.fixst);
   W.fixcap = Lo.fixcap;
-  W.ulog_cap = Lo.ulog_cap;
   W.utop = 0;
-  W.ulog_bad = 0;
   W.fcode = (int32_t*)(slot + Lo.fcode);
   W.ccode = (int32_t*)(slot + Lo.ccode);
   W.pool_owner = (int32_t*)(slot + Lo.pool_owner);
@@ -1673,16 +1482,14 @@ __device__ __noinline__ void sp_bind(uint8_t* slot, const SpLayout& Lo, uint32_t
   W.npend = 0;
   if (smem && sp_smem_bytes(n) <= smem_bytes) {
     // stage the per-step arrays in this warp's shared memory
-    const uint64_t a = (((uint64_t)n + 2) * 4u + 15) & ~15ull;
+    const uint64_t a = (((uint64_t)n + 2) * 2u + 15) & ~15ull;
     const uint32_t nw2 = W.nw, nsw2 = W.nsw;
     uint8_t* q = smem;
-    W.elem = (uint32_t*)q;
+    W.elem = (uint16_t*)q;
     q += a;
-    W.pos = (uint32_t*)q;
+    W.pos = (uint16_t*)q;
     q += a;
-    W.inlev = (uint32_t*)q;
-    q += a;
-    W.nsl = (uint32_t*)q;
+    W.nsl = (uint16_t*)q;
     q += a;
     W.stb = (uint64_t*)q;
     q += 8 * nw2;
@@ -1735,7 +1542,7 @@ __device__ __noinline__ SpResult sp_search(const BatchArgs& A, int g, uint8_t* s
   while (true) {
     if (pending) {
       pending = false;
-      code = sp_refine(level);
+      code = sp_refine();
       if (code < 0) {
         status = kInternal;
         break;
@@ -1862,7 +1669,7 @@ __device__ __noinline__ SpResult sp_search(const BatchArgs& A, int g, uint8_t* s
             pending = true;
             continue;
           }
-          code = sp_refine(level);
+          code = sp_refine();
           if (code < 0) {
             status = kInternal;
             break;
@@ -1946,7 +1753,7 @@ __device__ __noinline__ SpResult sp_search(const BatchArgs& A, int g, uint8_t* s
         level = 0;
         continue;
       }
-      if (!sp_backtrack_log(Lv)) {
+      if (!sp_backtrack(Lv)) {
         status = kInternal;
         break;
       }

@@ -11,9 +11,9 @@
 //   2. the siblings of the first path -- every member of every level's target
 //      cell except the first-path vertex -- become work items, deepest level
 //      first.  A persistent grid of warps takes items from an atomic counter;
-//      a warp rebuilds the item's parent node by backtracking a copy of the
-//      first leaf's partition (cells never move vertices across their
-//      boundaries, so reconstruct_at_level gives the node back), drops the
+//      a warp rebuilds the item's parent node from the first leaf's vertex
+//      order and the cell starts made at or above its level (later splits
+//      never move vertices across a cell's boundary), drops the
 //      item if the vertex is not the least of its orbit under the stored
 //      automorphisms that fix the path prefix, and otherwise runs the
 //      reference's DFS (other_path_node / classify_node, sequential.cpp:304-624)
@@ -271,7 +271,10 @@ __global__ void __launch_bounds__(32) wide_first_kernel(WideArgs A) {
     return;
   }
   sp_init_partition(A.color);
-  int code = sp_refine(0);
+  // level of the node whose refinement (or individualization) made each
+  // position a cell start; the root's are level 1
+  for (uint32_t i = lane; i < n; i += 32) P.linlev[i] = 1;
+  int code = sp_refine();
   if (code < 0) {
     wide_fail(H, kInternal);
     return;
@@ -303,13 +306,15 @@ __global__ void __launch_bounds__(32) wide_first_kernel(WideArgs A) {
       wide_fail(H, kInternal);
       return;
     }
-    code = sp_refine(level);
+    code = sp_refine();
     if (code < 0) {
       wide_fail(H, kInternal);
       return;
     }
     ++level;
     __syncwarp();
+    for (uint32_t i = W.umark[level - 1] + lane; i < W.utop; i += 32)
+      P.linlev[W.slog[i]] = level;
     if (lane == 0) P.fcode[level - 1] = code;
     __syncwarp();
   }
@@ -321,7 +326,6 @@ __global__ void __launch_bounds__(32) wide_first_kernel(WideArgs A) {
     P.flabel[i] = e;
     P.blabel[i] = e;
     P.lelem[i] = e;
-    P.linlev[i] = W.inlev[i];
   }
   for (uint32_t i = lane; i < seqlen; i += 32) {
     P.fseq[i] = W.seq[i];
@@ -877,8 +881,36 @@ __device__ __noinline__ int32_t wide_take_gift(const WidePtrs& P, uint64_t deadl
   return st;
 }
 
-// Rebuild the parent node of a handed-over subtree: the first leaf taken back
-// to the level its sequence shares with the first path, the rest of its
+// The first path's node of level L: the first leaf's vertex order with the
+// cell starts made at levels up to L (reconstruct_at_level,
+// partition_refinement.cpp:541-604; see the log of cell starts).
+__device__ __noinline__ void wide_load_node(const WidePtrs& P, uint32_t L) {
+  SpWarp& W = sp_w();
+  const uint32_t lane = lane_id();
+  const uint32_t n = W.n;
+  for (uint32_t i = lane; i < n; i += 32) {
+    const uint32_t x = P.lelem[i];
+    W.elem[i] = x;
+    W.pos[x] = i;
+  }
+  uint32_t cells = 0;
+  for (uint32_t w = 0; w < W.nw; ++w) {
+    const uint32_t p0 = w * 64 + lane, p1 = p0 + 32;
+    const uint64_t b = P.lstb[w] & ballot2(p0 < n && P.linlev[p0] <= L, p1 < n && P.linlev[p1] <= L);
+    if (lane == 0) W.stb[w] = b;
+    cells += popc64(b);
+  }
+  __syncwarp();
+  bm_resummarize(W.stb, W.sts, W.nw, W.nsw);
+  if (lane == 0) {
+    W.ncells = cells;
+    W.utop = 0;
+  }
+  __syncwarp();
+}
+
+// Rebuild the parent node of a handed-over subtree: the first path's node at
+// the level its sequence shares with the first path, the rest of its
 // vertices individualized and refined (each code checked against the one the
 // giver saw).  Leaves W at the parent (level L = *k + 1) with W.seq, W.pathcode
 // and the target-cell headers of the replayed levels; *tf, *tl: the parent's
@@ -903,18 +935,7 @@ __device__ __noinline__ int32_t wide_gift_node(const WidePtrs& P, const WideArgs
       break;
     }
   }
-  for (uint32_t i = lane; i < n; i += 32) {
-    const uint32_t x = P.lelem[i];
-    W.elem[i] = x;
-    W.pos[x] = i;
-    W.inlev[i] = P.linlev[i];
-  }
-  for (uint32_t w = lane; w < W.nw; w += 32) W.stb[w] = P.lstb[w];
-  __syncwarp();
-  bm_resummarize(W.stb, W.sts, W.nw, W.nsw);
-  if (lane == 0) W.ncells = n;
-  __syncwarp();
-  if (!sp_backtrack(c + 1)) return kInternal;
+  wide_load_node(P, c + 1);
   for (uint32_t i = lane; i < c; i += 32) W.seq[i] = P.fseq[i];
   for (uint32_t i = lane; i <= c; i += 32) W.pathcode[i] = P.fcode[i];
   __syncwarp();
@@ -938,7 +959,7 @@ __device__ __noinline__ int32_t wide_gift_node(const WidePtrs& P, const WideArgs
     }
     __syncwarp();
     if (!sp_individualize(lvl, u, t)) return kInternal;
-    const int code = sp_refine(lvl);
+    const int code = sp_refine();
     if (code < 0 || (uint32_t)code != __ldcg(e + 2 + np + lvl)) return kInternal;
     __syncwarp();
     if (lane == 0) W.pathcode[lvl] = code;
@@ -1148,38 +1169,19 @@ __global__ void __launch_bounds__(kSpThreads) wide_items_kernel(WideArgs A) {
     do {
     if (skip) break;
     if (!gift) {
-      // the parent node: the first leaf backtracked to level k+1
-      for (uint32_t i = lane; i < n; i += 32) {
-        const uint32_t e = P.lelem[i];
-        W.elem[i] = e;
-        W.pos[e] = i;
-        W.inlev[i] = P.linlev[i];
-      }
-      for (uint32_t w = lane; w < W.nw; w += 32) W.stb[w] = P.lstb[w];
-      __syncwarp();
-      bm_resummarize(W.stb, W.sts, W.nw, W.nsw);
-      if (lane == 0) W.ncells = n;
-      __syncwarp();
-      if (!sp_backtrack(k + 1) || sp_cell_end(W, tf) - tf != tl) {
+      // the parent node, at level k+1
+      wide_load_node(P, k + 1);
+      if (sp_cell_end(W, tf) - tf != tl) {
         status = kInternal;
         break;
       }
-      __syncwarp();
-      if (lane == 0) {  // the item's DFS logs its changes from here
-        W.utop = 0;
-        W.ulog_bad = 0;
-      }
-      __syncwarp();
       for (uint32_t i = lane; i < k; i += 32) W.seq[i] = P.fseq[i];
       for (uint32_t i = lane; i <= k; i += 32) W.pathcode[i] = P.fcode[i];
       __syncwarp();
-    } else {
-      if (lane == 0) {  // the subtree's DFS logs its changes from here
-        W.utop = 0;
-        W.ulog_bad = 0;
-      }
-      __syncwarp();
     }
+    __syncwarp();
+    if (lane == 0) W.utop = 0;  // the subtree's DFS logs its cell starts from here
+    __syncwarp();
     // the previous item's sequence shares the first path's first
     // min(k, prev_k) vertices with this one (a handed-over subtree's
     // sequence may share none)
@@ -1218,7 +1220,7 @@ __global__ void __launch_bounds__(kSpThreads) wide_items_kernel(WideArgs A) {
       status = kInternal;
       break;
     }
-    int code = sp_refine(level);
+    int code = sp_refine();
     cnt.add(kCntRefineCycles, cnt.now() - tr);
     if (code < 0) {
       status = kInternal;
@@ -1398,7 +1400,7 @@ __global__ void __launch_bounds__(kSpThreads) wide_items_kernel(WideArgs A) {
                 status = kInternal;
                 break;
               }
-              code = sp_refine(level);
+              code = sp_refine();
               cnt.add(kCntRefineCycles, cnt.now() - tr);
               if (code < 0) {
                 status = kInternal;
@@ -1417,7 +1419,7 @@ __global__ void __launch_bounds__(kSpThreads) wide_items_kernel(WideArgs A) {
       if (bt >= 0) {
         const uint32_t Lv = (uint32_t)bt;
         if (Lv <= k + 1) break;  // the item's subtree is done
-        if (!sp_backtrack_log(Lv)) {
+        if (!sp_backtrack(Lv)) {
           status = kInternal;
           break;
         }
