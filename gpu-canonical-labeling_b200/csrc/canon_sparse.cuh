@@ -54,10 +54,10 @@ struct SpTc {
 // Byte layout of one slot for graphs with at most n vertices and m2 CSR
 // entries, `pool` per-level representative arrays and `cap` ring slots.
 struct SpLayout {
-  uint64_t u32n[23];  // offsets of the n-sized u32 arrays
-  uint64_t elem, pos;
+  uint64_t u32n[13];  // offsets of the n-sized u32 arrays
+  uint64_t elem, pos, cnt;
   uint64_t fcode, ccode, pool_owner;
-  uint64_t stb, sts, act, acts, tcb, tcbs;
+  uint64_t stb, sts, act, acts, itm, nsb;
   uint64_t fcert, bcert, ccert;
   uint64_t tc, reps, auts, fixst;
   uint32_t fixcap;
@@ -78,9 +78,11 @@ __host__ __device__ inline SpLayout sp_layout(uint32_t n, uint64_t m2, uint32_t 
   };
   const uint64_t N1 = (uint64_t)n + 2;
   L.stride = (uint32_t)N1;
-  for (int i = 0; i < 23; ++i) L.u32n[i] = take(4 * N1);
+  // (256 entries at least: the colour sort's histogram)
+  for (int i = 0; i < 13; ++i) L.u32n[i] = take(4 * (N1 < 256 ? 256 : N1));
   L.elem = take(2 * N1);
   L.pos = take(2 * N1);
+  L.cnt = take(2 * N1);
   L.fcode = take(4 * (N1 + 1));
   L.ccode = take(4 * (N1 + 1));
   L.pool_owner = take(4 * ((uint64_t)pool + 1));
@@ -90,8 +92,8 @@ __host__ __device__ inline SpLayout sp_layout(uint32_t n, uint64_t m2, uint32_t 
   L.sts = take(8ull * L.nsw);
   L.act = take(8ull * L.nw);
   L.acts = take(8ull * L.nsw);
-  L.tcb = take(8ull * L.nw);
-  L.tcbs = take(8ull * L.nsw);
+  L.itm = take(8ull * L.nw);
+  L.nsb = take(8ull * L.nw);
   L.fcert = take(4 * (m2 + 1));
   L.bcert = take(4 * (m2 + 1));
   L.ccert = take(4 * (m2 + 1));
@@ -104,38 +106,53 @@ __host__ __device__ inline SpLayout sp_layout(uint32_t n, uint64_t m2, uint32_t 
   return L;
 }
 
-// Shared-memory staging: the arrays every refinement step touches (elem,
-// pos, the list of non-singleton cells and the start / active / touched-cell
-// bitmaps with their summaries) live in the warp's shared-memory region when
-// they fit.
-__host__ __device__ inline uint64_t sp_smem_bytes(uint32_t n) {
-  const uint64_t nw = (n + 63) / 64 + 1, nsw = (nw + 63) / 64 + 1;
-  const uint64_t a = ((uint64_t)n + 2) * 2u;
-  return 3 * ((a + 15) & ~15ull) + 3 * 8 * (nw + nsw);
+// Shared-memory staging: the arrays every refinement step touches (elem, pos,
+// neighbour counts by position, the start and active bitmaps with their
+// summaries, the marks of the hash) live in the warp's shared-memory region
+// when they fit.  elem lies at offset 0.
+struct SpStage {
+  uint32_t pos, cnt, stb, sts, act, acts, itm, nsb, bytes;
+};
+__host__ __device__ inline SpStage sp_stage(uint32_t n) {
+  const uint32_t nw = (n + 63) / 64 + 1, nsw = (nw + 63) / 64 + 1;
+  const uint32_t a = ((n + 2) * 2u + 15) & ~15u;
+  SpStage G{};
+  G.pos = a;
+  G.cnt = 2 * a;
+  G.stb = 3 * a;
+  G.sts = G.stb + 8 * nw;
+  G.act = G.sts + 8 * nsw;
+  G.acts = G.act + 8 * nw;
+  G.itm = G.acts + 8 * nsw;
+  G.nsb = G.itm + 8 * nw;
+  G.bytes = (G.nsb + 8 * nw + 15) & ~15u;
+  return G;
 }
+__host__ __device__ inline uint64_t sp_smem_bytes(uint32_t n) { return sp_stage(n).bytes; }
+extern __shared__ __align__(16) uint8_t sp_dyn[];
 
 struct SpWarp {
   uint16_t *elem, *pos;  // position -> vertex, vertex -> position (n <= 65536)
-  uint32_t *slog, *cnt, *T, *Tc, *cellcnt, *off, *fill, *G, *tmp, *lst1, *lst2;
-  uint32_t *seq, *fseq, *bseq, *flabel, *blabel, *dsu, *hist, *pre, *fpos;
-  uint16_t* nsl;
+  uint16_t* cnt;         // position -> neighbours in the splitter, zero between steps
+  uint32_t soff;         // the warp's shared-memory region (offset in sp_dyn), or kNone
+  uint32_t *slog, *tmp, *lst1, *hist, *pre;
+  uint32_t *seq, *fseq, *bseq, *flabel, *blabel, *dsu;
   int32_t *fcode, *ccode, *pool_owner, *pathcode;
   uint32_t *umark;  // per level: start-log size when the level's child was made
   uint2* fixst;     // per stored automorphism: {prefix of seq it fixes, first
                     // position of seq it moves or kNone}, valid for the path
-  uint64_t *stb, *sts, *act, *acts, *tcb, *tcbs;
+  uint64_t *stb, *sts, *act, *acts;  // cell starts (position n too) and active cells
+  uint32_t *itm, *nsb;  // marks of the hash: touched fragments, fragment starts
   uint32_t *fcert, *bcert, *ccert, *reps;
   SpTc* tc;
   uint16_t* auts;
   const int32_t* rp;
   const int32_t* col;
   uint32_t n, nw, nsw, stride;  // stride: elements per pool / ring entry
-  uint32_t ncells, nact, ntouched, nl1, nl2, npend;
+  uint32_t ncells, nact;
   uint32_t pool_top, pool_cap, aut_cap, max_aut;
   uint32_t utop;  // entries of slog
   uint32_t fixcap;  // store entries whose fix state is kept (later ones are checked in full)
-  // values the serial fold hands to the whole warp
-  uint32_t lc, hint;
 };
 
 __shared__ SpWarp g_sp[kSpWarps];
@@ -247,669 +264,668 @@ __device__ __forceinline__ void add_start(SpWarp& W, uint32_t p) {
 }
 
 // ---------------------------------------------------------------------------
-// Rearranging a split cell.  `seg` holds the k touched vertices of the cell
-// (cnt[] > 0); they must end up exactly in [r0, r0 + k) -- the neighbour
-// fragment for a singleton splitter, the tail for a non-singleton one.
-// Touched vertices outside the region swap with untouched vertices inside.
-// When `order` is non-null the region is then written in that order.
+// The refinement's view of the partition: the arrays and bitmaps every step
+// touches, in the warp's shared memory (kS, so the compiler emits shared-memory
+// loads and atomics) or in its device-memory slot.
 // ---------------------------------------------------------------------------
-__device__ __noinline__ void sp_regroup(const uint32_t* seg, uint32_t k, uint32_t r0,
-                                        const uint32_t* order) {
-  SpWarp& W = sp_w();
-  const uint32_t lane = lane_id();
-  if (lane == 0) W.nl1 = W.nl2 = 0;
-  __syncwarp();
-  for (uint32_t i = lane; i < k; i += 32) {
-    const uint32_t u = seg[i], p = W.pos[u];
-    if (p < r0 || p >= r0 + k) W.lst1[atomicAdd(&W.nl1, 1u)] = p;  // touched, misplaced
-  }
-  for (uint32_t q = r0 + lane; q < r0 + k; q += 32) {
-    const uint32_t x = W.elem[q];
-    if (W.cnt[x] == 0) W.lst2[atomicAdd(&W.nl2, 1u)] = q;  // hole: untouched inside
-  }
-  __syncwarp();
-  const uint32_t m = W.nl1;  // == nl2
-  // read both sides first, then write
-  for (uint32_t i0 = 0; i0 < m; i0 += 32) {
-    const uint32_t i = i0 + lane;
-    uint32_t po = 0, ph = 0, vo = 0, vh = 0;
-    if (i < m) {
-      po = W.lst1[i];
-      ph = W.lst2[i];
-      vo = W.elem[po];
-      vh = W.elem[ph];
-    }
-    __syncwarp();
-    if (i < m) {
-      W.elem[po] = vh;
-      W.pos[vh] = po;
-      W.elem[ph] = vo;
-      W.pos[vo] = ph;
-    }
-    __syncwarp();
-  }
-  if (order) {
-    for (uint32_t j = lane; j < k; j += 32) {
-      const uint32_t u = order[j];
-      W.elem[r0 + j] = u;
-      W.pos[u] = r0 + j;
+template <bool kS>
+struct SpRef {
+  uint16_t *elem, *pos, *cnt;
+  uint64_t *stb, *sts, *act, *acts;
+  uint32_t *itm, *nsb;
+  __device__ __forceinline__ explicit SpRef(const SpWarp& W) {
+    if constexpr (kS) {
+      const SpStage G = sp_stage(W.n);
+      uint8_t* b = sp_dyn + W.soff;
+      elem = (uint16_t*)b;
+      pos = (uint16_t*)(b + G.pos);
+      cnt = (uint16_t*)(b + G.cnt);
+      stb = (uint64_t*)(b + G.stb);
+      sts = (uint64_t*)(b + G.sts);
+      act = (uint64_t*)(b + G.act);
+      acts = (uint64_t*)(b + G.acts);
+      itm = (uint32_t*)(b + G.itm);
+      nsb = (uint32_t*)(b + G.nsb);
+    } else {
+      elem = W.elem;
+      pos = W.pos;
+      cnt = W.cnt;
+      stb = W.stb;
+      sts = W.sts;
+      act = W.act;
+      acts = W.acts;
+      itm = W.itm;
+      nsb = W.nsb;
     }
   }
-  __syncwarp();
-}
+};
 
-// Ascending start positions of the non-singleton cells into W.nsl; returns
-// their number.  Each lane scans a contiguous range of start-bitmap words and
-// an exclusive warp scan places its cells.
-__device__ __noinline__ uint32_t sp_list_nonsingleton() {
-  SpWarp& W = sp_w();
-  const uint32_t lane = lane_id();
-  const uint32_t n = W.n, nwr = (n + 63) / 64;
-  const uint32_t per = (nwr + 31) / 32;
-  const uint32_t w0 = min(nwr, lane * per), w1 = min(nwr, w0 + per);
-  const uint64_t lastp = bit64((n - 1) & 63);
-  uint32_t cnt = 0;
-  for (uint32_t w = w0; w < w1; ++w) {
-    const uint64_t b = W.stb[w];
-    uint64_t succ = (b >> 1) | ((w + 1 < nwr ? W.stb[w + 1] : 0ull) << 63);
-    if (w == nwr - 1) succ |= lastp;
-    cnt += popc64(b & ~succ);
-  }
-  uint32_t off = cnt;
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(GCL_FULL, off, o);
-    if (lane >= (uint32_t)o) off += y;
-  }
-  const uint32_t total = __shfl_sync(GCL_FULL, off, 31);
-  off -= cnt;
-  for (uint32_t w = w0; w < w1; ++w) {
-    const uint64_t b = W.stb[w];
-    uint64_t succ = (b >> 1) | ((w + 1 < nwr ? W.stb[w + 1] : 0ull) << 63);
-    if (w == nwr - 1) succ |= lastp;
-    uint64_t ns = b & ~succ;
-    while (ns) {
-      W.nsl[off++] = w * 64 + ctz64(ns);
-      ns &= ns - 1;
-    }
-  }
-  __syncwarp();
-  return total;
+__device__ __forceinline__ void or_bit32(uint32_t* B, uint32_t p) {
+  atomicOr(B + (p >> 5), 1u << (p & 31u));
+}
+// any lane: set a bit of a two-level bitmap
+__device__ __forceinline__ void bm_or(uint64_t* B, uint64_t* Sm, uint32_t p) {
+  or_bit32((uint32_t*)B, p);
+  or_bit32((uint32_t*)Sm, p >> 6);
+}
+// starts of the non-singleton cells among positions 32 wi .. 32 wi + 31
+__device__ __forceinline__ uint32_t sp_nonsingle_word(const uint64_t* stb, uint32_t n,
+                                                      uint32_t wi) {
+  const uint32_t* s = (const uint32_t*)stb;
+  const uint32_t b = s[wi];
+  const uint32_t ns = b & ~((b >> 1) | (s[wi + 1] << 31));
+  const uint32_t left = n - wi * 32;  // position n is marked as a start
+  return left >= 32 ? ns : ns & ((1u << left) - 1u);
+}
+// the j-th (from 0) set bit of x, found by clearing the lower ones: j is
+// almost always 0 or 1 here, where __fns takes a long search
+__device__ __forceinline__ uint32_t nth_bit(uint32_t x, uint32_t j) {
+  for (; j; --j) x &= x - 1;
+  return (uint32_t)(__ffs((int)x) - 1);
 }
 
 // ---------------------------------------------------------------------------
-// One refinement step with a non-singleton splitter of at most 32 members
-// whose members have at most 32 neighbours in all (partition_refinement.cpp:
-// 244-465), warp-synchronously: lane i takes the i-th edge out of the
-// splitter; lanes holding the same neighbour are grouped (its count is the
-// group's size), the neighbours' leaders are grouped by cell, and each
-// touched cell ranks its touched vertices by count with a radix pass over
-// ballots.  A cell that splits is rearranged in place: its untouched
-// vertices first, then its touched ones in ascending count (the reference's
-// fragment order; order inside a fragment is immaterial).  The hash then
-// folds every non-singleton cell in position order -- an untouched one
-// contributes its start, a touched one its fragments -- and lane 0 does the
-// bookkeeping of the splits (starts, active set, hint) in the same order.  Nothing goes through the per-step scratch arrays of the general
-// path.  Returns false, having changed nothing, when the splitter is too
-// large; `lc` and `hint` are the refinement's running hash and hint.
+// The invariant hash of a non-singleton splitter (partition_refinement.cpp:
+// 253-373): mash folded in position order over one item per fragment start,
+// the start plus its vertices' neighbour count (zero unless the position is
+// marked in `itm`).  The fragment starts are the old non-singleton cells' and
+// the marked positions, or, when `listed`, the bits of `nsb`.
+//
+// A lane takes kW words of 32 positions.  Few items are folded one after the
+// other, two instructions each.  Many are folded one bit of the running value
+// at a time over all positions at once: bit j of the value before item i is bit
+// j of the initial value xor the parity of the flips of the items before it
+// (a prefix parity within the word, a ballot across the lanes), and that gives
+// the carries into bit j + 1.  A position's own bits are constants of its word,
+// so no list of cells is ever built.  Listing the cells and taking 15 ballots
+// per 32 of them took 61,700 of a step's 67,600 cycles on a 64 x 64 torus
+// (about 1,200 cells); with this fold the search of that torus takes 71 ms
+// instead of 270.
 // ---------------------------------------------------------------------------
-__device__ __noinline__ bool sp_refine_small(uint32_t s, uint32_t len, uint32_t* lc_io,
-                                             uint32_t* hint_io) {
-  SpWarp& W = sp_w();
-  const uint32_t lane = lane_id();
-  if (len > 32) return false;
-  // the splitter's edges, lane by lane
-  uint32_t d = 0;
-  int32_t b = 0;
-  if (lane < len) {
-    const uint32_t w = W.elem[s + lane];
-    b = W.rp[w];
-    d = (uint32_t)(W.rp[w + 1] - b);
-  }
-  uint32_t incl = d;
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(GCL_FULL, incl, o);
-    if (lane >= (uint32_t)o) incl += y;
-  }
-  const uint32_t D = __shfl_sync(GCL_FULL, incl, 31);
-  if (D > 32) return false;
-  const uint32_t excl = incl - d;
-  const uint32_t nonempty = __ballot_sync(GCL_FULL, d > 0);
-  const uint32_t firsts = __reduce_or_sync(GCL_FULL, d > 0 ? (1u << excl) : 0u);
-  uint32_t u = kNone;
-  {
-    // lane i < D: member = the k-th non-empty one, k = firsts up to lane i
-    const uint32_t k = (uint32_t)__popc(firsts & (lanemask_lt() | (1u << lane)));
-    const int src = lane < D ? __fns(nonempty, 0, (int)k) : 0;
-    const int32_t bs = __shfl_sync(GCL_FULL, b, src);
-    const uint32_t es = __shfl_sync(GCL_FULL, excl, src);
-    if (lane < D) u = (uint32_t)W.col[bs + (int32_t)(lane - es)];
-  }
-  // the neighbour's cell; singleton cells never split (:257-259)
-  uint32_t p = 0, c = kNone, L = 0;
-  if (u != kNone) {
-    p = W.pos[u];
-    c = sp_cell_of(W, p);
-    L = sp_cell_end(W, c) - c;
-    if (L <= 1) u = kNone;
-  }
-  const uint32_t gu = __match_any_sync(GCL_FULL, u);
-  const uint32_t cnt = (uint32_t)__popc(gu);  // u's neighbours in the splitter
-  const bool lead = u != kNone && lane == (uint32_t)(__ffs(gu) - 1);
-  const uint32_t gc = __match_any_sync(GCL_FULL, lead ? c : kNone);
-  const uint32_t k = lead ? (uint32_t)__popc(gc) : 0u;  // touched vertices of the cell
-  // rank by count within the cell (radix pass, counts <= 32: 6 bits)
-  uint32_t peers = lead ? gc : 0u, less = 0;
-  for (int bit = 5; bit >= 0; --bit) {
-    const bool one = (cnt >> bit) & 1u;
-    const uint32_t m1 = __ballot_sync(GCL_FULL, lead && one);
-    if (lead) {
-      if (one) {
-        less += (uint32_t)__popc(peers & ~m1);
-        peers &= m1;
-      } else {
-        peers &= ~m1;
+template <bool kS, int kW>
+__device__ __noinline__ uint32_t sp_fold(uint32_t lc, bool listed) {
+  constexpr uint32_t C = 065435u;
+  // items above which the bit-wise fold is the faster one: about 20 cycles per
+  // item against about 2,000 (one word per lane) or 3,500 (four)
+  constexpr uint32_t kDense = kW == 1 ? 96 : 176;
+  const SpWarp& W = sp_w();
+  const SpRef<kS> R(W);
+  const uint32_t lane = lane_id(), n = W.n, nwd = (n + 31) / 32, lt = lanemask_lt();
+  for (uint32_t base = 0; base < nwd; base += 32 * kW) {
+    uint32_t vw[kW], mw[kW], K = 0;
+    const uint32_t w0 = base + lane * kW;
+#pragma unroll
+    for (int w = 0; w < kW; ++w) {
+      const uint32_t wi = w0 + w;
+      vw[w] = mw[w] = 0;
+      if (wi < nwd) {
+        const uint32_t m = R.itm[wi];
+        vw[w] = listed ? R.nsb[wi] : sp_nonsingle_word(R.stb, n, wi) | m;
+        mw[w] = m & vw[w];
+        K += (uint32_t)__popc(vw[w]);
       }
     }
-  }
-  const uint32_t eqidx = (uint32_t)__popc(peers & lanemask_lt());
-  const uint32_t fsize = (uint32_t)__popc(peers);
-  const bool uniform = lead && k == L && fsize == k;  // one common count: no split
-  const bool split = lead && !uniform;
-  const uint32_t R0 = c + (L - k);
-  const uint32_t f = R0 + less;  // this vertex's fragment start
-  const bool cell_lead = lead && lane == (uint32_t)(__ffs(gc) - 1);
-  // rearrange the split cells: touched vertices to R0 + rank, the untouched
-  // vertices found in [R0, c + L) to the positions the touched ones leave
-  uint32_t x = 0, h = 0;
-  bool out = false;
-  if (split) {
-    const bool in = p >= R0;
-    const uint32_t inner = __reduce_or_sync(gc, in ? (1u << (p - R0)) : 0u);
-    const uint32_t outs = __ballot_sync(gc, !in);
-    if (!in) {
-      const uint32_t j = (uint32_t)__popc(outs & lanemask_lt());
-      const uint32_t holes = ~inner & (k >= 32 ? 0xffffffffu : ((1u << k) - 1u));
-      h = R0 + (uint32_t)__fns(holes, 0, (int)j + 1);
-      x = W.elem[h];
-      out = true;
-    }
-  }
-  __syncwarp();
-  if (out) {
-    W.elem[p] = x;
-    W.pos[x] = p;
-  }
-  if (split) {
-    const uint32_t t = f + eqidx;
-    W.elem[t] = u;
-    W.pos[u] = t;
-  }
-  if (cell_lead) bm_set_atomic(W.tcb, W.tcbs, c);
-  __syncwarp();
-  // the fold over the non-singleton cells in position order (:253-465)
-  uint32_t lc = *lc_io, hint = *hint_io;
-  const uint32_t K = sp_list_nonsingleton();
-  uint32_t pend = 0;  // lanes whose fragment is a new cell start
-  for (uint32_t i0 = 0; i0 < K; i0 += 32) {
-    const uint32_t il = i0 + lane;
-    const uint32_t cl = il < K ? W.nsl[il] : 0u;
-    const uint32_t tmask = __ballot_sync(GCL_FULL, il < K && bm_test(W.tcb, cl));
-    const uint32_t cnt32 = min(32u, K - i0);
-    if (!tmask) {  // 32 untouched cells: each member has count 0, item = start
-      lc = mash_fold32(lc, cl, cnt32);
-      continue;
-    }
-    for (uint32_t jj = 0; jj < cnt32; ++jj) {
-      const uint32_t cc = __shfl_sync(GCL_FULL, cl, (int)jj);
-      if (!((tmask >> jj) & 1u)) {
-        lc = mash(lc, cc);  // untouched: every member has count 0
-        continue;
-      }
-      const uint32_t src = (uint32_t)__ffs(__ballot_sync(GCL_FULL, cell_lead && c == cc)) - 1;
-      const bool uni = __shfl_sync(GCL_FULL, uniform, (int)src);
-      if (uni) {
-        lc = mash(lc, __shfl_sync(GCL_FULL, cnt, (int)src) + cc);
-        continue;
-      }
-      const uint32_t Lc = __shfl_sync(GCL_FULL, L, (int)src);
-      const uint32_t kc = __shfl_sync(GCL_FULL, k, (int)src);
-      const bool was = bm_test(W.act, cc);
-      __syncwarp();
-      uint32_t maxsz = 0, maxf = cc;
-      if (Lc > kc) {  // the untouched fragment first
-        lc = mash(lc, 0u + cc);
-        maxsz = Lc - kc;
-      }
-      // the touched fragments in ascending count (= ascending start)
-      uint32_t F = __ballot_sync(GCL_FULL, split && c == cc && eqidx == 0);
-      while (F) {
-        const uint32_t fm = __reduce_min_sync(GCL_FULL, ((F >> lane) & 1u) ? f : kNone);
-        const uint32_t s2 = (uint32_t)__ffs(__ballot_sync(GCL_FULL, ((F >> lane) & 1u) && f == fm)) - 1;
-        F &= ~(1u << s2);
-        const uint32_t sz = __shfl_sync(GCL_FULL, fsize, (int)s2);
-        lc = mash(lc, __shfl_sync(GCL_FULL, cnt, (int)s2) + fm);
-        if (fm != cc) {
-          pend |= 1u << s2;
-          if (sz == 1) hint = fm;
+    bool dense = __reduce_add_sync(GCL_FULL, K) > kDense;
+    uint32_t kb[6][kW];
+    if (dense) {  // the counts, one bit per word (larger counts take the other way)
+      bool big = false;
+#pragma unroll
+      for (int w = 0; w < kW; ++w) {
+#pragma unroll
+        for (int j = 0; j < 6; ++j) kb[j][w] = 0;
+        for (uint32_t m = mw[w]; m; m &= m - 1) {
+          const uint32_t b = (uint32_t)__ffs((int)m) - 1, k = R.cnt[(w0 + w) * 32 + b];
+          big |= k >= 64;
+#pragma unroll
+          for (int j = 0; j < 6; ++j) kb[j][w] |= ((k >> j) & 1u) << b;
         }
-        if (lane == 0 && fm != cc) {
-          W.ncells += 1;
-          if (!bm_test(W.act, fm)) {
-            bm_set1(W.act, W.acts, fm);
-            W.nact += 1;
+      }
+      dense = !__any_sync(GCL_FULL, big);
+    }
+    if (!dense) {
+      uint32_t some = 0;
+#pragma unroll
+      for (int w = 0; w < kW; ++w) some |= vw[w];
+      for (uint32_t any = __ballot_sync(GCL_FULL, some != 0); any; any &= any - 1) {
+        const int src = __ffs((int)any) - 1;
+#pragma unroll
+        for (int w = 0; w < kW; ++w) {
+          const uint32_t m = __shfl_sync(GCL_FULL, mw[w], src);
+          uint32_t x = __shfl_sync(GCL_FULL, vw[w], src);
+          const uint32_t pb = (base + (uint32_t)src * kW + w) * 32;
+          for (; x; x &= x - 1) {
+            const uint32_t b = (uint32_t)__ffs((int)x) - 1;
+            uint32_t v = pb + b;
+            if ((m >> b) & 1u) v += R.cnt[v];
+            lc = (lc ^ C) + v;
           }
         }
-        if (sz > maxsz) {
-          maxsz = sz;
-          maxf = fm;
-        }
       }
-      if (lane == 0 && !was) {
-        if (!bm_test(W.act, cc)) {
-          bm_set1(W.act, W.acts, cc);
-          W.nact += 1;
-        }
-        if (bm_test(W.act, maxf)) {
-          bm_clear1(W.act, W.acts, maxf);
-          W.nact -= 1;
-        }
+      continue;
+    }
+    uint32_t carry[kW], cp[kW], out = 0;
+#pragma unroll
+    for (int w = 0; w < kW; ++w) carry[w] = cp[w] = 0;
+#pragma unroll
+    for (int j = 0; j < 15; ++j) {
+      constexpr uint32_t kPat[5] = {0xaaaaaaaau, 0xccccccccu, 0xf0f0f0f0u, 0xff00ff00u,
+                                    0xffff0000u};
+      const uint32_t Cm = ((C >> j) & 1u) ? 0xffffffffu : 0u;
+      uint32_t vj[kW], inc[kW], par = 0;
+#pragma unroll
+      for (int w = 0; w < kW; ++w) {
+        // bit j of the item: position plus count
+        const uint32_t pj = j < 5 ? kPat[j < 5 ? j : 0] : 0u - (((w0 + w) * 32 >> j) & 1u);
+        const uint32_t kj = j < 6 ? kb[j < 6 ? j : 0][w] : 0u;
+        vj[w] = pj ^ kj ^ cp[w];
+        cp[w] = (pj & kj) | (cp[w] & (pj ^ kj));
+        uint32_t f = vw[w] & (Cm ^ vj[w] ^ carry[w]);
+        f ^= f << 1;
+        f ^= f << 2;
+        f ^= f << 4;
+        f ^= f << 8;
+        f ^= f << 16;
+        inc[w] = f;
+        par ^= f;
       }
-      __syncwarp();
+      const uint32_t B = __ballot_sync(GCL_FULL, par >> 31);
+      const uint32_t x0 = (lc >> j) & 1u;
+      uint32_t run = x0 ^ ((uint32_t)__popc(B & lt) & 1u);
+#pragma unroll
+      for (int w = 0; w < kW; ++w) {
+        const uint32_t y = (0u - run) ^ (inc[w] << 1) ^ Cm;  // the value before, xor 065435
+        carry[w] = (y & vj[w]) | (carry[w] & (y ^ vj[w]));
+        run ^= inc[w] >> 31;
+      }
+      out |= (x0 ^ ((uint32_t)__popc(B) & 1u)) << j;
+    }
+    lc = out;
+  }
+  return lc;
+}
+
+// ---------------------------------------------------------------------------
+// A step whose splitter has more than 32 edges.  Neighbour counts are kept by
+// position, so a cell's counts are contiguous: a lane tests whole small cells
+// for a common count, and each cell without one is sorted by count -- up to 32
+// vertices by a radix pass over ballots, larger ones by a counting sort.  A
+// singleton splitter's cells split into [neighbours, non-neighbours]
+// (:296-309, 399-435), the others into ascending counts (:326-465).
+// ---------------------------------------------------------------------------
+struct SpStep {
+  uint32_t lc, hint, made;  // made: new cell starts
+};
+
+template <bool kS>
+__device__ __noinline__ SpStep sp_refine_general(uint32_t s, uint32_t e, uint32_t lc,
+                                                 uint32_t hint, uint32_t utop) {
+  SpWarp& W = sp_w();
+  const SpRef<kS> R(W);
+  const uint32_t lane = lane_id(), n = W.n, nw = W.nw, nsw = W.nsw, lt = lanemask_lt();
+  const uint32_t nwd = (n + 31) / 32;
+  const bool single = e - s == 1;
+  const uint32_t flip = single ? 1u : 0u;  // a neighbour's key is 0, a non-neighbour's 1
+  const uint32_t utop0 = utop;
+  auto add = [&](uint32_t u) {
+    const uint32_t p = R.pos[u];
+    atomicAdd((uint32_t*)R.cnt + (p >> 1), 1u << ((p & 1u) * 16u));
+  };
+  if (e - s <= 8) {
+    for (uint32_t q = s; q < e; ++q) {
+      const uint32_t w = R.elem[q];
+      const int32_t f = W.rp[w + 1];
+      for (int32_t i = W.rp[w] + (int32_t)lane; i < f; i += 32) add((uint32_t)W.col[i]);
+    }
+  } else {
+    for (uint32_t q = s + lane; q < e; q += 32) {
+      const uint32_t w = R.elem[q];
+      const int32_t f = W.rp[w + 1];
+      for (int32_t i = W.rp[w]; i < f; ++i) add((uint32_t)W.col[i]);
     }
   }
-  // the new starts, set after the fold (which walked the old ones)
-  while (pend) {
-    const uint32_t s2 = (uint32_t)__ffs(pend) - 1;
-    pend &= pend - 1;
-    const uint32_t fs = __shfl_sync(GCL_FULL, f, (int)s2);
-    if (lane == 0) add_start(W, fs);
-  }
-  if (cell_lead) {  // the touched-cell marks go
-    W.tcb[c >> 6] = 0;
-    W.tcbs[c >> 12] = 0;
+  for (uint32_t wi = lane; wi < nwd; wi += 32) R.nsb[wi] = sp_nonsingle_word(R.stb, n, wi);
+  __syncwarp();
+  // a fragment of a split cell: its start, hint and place in the active set
+  // are those of partition_refinement.cpp:399-460; returns the new starts
+  auto fragment = [&](bool frag, uint32_t c, uint32_t f, uint32_t size, uint32_t count,
+                      bool active) {
+    const bool fresh = frag && f != c;
+    const uint32_t m = __ballot_sync(GCL_FULL, fresh);
+    if (frag && count && !single) or_bit32(R.itm, f);
+    if (fresh) {
+      W.slog[utop + (uint32_t)__popc(m & lt)] = f;
+      bm_or(R.stb, R.sts, f);
+      or_bit32(R.nsb, f);
+    }
+    if (frag && active) bm_or(R.act, R.acts, f);
+    utop += (uint32_t)__popc(m);
+    if (!single) {
+      const uint32_t h = __reduce_max_sync(GCL_FULL, fresh && size == 1 ? f + 1 : 0u);
+      if (h) hint = h - 1;
+    }
+  };
+  // the split of a singleton splitter: nb neighbours, nn others
+  auto split_single = [&](uint32_t c, uint32_t nb, uint32_t nn, bool was) {
+    const bool rest = was || nb >= nn;
+    lc = (lc ^ 065435u) + (c + nb - 1);
+    if (rest && nn == 1) hint = c + nb;
+    if (!rest && nb == 1) hint = c;
+    fragment(lane < 2, c, lane == 1 ? c + nb : c, 0, 0, lane == (rest ? 1u : 0u));
+  };
+  for (uint32_t base = 0; base < nwd; base += 32) {
+    const uint32_t wi = base + lane;
+    uint32_t pend = 0;
+    for (uint32_t x = wi < nwd ? R.nsb[wi] : 0u; x; x &= x - 1) {
+      const uint32_t b = (uint32_t)__ffs((int)x) - 1, c = wi * 32 + b;
+      const uint32_t ce = bm_next(R.stb, R.sts, c + 1, n, nw, nsw);
+      bool differ = ce - c > 32;  // large cells are tested by the whole warp
+      if (!differ) {
+        const uint32_t a = R.cnt[c];
+        for (uint32_t q = c + 1; q < ce; ++q) differ |= R.cnt[q] != a;
+        if (!differ && a && !single) or_bit32(R.itm, c);
+      }
+      if (differ) pend |= 1u << b;
+    }
+    __syncwarp();
+    for (uint32_t any = __ballot_sync(GCL_FULL, pend != 0); any; any &= any - 1) {
+      const int src = __ffs((int)any) - 1;
+      for (uint32_t m = __shfl_sync(GCL_FULL, pend, src); m; m &= m - 1) {
+        const uint32_t c = (base + (uint32_t)src) * 32 + (uint32_t)__ffs((int)m) - 1;
+        const uint32_t ce = bm_next(R.stb, R.sts, c + 1, n, nw, nsw), L = ce - c;
+        const bool was = bm_test(R.act, c);
+        if (L <= 32) {
+          const bool in = lane < L;
+          const uint32_t v = in ? R.elem[c + lane] : 0u, a = in ? R.cnt[c + lane] : 0u;
+          const uint32_t key = in ? a ^ flip : 0u;
+          uint32_t peers = L == 32 ? 0xffffffffu : (1u << L) - 1u, less = 0;
+          const uint32_t top = __reduce_max_sync(GCL_FULL, key);
+          for (int bit = 31 - __clz((int)top); bit >= 0; --bit) {
+            const bool one = (key >> bit) & 1u;
+            const uint32_t m1 = __ballot_sync(GCL_FULL, in && one);
+            if (one) {
+              less += (uint32_t)__popc(peers & ~m1);
+              peers &= m1;
+            } else {
+              peers &= ~m1;
+            }
+          }
+          const uint32_t eq = (uint32_t)__popc(peers & lt), size = (uint32_t)__popc(peers);
+          const uint32_t f = c + less;
+          __syncwarp();
+          if (in) {
+            R.elem[f + eq] = (uint16_t)v;
+            R.pos[v] = (uint16_t)(f + eq);
+            R.cnt[f + eq] = (uint16_t)a;
+          }
+          if (single) {
+            const uint32_t nb = (uint32_t)__popc(__ballot_sync(GCL_FULL, in && key == 0));
+            split_single(c, nb, L - nb, was);
+          } else {
+            const bool frag = in && eq == 0;
+            const uint32_t rank = frag ? (size << 6) | (63u - less) : 0u;
+            const uint32_t best = __reduce_max_sync(GCL_FULL, rank);
+            fragment(frag, c, f, size, a, was ? f != c : rank != best);
+          }
+          __syncwarp();
+          continue;
+        }
+        uint32_t mn = 0xffffffffu, mx = 0;
+        for (uint32_t i = lane; i < L; i += 32) {
+          const uint32_t x = R.cnt[c + i];
+          mn = min(mn, x);
+          mx = max(mx, x);
+        }
+        mn = __reduce_min_sync(GCL_FULL, mn);
+        mx = __reduce_max_sync(GCL_FULL, mx);
+        if (mn == mx) {
+          if (mn && !single && lane == 0) or_bit32(R.itm, c);
+          __syncwarp();
+          continue;
+        }
+        const uint32_t range = mx - mn + 1;
+        for (uint32_t i = lane; i < range; i += 32) W.hist[i] = 0;
+        __syncwarp();
+        for (uint32_t i = lane; i < L; i += 32)
+          atomicAdd(&W.hist[(uint32_t)(R.cnt[c + i] - mn) ^ flip], 1u);
+        __syncwarp();
+        // fragment starts (relative) and the first largest fragment
+        uint32_t run = 0, best = 0, bestf = 0;
+        for (uint32_t i0 = 0; i0 < range; i0 += 32) {
+          const uint32_t i = i0 + lane, h = i < range ? W.hist[i] : 0u;
+          uint32_t incl = h;
+          for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(GCL_FULL, incl, o);
+            if (lane >= (uint32_t)o) incl += y;
+          }
+          const uint32_t f = run + incl - h;
+          if (i < range) W.pre[i] = f;
+          const uint32_t mxh = __reduce_max_sync(GCL_FULL, h);
+          if (mxh > best) {
+            best = mxh;
+            bestf = __shfl_sync(GCL_FULL, f, __ffs((int)__ballot_sync(GCL_FULL, h == mxh)) - 1);
+          }
+          run += __shfl_sync(GCL_FULL, incl, 31);
+        }
+        __syncwarp();
+        if (single) {
+          split_single(c, W.hist[0], W.hist[1], was);
+        } else {
+          for (uint32_t i0 = 0; i0 < range; i0 += 32) {
+            const uint32_t i = i0 + lane, h = i < range ? W.hist[i] : 0u;
+            const uint32_t f = i < range ? W.pre[i] : 0u;
+            fragment(h != 0, c, c + f, h, mn + i, was ? f != 0 : f != bestf);
+          }
+        }
+        __syncwarp();
+        for (uint32_t i = lane; i < L; i += 32) {
+          const uint32_t a = R.cnt[c + i];
+          W.tmp[atomicAdd(&W.pre[(a - mn) ^ flip], 1u)] = (a << 16) | R.elem[c + i];
+        }
+        __syncwarp();
+        for (uint32_t i = lane; i < L; i += 32) {
+          const uint32_t x = W.tmp[i], v = x & 0xffffu;
+          R.elem[c + i] = (uint16_t)v;
+          R.pos[v] = (uint16_t)(c + i);
+          R.cnt[c + i] = (uint16_t)(x >> 16);
+        }
+        __syncwarp();
+      }
+    }
   }
   __syncwarp();
-  *lc_io = lc;
-  *hint_io = hint;
-  return true;
+  if (!single) lc = n <= 1024 ? sp_fold<kS, 1>(lc, true) : sp_fold<kS, 4>(lc, true);
+  __syncwarp();
+  uint4* z = (uint4*)R.cnt;
+  for (uint32_t i = lane; i < (2 * (n + 2) + 15) / 16; i += 32) z[i] = make_uint4(0, 0, 0, 0);
+  for (uint32_t wi = lane; wi < nwd; wi += 32) R.itm[wi] = 0;
+  __syncwarp();
+  return {lc, hint, utop - utop0};
 }
 
 // ---------------------------------------------------------------------------
 // Partition_s_refinement (partition_refinement.cpp:150-485).  The active
 // bitmap holds the initially active cells; returns the code (-1 on a failed
 // consistency check).  The caller increments the level.
+//
+// Steps whose splitter has at most 32 edges -- nearly all -- are
+// warp-synchronous: lane i takes the i-th edge, cells are grouped with
+// match_any, and every split cell's start, log entry and active bits are
+// written by its own lane with shared-memory atomics; only the hash follows
+// position order.  A split makes as many active cells as cell starts: a cell
+// that was active gets its new fragments, one that was not all but its first
+// largest.  Singleton neighbours end a step early.  With one lane writing the
+// splits one after the other a singleton step took 1,900-2,500 cycles and a
+// non-singleton one 6,000 beside its hash; a mixed batch up to 256 vertices
+// took 432 ms then and 252 ms now, four copies of a 4-regular graph on 64
+// vertices 219 ms and 133 ms.
 // ---------------------------------------------------------------------------
-__device__ __noinline__ int sp_refine() {
+template <bool kS>
+__device__ __noinline__ int sp_refine_t() {
   SpWarp& W = sp_w();
-  const uint32_t lane = lane_id();
+  const SpRef<kS> R(W);
+  const uint32_t lane = lane_id(), lt = lanemask_lt();
   const uint32_t n = W.n, nw = W.nw, nsw = W.nsw;
-  uint32_t lc = W.ncells, hint = 0;
-  uint64_t iters = 0;
+  constexpr uint32_t C = 065435u;
+  uint32_t ncells = W.ncells, nact = W.nact, utop = W.utop;
+  uint32_t lc = ncells, hint = 0, iters = 0;
   int ok = 1;
-  // the arrays a step touches, in registers for the whole refinement (the
-  // warp record's pointers would otherwise be reloaded after every store)
-  uint16_t* const elem = W.elem;
-  uint16_t* const pos = W.pos;
-  uint64_t* const stb = W.stb;
-  uint64_t* const sts = W.sts;
-  uint64_t* const act = W.act;
-  uint64_t* const acts = W.acts;
   const int32_t* const rp = W.rp;
   const int32_t* const col = W.col;
   uint32_t* const slog = W.slog;
-  // the cell and active counts and the start log's top, kept by every lane
-  // alike during the singleton steps; the warp record holds them while the
-  // other paths run (they update them there) and after the refinement
-  uint32_t ncells = W.ncells, nact = W.nact, utop = W.utop;
+  // whether the vertex at position p is not alone in its cell (position n is
+  // marked as a start)
+  auto shared_cell = [&](uint32_t p) {
+    const uint32_t* s = (const uint32_t*)R.stb;
+    return !((s[p >> 5] >> (p & 31u)) & (s[(p + 1) >> 5] >> ((p + 1) & 31u)) & 1u);
+  };
   while (ncells < n && nact > 0) {
-    if (++iters > 4ull * n + 64) {  // every step removes an active cell or splits one
+    if (++iters > 4 * n + 64) {  // every step removes an active cell or splits one
       ok = 0;
       break;
     }
-    uint32_t s;
-    if (bm_test(act, hint)) {
-      s = hint;
-    } else {
-      s = bm_next(act, acts, hint + 1, n, nw, nsw);
-      if (s >= n) s = bm_next(act, acts, 0, n, nw, nsw);
-    }
+    // splitter: hint if active, else the next active after it, else wrap
+    uint32_t s = bm_next(R.act, R.acts, hint, n, nw, nsw);
+    if (s >= n) s = bm_next(R.act, R.acts, 0, n, nw, nsw);
     if (s >= n) {
       ok = 0;
       break;
     }
+    const uint32_t e = bm_next(R.stb, R.sts, s + 1, n, nw, nsw);
     __syncwarp();
-    if (lane == 0) bm_clear1(act, acts, s);
+    if (lane == 0) bm_clear1(R.act, R.acts, s);
     nact -= 1;
-    const uint32_t e = bm_test(stb, s + 1) || s + 1 >= n ? s + 1
-                                                          : bm_next(stb, sts, s + 1, n, nw, nsw);
     const uint32_t len = e - s;
-    lc = mash(lc, s + e - 1);
-    if (len > 1) lc = mash(lc, len);
-
-    // Singleton splitter {w} with at most 32 neighbours: lane i holds
-    // neighbour i; lanes whose neighbours share a (non-singleton) cell are
-    // grouped with match_any; a cell that is not all neighbours splits into
-    // [neighbours, non-neighbours]: its misplaced neighbours swap with the
-    // non-neighbours inside its first k positions, then the split cells are
-    // folded in position order (:296-309, 399-435).
-    int32_t sb = 0, sd = 0;
+    lc = (lc ^ C) + (s + e - 1);
     if (len == 1) {
-      const uint32_t w = elem[s];
-      sb = rp[w];
-      sd = rp[w + 1] - sb;
-    }
-    if (len == 1 && sd <= 32) {
-      const bool have = (int32_t)lane < sd;
-      uint32_t u = 0, p = 0, c = kNone, L = 0;
-      if (have) {
-        u = (uint32_t)col[sb + (int32_t)lane];
-        p = pos[u];
-        c = bm_prev(stb, sts, p);
-        L = bm_next(stb, sts, c + 1, n, nw, nsw) - c;
-      }
-      const bool act_l = have && L > 1;
-      const uint32_t grp = __match_any_sync(GCL_FULL, act_l ? c : kNone);
-      const uint32_t k = (uint32_t)__popc(grp);
-      const bool spl_l = act_l && k < L;
-      uint32_t h = 0, x = 0;
-      bool mv = false;
-      if (spl_l) {
-        const bool in = p < c + k;
-        const uint32_t inner = __reduce_or_sync(grp, in ? (1u << (p - c)) : 0u);
-        const uint32_t outs = __ballot_sync(grp, !in);
-        if (!in) {
-          const uint32_t j = (uint32_t)__popc(outs & lanemask_lt());
-          const uint32_t holes = ~inner & (k >= 32 ? 0xffffffffu : ((1u << k) - 1u));
-          h = c + (uint32_t)__fns(holes, 0, (int)j + 1);
-          x = elem[h];
-          mv = true;
+      const uint32_t w = R.elem[s];
+      const int32_t sb = rp[w], sd = rp[w + 1] - sb;
+      if (sd <= 32) {
+        // Singleton splitter: a cell splits into [neighbours, non-neighbours]
+        // when only some of its vertices are neighbours (:296-309, 399-435).
+        uint32_t u = 0, p = 0, c = kNone, L = 0;
+        bool on = false;
+        if ((int32_t)lane < sd) {
+          u = (uint32_t)col[sb + (int32_t)lane];
+          p = R.pos[u];
+          on = shared_cell(p);
         }
-      }
-      // whether each split cell was active, read before any of this step's
-      // active-set writes (they only touch the split cells' own starts)
-      const bool lead = spl_l && lane == (uint32_t)(__ffs(grp) - 1);
-      const bool was_l = lead && bm_test(act, c);
-      __syncwarp();
-      if (mv) {
-        elem[h] = u;
-        pos[u] = h;
-        elem[p] = x;
-        pos[x] = p;
-      }
-      // split cells in position order: hash, starts, active set;
-      // hint and hash are the same on every lane, lane 0 writes
-      uint32_t leaders = __ballot_sync(GCL_FULL, lead);
-      while (leaders) {
-        const bool mine = (leaders >> lane) & 1u;
-        const uint32_t cmin = __reduce_min_sync(GCL_FULL, mine ? c : kNone);
-        const uint32_t src = (uint32_t)__ffs(__ballot_sync(GCL_FULL, mine && c == cmin)) - 1;
-        const uint32_t kk = __shfl_sync(GCL_FULL, k, (int)src);
-        const uint32_t LL = __shfl_sync(GCL_FULL, L, (int)src);
-        const bool was = __shfl_sync(GCL_FULL, was_l, (int)src);
-        leaders &= ~(1u << src);
-        const uint32_t pp = cmin + kk;
-        lc = mash(lc, pp - 1);  // cell.first + neighbors_size - 1
-        const uint32_t nb = kk, nn = LL - kk;
-        const bool to_rest = was || nb >= nn;
-        if (to_rest) {
-          if (nn == 1) hint = pp;
+        __syncwarp();
+        if (!__any_sync(GCL_FULL, on)) continue;
+        if (on) {
+          c = bm_prev(R.stb, R.sts, p);
+          L = bm_next(R.stb, R.sts, p + 1, n, nw, nsw) - c;
+        }
+        const uint32_t grp = __match_any_sync(GCL_FULL, c);
+        const uint32_t k = (uint32_t)__popc(grp);
+        const bool spl = on && k < L;
+        if (!__any_sync(GCL_FULL, spl)) continue;
+        // misplaced neighbours swap with the non-neighbours inside the cell's
+        // first k positions
+        uint32_t h = c, x = 0;
+        bool mv = false;
+        if (__any_sync(GCL_FULL, spl && k > 1)) {
+          const bool in = p < c + k;
+          uint32_t inner = 0;
+          if (spl) inner = __reduce_or_sync(grp, in ? 1u << (p - c) : 0u);
+          const uint32_t outs = __ballot_sync(GCL_FULL, spl && !in) & grp;
+          mv = spl && !in;
+          if (mv)
+            h = c + nth_bit(~inner & (k >= 32 ? 0xffffffffu : (1u << k) - 1u),
+                            (uint32_t)__popc(outs & lt));
         } else {
-          if (nb == 1) hint = cmin;
+          mv = spl && p != c;
         }
-        if (lane == 0) {
-          slog[utop] = pp;
-          bm_set1(stb, sts, pp);
-          bm_set1(act, acts, to_rest ? pp : cmin);
+        if (mv) x = R.elem[h];
+        const bool lead = spl && lane == (uint32_t)(__ffs((int)grp) - 1);
+        const bool was = lead && bm_test(R.act, c);
+        const uint32_t leaders = __ballot_sync(GCL_FULL, lead);
+        const uint32_t made = (uint32_t)__popc(leaders);
+        __syncwarp();
+        if (mv) {
+          R.elem[h] = (uint16_t)u;
+          R.pos[u] = (uint16_t)h;
+          R.elem[p] = (uint16_t)x;
+          R.pos[x] = (uint16_t)p;
         }
-        utop += 1;
-        ncells += 1;
-        nact += 1;
-      }
-      __syncwarp();
-      continue;
-    }
-    // the other paths keep the counts in the warp record
-    if (lane == 0) {
-      W.ncells = ncells;
-      W.nact = nact;
-      W.utop = utop;
-      W.ntouched = 0;
-    }
-    __syncwarp();
-
-    // a small non-singleton splitter: warp-synchronous, no scratch arrays
-    if (len > 1 && sp_refine_small(s, len, &lc, &hint)) {
-      ncells = W.ncells;
-      nact = W.nact;
-      utop = W.utop;
-      continue;
-    }
-
-    // count neighbours in the splitter, record touched vertices and cells
-    // (cells that are singletons never split and are skipped, :257-259)
-    if (len == 1) {
-      const uint32_t w = W.elem[s];
-      const int32_t b = W.rp[w], d = W.rp[w + 1] - b;
-      for (int32_t i = (int32_t)lane; i < d; i += 32) {
-        const uint32_t u = (uint32_t)W.col[b + i];
-        const uint32_t c = sp_cell_of(W, W.pos[u]);
-        if (sp_cell_end(W, c) - c == 1) continue;
-        if (atomicAdd(&W.cnt[u], 1u) == 0) {
-          const uint32_t t = atomicAdd(&W.ntouched, 1u);
-          W.T[t] = u;
-          W.Tc[t] = c;
-          if (atomicAdd(&W.cellcnt[c], 1u) == 0) bm_set_atomic(W.tcb, W.tcbs, c);
+        uint32_t hv = 0, key = kNone;
+        if (lead) {
+          const uint32_t pp = c + k, nn = L - k;
+          const bool rest = was || k >= nn;
+          hv = rest ? (nn == 1 ? pp + 1 : 0u) : (k == 1 ? c + 1 : 0u);
+          key = (c << 6) | k;
+          slog[utop + (uint32_t)__popc(leaders & lt)] = pp;
+          bm_or(R.stb, R.sts, pp);
+          bm_or(R.act, R.acts, rest ? pp : c);
         }
+        utop += made;
+        ncells += made;
+        nact += made;
+        // hash (cell.first + neighbors_size - 1) in position order; the hint
+        // is the last split cell's that sets one
+        if (made == 1) {
+          key = __shfl_sync(GCL_FULL, key, __ffs((int)leaders) - 1);
+          hv = __shfl_sync(GCL_FULL, hv, __ffs((int)leaders) - 1);
+          lc = (lc ^ C) + ((key >> 6) + (key & 63u) - 1);
+        } else {
+          for (uint32_t i = 0; i < made; ++i) {
+            const uint32_t m = __reduce_min_sync(GCL_FULL, key);
+            if (key == m) key = kNone;
+            lc = (lc ^ C) + ((m >> 6) + (m & 63u) - 1);
+          }
+          hv = __reduce_max_sync(GCL_FULL, hv);
+        }
+        if (hv) hint = hv - 1;
+        __syncwarp();
+        continue;
       }
     } else {
-      for (uint32_t q = s + lane; q < e; q += 32) {
-        const uint32_t w = W.elem[q];
-        const int32_t b = W.rp[w], f = W.rp[w + 1];
-        for (int32_t i = b; i < f; ++i) {
-          const uint32_t u = (uint32_t)W.col[i];
-          const uint32_t c = sp_cell_of(W, W.pos[u]);
-          if (sp_cell_end(W, c) - c == 1) continue;
-          if (atomicAdd(&W.cnt[u], 1u) == 0) {
-            const uint32_t t = atomicAdd(&W.ntouched, 1u);
-            W.T[t] = u;
-            W.Tc[t] = c;
-            if (atomicAdd(&W.cellcnt[c], 1u) == 0) bm_set_atomic(W.tcb, W.tcbs, c);
+      lc = (lc ^ C) + len;
+    }
+    if (len > 1 && len <= 32) {
+      // the splitter's edges, lane by lane
+      uint32_t d = 0;
+      int32_t b = 0;
+      if (lane < len) {
+        const uint32_t w = R.elem[s + lane];
+        b = rp[w];
+        d = (uint32_t)(rp[w + 1] - b);
+      }
+      uint32_t incl = d;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(GCL_FULL, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+      }
+      const uint32_t D = __shfl_sync(GCL_FULL, incl, 31);
+      if (D <= 32) {
+        const uint32_t excl = incl - d;
+        const uint32_t nonempty = __ballot_sync(GCL_FULL, d > 0);
+        const uint32_t firsts = __reduce_or_sync(GCL_FULL, d > 0 ? 1u << excl : 0u);
+        // lane i < D: member = the k-th non-empty one, k = firsts up to lane i
+        const uint32_t kth = (uint32_t)__popc(firsts & (lt | (1u << lane)));
+        int src = 0;
+        if (lane < D)
+          src = (nonempty & (nonempty + 1)) == 0 ? (int)kth - 1 : (int)nth_bit(nonempty, kth - 1);
+        const int32_t bs = __shfl_sync(GCL_FULL, b, src);
+        const uint32_t es = __shfl_sync(GCL_FULL, excl, src);
+        uint32_t u = kNone, p = 0, c = kNone, L = 0;
+        if (lane < D) {
+          u = (uint32_t)col[bs + (int32_t)(lane - es)];
+          p = R.pos[u];
+          if (!shared_cell(p)) u = kNone;  // singleton cells never split (:257-259)
+        }
+        // lanes on the same neighbour: the group's size is its count
+        const uint32_t gu = __match_any_sync(GCL_FULL, u);
+        const uint32_t cnt = (uint32_t)__popc(gu);
+        const bool lead = u != kNone && lane == (uint32_t)(__ffs((int)gu) - 1);
+        if (lead) {
+          c = bm_prev(R.stb, R.sts, p);
+          L = bm_next(R.stb, R.sts, p + 1, n, nw, nsw) - c;
+        }
+        const uint32_t gc = __match_any_sync(GCL_FULL, c);
+        const uint32_t k = (uint32_t)__popc(gc);  // touched vertices of the cell
+        // rank by count within the cell: a radix pass over ballots
+        uint32_t peers = lead ? gc : 0u, less = 0;
+        const uint32_t top = __reduce_max_sync(GCL_FULL, lead ? cnt : 0u);
+        for (int bit = 31 - __clz((int)top); bit >= 0; --bit) {
+          const bool one = (cnt >> bit) & 1u;
+          const uint32_t m1 = __ballot_sync(GCL_FULL, lead && one);
+          if (one) {
+            less += (uint32_t)__popc(peers & ~m1);
+            peers &= m1;
+          } else {
+            peers &= ~m1;
           }
         }
+        const uint32_t eq = (uint32_t)__popc(peers & lt), size = (uint32_t)__popc(peers);
+        const bool uniform = lead && k == L && size == k;  // one common count: no split
+        const bool split = lead && !uniform;
+        const bool cell_lead = lead && lane == (uint32_t)(__ffs((int)gc) - 1);
+        const uint32_t R0 = c + (L - k), f = R0 + less;
+        uint32_t h = 0, x = 0, made = 0;
+        if (__any_sync(GCL_FULL, split)) {
+          // untouched vertices first, then ascending count: touched vertices go
+          // to R0 + rank, the untouched ones found in [R0, c + L) to the
+          // positions the touched ones leave
+          const bool in = p >= R0;
+          const bool frag = split && eq == 0;
+          const uint32_t rank = frag ? (size << 6) | (63u - less) : 0u;
+          uint32_t inner = 0, best = 0;
+          if (split) {
+            inner = __reduce_or_sync(gc, in ? 1u << (p - R0) : 0u);
+            best = __reduce_max_sync(gc, rank);
+          }
+          const uint32_t outs = __ballot_sync(GCL_FULL, split && !in) & gc;
+          const bool mv = split && !in;
+          if (mv) {
+            h = R0 + nth_bit(~inner & (k >= 32 ? 0xffffffffu : (1u << k) - 1u),
+                             (uint32_t)__popc(outs & lt));
+            x = R.elem[h];
+          }
+          const bool was = split && bm_test(R.act, c);
+          // the first largest fragment is the untouched one (it comes first)
+          const bool rest = L - k >= (best >> 6);
+          const bool fresh = frag && f != c;
+          const uint32_t fm = __ballot_sync(GCL_FULL, fresh);
+          made = (uint32_t)__popc(fm);
+          __syncwarp();
+          if (mv) {
+            R.elem[p] = (uint16_t)x;
+            R.pos[x] = (uint16_t)p;
+          }
+          if (split) {
+            R.elem[f + eq] = (uint16_t)u;
+            R.pos[u] = (uint16_t)(f + eq);
+          }
+          if (frag && (was ? f != c : rest || rank != best)) bm_or(R.act, R.acts, f);
+          if (cell_lead && split && L > k && !was && !rest) bm_or(R.act, R.acts, c);
+          if (fresh) slog[utop + (uint32_t)__popc(fm & lt)] = f;
+          const uint32_t hv = __reduce_max_sync(GCL_FULL, fresh && size == 1 ? f + 1 : 0u);
+          if (hv) hint = hv - 1;
+        }
+        const bool item = (uniform && cell_lead) || (split && eq == 0);
+        if (item) {
+          R.cnt[f] = (uint16_t)cnt;
+          or_bit32(R.itm, f);
+        }
+        __syncwarp();
+        lc = n <= 1024 ? sp_fold<kS, 1>(lc, false) : sp_fold<kS, 4>(lc, false);
+        __syncwarp();
+        if (item) {
+          R.cnt[f] = 0;
+          R.itm[f >> 5] = 0;
+          if (split && f != c) bm_or(R.stb, R.sts, f);
+        }
+        utop += made;
+        ncells += made;
+        nact += made;
+        __syncwarp();
+        continue;
       }
     }
     __syncwarp();
-    const uint32_t nt = W.ntouched;
-    // group the touched vertices by cell (counting sort, cells in order)
-    {
-      uint32_t run = 0;
-      uint32_t c = bm_next(W.tcb, W.tcbs, 0, n, nw, nsw);
-      while (c < n) {
-        const uint32_t k = W.cellcnt[c];
-        if (lane == 0) W.off[c] = run;
-        run += k;
-        c = bm_next(W.tcb, W.tcbs, c + 1, n, nw, nsw);
-      }
-      __syncwarp();
-      for (uint32_t i = lane; i < nt; i += 32) {
-        const uint32_t c2 = W.Tc[i];
-        W.G[W.off[c2] + atomicAdd(&W.fill[c2], 1u)] = W.T[i];
-      }
-      __syncwarp();
-    }
-
-    if (len == 1) {
-      // every touched cell that is not all neighbours splits into
-      // [neighbours, non-neighbours] (:296-309, 399-435)
-      uint32_t c = bm_next(W.tcb, W.tcbs, 0, n, nw, nsw);
-      while (c < n) {
-        const uint32_t k = W.cellcnt[c], ce = sp_cell_end(W, c), L = ce - c;
-        const uint32_t cnext = bm_next(W.tcb, W.tcbs, c + 1, n, nw, nsw);
-        if (k < L) {
-          sp_regroup(W.G + W.off[c], k, c, nullptr);
-          const uint32_t p = c + k;
-          lc = mash(lc, p - 1);
-          const bool was = bm_test(W.act, c);
-          if (lane == 0) {
-            add_start(W, p);
-            W.ncells += 1;
-            const uint32_t nb = k, nn = L - k;
-            if (was || nb >= nn) {
-              bm_set1(W.act, W.acts, p);
-              W.nact += 1;
-              if (nn == 1) hint = p;
-            } else {
-              if (!was) {
-                bm_set1(W.act, W.acts, c);
-                W.nact += 1;
-              }
-              if (nb == 1) hint = c;
-            }
-            W.hint = hint;
-          }
-          __syncwarp();
-          hint = W.hint;
-        }
-        c = cnext;
-      }
-    } else {
-      // every non-singleton cell in order: common count, or fragments in
-      // ascending count with the untouched (count 0) fragment first.  Cells
-      // are taken 32 at a time; untouched ones only hash their start.
-      const uint32_t K = sp_list_nonsingleton();
-      for (uint32_t i0 = 0; i0 < K; i0 += 32) {
-        const uint32_t il = i0 + lane;
-        const uint32_t cl = il < K ? W.nsl[il] : 0u;
-        const uint32_t tmask = __ballot_sync(GCL_FULL, il < K && bm_test(W.tcb, cl));
-        const uint32_t cnt32 = min(32u, K - i0);
-        if (!tmask) {  // 32 untouched cells: item = start
-          lc = mash_fold32(lc, cl, cnt32);
-          continue;
-        }
-        for (uint32_t jj = 0; jj < cnt32; ++jj) {
-          const uint32_t c = __shfl_sync(GCL_FULL, cl, (int)jj);
-          if (!((tmask >> jj) & 1u)) {
-            lc = mash(lc, c);  // every member has count 0
-            continue;
-          }
-          const uint32_t ce = sp_cell_end(W, c), L = ce - c;
-          const uint32_t k = W.cellcnt[c];
-          const uint32_t* seg = W.G + W.off[c];
-          uint32_t mn = 0xffffffffu, mx = 0;
-          for (uint32_t i = lane; i < k; i += 32) {
-            const uint32_t x = W.cnt[seg[i]];
-            mn = min(mn, x);
-            mx = max(mx, x);
-          }
-          mn = __reduce_min_sync(GCL_FULL, mn);
-          mx = __reduce_max_sync(GCL_FULL, mx);
-          if (k == L && mn == mx) {
-            lc = mash(lc, mn + c);
-            continue;
-          }
-          // counting sort of the touched vertices by count
-          const uint32_t range = mx - mn + 1;
-          for (uint32_t i = lane; i < range; i += 32) W.hist[i] = 0;
-          __syncwarp();
-          for (uint32_t i = lane; i < k; i += 32) atomicAdd(&W.hist[W.cnt[seg[i]] - mn], 1u);
-          __syncwarp();
-          if (lane == 0) {
-            uint32_t run = 0;
-            for (uint32_t i = 0; i < range; ++i) {
-              W.pre[i] = run;
-              run += W.hist[i];
-            }
-          }
-          __syncwarp();
-          for (uint32_t i = lane; i < k; i += 32) {
-            const uint32_t u = seg[i];
-            const uint32_t d = W.cnt[u] - mn;
-            W.tmp[atomicAdd(&W.pre[d], 1u)] = u;  // pre[d] ends at the fragment end
-          }
-          __syncwarp();
-          const uint32_t r0 = c + (L - k);
-          sp_regroup(seg, k, r0, W.tmp);
-          // fragments: hash, starts, active (:326-465)
-          const bool was = bm_test(W.act, c);
-          __syncwarp();
-          if (lane == 0) {
-            uint32_t maxsz = 0, maxf = c;
-            if (L > k) {  // untouched fragment first
-              lc = mash(lc, 0u + c);
-              maxsz = L - k;
-            }
-            uint32_t f = r0;
-            for (uint32_t i = 0; i < range; ++i) {
-              const uint32_t sz = W.hist[i];
-              if (!sz) continue;
-              lc = mash(lc, mn + i + f);
-              if (f != c) {
-                W.fpos[W.npend++] = f;  // set after the fold: the fold walks the old starts
-                W.ncells += 1;
-                if (!bm_test(W.act, f)) {
-                  bm_set1(W.act, W.acts, f);
-                  W.nact += 1;
-                }
-                if (sz == 1) hint = f;
-              }
-              if (sz > maxsz) {
-                maxsz = sz;
-                maxf = f;
-              }
-              f += sz;
-            }
-            if (!was) {
-              if (!bm_test(W.act, c)) {
-                bm_set1(W.act, W.acts, c);
-                W.nact += 1;
-              }
-              if (bm_test(W.act, maxf)) {
-                bm_clear1(W.act, W.acts, maxf);
-                W.nact -= 1;
-              }
-            }
-            W.lc = lc;
-            W.hint = hint;
-          }
-          __syncwarp();
-          lc = W.lc;
-          hint = W.hint;
-        }
-      }
-    }
-    // new starts of the non-singleton fold
-    __syncwarp();
-    if (lane == 0) {
-      for (uint32_t i = 0; i < W.npend; ++i) add_start(W, W.fpos[i]);
-      W.npend = 0;
-    }
-    // reset per-step scratch
-    __syncwarp();
-    for (uint32_t i = lane; i < nt; i += 32) {
-      const uint32_t u = W.T[i], c = W.Tc[i];
-      W.cnt[u] = 0;
-      W.cellcnt[c] = 0;
-      W.fill[c] = 0;
-      W.tcb[c >> 6] = 0;
-      W.tcbs[c >> 12] = 0;
-    }
-    __syncwarp();
-    ncells = W.ncells;
-    nact = W.nact;
-    utop = W.utop;
-  }
-  if (lane == 0) {
-    W.ncells = ncells;
-    W.utop = utop;
+    const SpStep st = sp_refine_general<kS>(s, e, lc, hint, utop);
+    lc = st.lc;
+    hint = st.hint;
+    utop += st.made;
+    ncells += st.made;
+    nact += st.made;
   }
   // clear what is left of the active set
   __syncwarp();
-  for (uint32_t w = lane; w < nw; w += 32) W.act[w] = 0;
-  for (uint32_t w = lane; w < nsw; w += 32) W.acts[w] = 0;
-  if (lane == 0) W.nact = 0;
+  for (uint32_t w = lane; w < nw; w += 32) R.act[w] = 0;
+  for (uint32_t w = lane; w < nsw; w += 32) R.acts[w] = 0;
+  if (lane == 0) {
+    W.ncells = ncells;
+    W.utop = utop;
+    W.nact = 0;
+  }
   __syncwarp();
   if (!ok) return -1;
-  return cleanup(mash(lc, W.ncells));
+  return cleanup(mash(lc & 077777u, ncells));
+}
+
+__device__ __forceinline__ int sp_refine() {
+  return sp_w().soff != kNone ? sp_refine_t<true>() : sp_refine_t<false>();
 }
 
 // split_by_and_refine's split (partition_refinement.cpp:486-528)
@@ -1062,11 +1078,8 @@ __device__ __forceinline__ uint32_t sp_first_nonsingleton() {
     uint64_t ns = 0;
     if (w < nw) {
       const uint64_t b = W.stb[w];
-      const uint64_t nb = (w + 1 < nw) ? W.stb[w + 1] : 0ull;
-      uint64_t succ = (b >> 1) | (nb << 63);  // bit p set: p+1 is a start
-      const uint32_t lastp = n - 1;
-      if ((lastp >> 6) == w) succ |= bit64(lastp & 63);  // the last position ends its cell
-      ns = b & ~succ;
+      ns = b & ~((b >> 1) | (W.stb[w + 1] << 63));  // starts whose successor is none
+      if (n - w * 64 < 64) ns &= low_mask(n - w * 64);  // position n is marked as a start
     }
     const uint32_t bal = __ballot_sync(GCL_FULL, ns != 0);
     if (bal) {
@@ -1267,6 +1280,17 @@ __device__ __forceinline__ void sp_store_aut(const uint32_t* label, uint16_t* ds
   __syncwarp();
 }
 
+// The refinement's scratch starts clear: no counts, marks or active cells.
+__device__ __forceinline__ void sp_clear_scratch() {
+  SpWarp& W = sp_w();
+  const uint32_t lane = lane_id();
+  for (uint32_t i = lane; i < W.n; i += 32) W.cnt[i] = 0;
+  for (uint32_t w = lane; w < 2 * W.nw; w += 32) W.itm[w] = 0;
+  for (uint32_t w = lane; w < W.nw; w += 32) W.act[w] = 0;
+  for (uint32_t w = lane; w < W.nsw; w += 32) W.acts[w] = 0;
+  __syncwarp();
+}
+
 // Colour partition (initializePartition_s, partition_refinement.cpp:28-68):
 // a stable LSD radix sort of the identity order by colour.
 __device__ __noinline__ void sp_init_partition(const int32_t* color) {
@@ -1318,24 +1342,14 @@ __device__ __noinline__ void sp_init_partition(const int32_t* color) {
     __syncwarp();
   }
   for (uint32_t i = lane; i < n; i += 32) W.pos[W.elem[i]] = i;
-  for (uint32_t w = lane; w < W.nw; w += 32) {
-    W.stb[w] = 0;
-    W.act[w] = 0;
-    W.tcb[w] = 0;
-  }
-  for (uint32_t i = lane; i < n; i += 32) {
-    W.cnt[i] = 0;
-    W.cellcnt[i] = 0;
-    W.fill[i] = 0;
-  }
-  __syncwarp();
+  for (uint32_t w = lane; w < W.nw; w += 32) W.stb[w] = 0;
+  sp_clear_scratch();
   // cell starts where the colour changes
   for (uint32_t i = lane; i < n; i += 32) {
     const bool st = i == 0 || (color && color[W.elem[i]] != color[W.elem[i - 1]]);
-    if (st) atomicOr((unsigned long long*)&W.stb[i >> 6], (unsigned long long)bit64(i & 63));
+    if (st) or_bit32((uint32_t*)W.stb, i);
   }
   __syncwarp();
-  bm_resummarize(W.stb, W.sts, W.nw, W.nsw);
   uint32_t cells = 0;
   for (uint32_t w = lane; w < W.nw; w += 32) cells += popc64(W.stb[w]);
   cells = __reduce_add_sync(GCL_FULL, cells);
@@ -1343,7 +1357,9 @@ __device__ __noinline__ void sp_init_partition(const int32_t* color) {
   for (uint32_t w = lane; w < W.nw; w += 32) W.act[w] = W.stb[w];
   __syncwarp();
   bm_resummarize(W.act, W.acts, W.nw, W.nsw);
-  for (uint32_t w = lane; w < W.nsw; w += 32) W.tcbs[w] = 0;
+  if (lane == 0) or_bit32((uint32_t*)W.stb, n);
+  __syncwarp();
+  bm_resummarize(W.stb, W.sts, W.nw, W.nsw);
   if (lane == 0) {
     W.ncells = cells;
     W.nact = cells;
@@ -1429,32 +1445,23 @@ __device__ __noinline__ void sp_bind(uint8_t* slot, const SpLayout& Lo, uint32_t
   if (lane_id() != 0) return;
   W.elem = (uint16_t*)(slot + Lo.elem);
   W.pos = (uint16_t*)(slot + Lo.pos);
+  W.cnt = (uint16_t*)(slot + Lo.cnt);
   // the n-sized u32 arrays
-  uint32_t* base[23];
-  for (int i = 0; i < 23; ++i) base[i] = (uint32_t*)(slot + Lo.u32n[i]);
+  uint32_t* base[13];
+  for (int i = 0; i < 13; ++i) base[i] = (uint32_t*)(slot + Lo.u32n[i]);
   W.slog = base[0];
   W.umark = base[1];
-  W.nsl = (uint16_t*)base[2];
-  W.cnt = base[3];
-  W.T = base[4];
-  W.Tc = base[5];
-  W.cellcnt = base[6];
-  W.off = base[7];
-  W.fill = base[8];
-  W.G = base[9];
-  W.tmp = base[10];
-  W.lst1 = base[11];
-  W.lst2 = base[12];
-  W.seq = base[13];
-  W.fseq = base[14];
-  W.bseq = base[15];
-  W.flabel = base[16];
-  W.blabel = base[17];
-  W.dsu = base[18];
-  W.hist = base[19];
-  W.pre = base[20];
-  W.fpos = base[21];
-  W.pathcode = (int32_t*)base[22];
+  W.tmp = base[2];
+  W.lst1 = base[3];
+  W.hist = base[4];
+  W.pre = base[5];
+  W.seq = base[6];
+  W.fseq = base[7];
+  W.bseq = base[8];
+  W.flabel = base[9];
+  W.blabel = base[10];
+  W.dsu = base[11];
+  W.pathcode = (int32_t*)base[12];
   W.fixst = (uint2*)(slot + Lo.fixst);
   W.fixcap = Lo.fixcap;
   W.utop = 0;
@@ -1465,8 +1472,8 @@ __device__ __noinline__ void sp_bind(uint8_t* slot, const SpLayout& Lo, uint32_t
   W.sts = (uint64_t*)(slot + Lo.sts);
   W.act = (uint64_t*)(slot + Lo.act);
   W.acts = (uint64_t*)(slot + Lo.acts);
-  W.tcb = (uint64_t*)(slot + Lo.tcb);
-  W.tcbs = (uint64_t*)(slot + Lo.tcbs);
+  W.itm = (uint32_t*)(slot + Lo.itm);
+  W.nsb = (uint32_t*)(slot + Lo.nsb);
   W.fcert = (uint32_t*)(slot + Lo.fcert);
   W.bcert = (uint32_t*)(slot + Lo.bcert);
   W.ccert = (uint32_t*)(slot + Lo.ccert);
@@ -1479,35 +1486,25 @@ __device__ __noinline__ void sp_bind(uint8_t* slot, const SpLayout& Lo, uint32_t
   W.nw = (n + 63) / 64 + 1;
   W.nsw = (W.nw + 63) / 64 + 1;
   W.stride = Lo.stride;
-  W.npend = 0;
+  W.soff = kNone;
   if (smem && sp_smem_bytes(n) <= smem_bytes) {
     // stage the per-step arrays in this warp's shared memory
-    const uint64_t a = (((uint64_t)n + 2) * 2u + 15) & ~15ull;
-    const uint32_t nw2 = W.nw, nsw2 = W.nsw;
-    uint8_t* q = smem;
-    W.elem = (uint16_t*)q;
-    q += a;
-    W.pos = (uint16_t*)q;
-    q += a;
-    W.nsl = (uint16_t*)q;
-    q += a;
-    W.stb = (uint64_t*)q;
-    q += 8 * nw2;
-    W.sts = (uint64_t*)q;
-    q += 8 * nsw2;
-    W.act = (uint64_t*)q;
-    q += 8 * nw2;
-    W.acts = (uint64_t*)q;
-    q += 8 * nsw2;
-    W.tcb = (uint64_t*)q;
-    q += 8 * nw2;
-    W.tcbs = (uint64_t*)q;
+    const SpStage G = sp_stage(n);
+    W.soff = (uint32_t)(smem - sp_dyn);
+    W.elem = (uint16_t*)smem;
+    W.pos = (uint16_t*)(smem + G.pos);
+    W.cnt = (uint16_t*)(smem + G.cnt);
+    W.stb = (uint64_t*)(smem + G.stb);
+    W.sts = (uint64_t*)(smem + G.sts);
+    W.act = (uint64_t*)(smem + G.act);
+    W.acts = (uint64_t*)(smem + G.acts);
+    W.itm = (uint32_t*)(smem + G.itm);
+    W.nsb = (uint32_t*)(smem + G.nsb);
   }
   W.pool_top = 0;
   W.pool_cap = pool;
   W.aut_cap = cap;
   W.max_aut = max_aut;
-  W.ntouched = 0;
 }
 
 __device__ __noinline__ SpResult sp_search(const BatchArgs& A, int g, uint8_t* slot,

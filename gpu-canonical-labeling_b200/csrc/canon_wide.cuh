@@ -896,9 +896,10 @@ __device__ __noinline__ void wide_load_node(const WidePtrs& P, uint32_t L) {
   uint32_t cells = 0;
   for (uint32_t w = 0; w < W.nw; ++w) {
     const uint32_t p0 = w * 64 + lane, p1 = p0 + 32;
-    const uint64_t b = P.lstb[w] & ballot2(p0 < n && P.linlev[p0] <= L, p1 < n && P.linlev[p1] <= L);
-    if (lane == 0) W.stb[w] = b;
+    uint64_t b = P.lstb[w] & ballot2(p0 < n && P.linlev[p0] <= L, p1 < n && P.linlev[p1] <= L);
     cells += popc64(b);
+    if (n >> 6 == w) b |= bit64(n & 63);  // position n is marked as a start
+    if (lane == 0) W.stb[w] = b;
   }
   __syncwarp();
   bm_resummarize(W.stb, W.sts, W.nw, W.nsw);
@@ -1016,7 +1017,6 @@ __device__ __noinline__ uint32_t wide_gift_orbit_min(const WidePtrs& P, uint32_t
 
 template <bool kShare, bool kCount>
 __global__ void __launch_bounds__(kSpThreads) wide_items_kernel(WideArgs A) {
-  extern __shared__ __align__(16) uint8_t sp_dyn[];
   const int warp = (int)(threadIdx.x >> 5);
   const uint32_t lane = lane_id();
   const WidePtrs P = wide_ptrs(A);
@@ -1039,27 +1039,13 @@ __global__ void __launch_bounds__(kSpThreads) wide_items_kernel(WideArgs A) {
     W.auts = P.auts;
     W.stride = A.WL.stride;
     W.nact = 0;
-    W.ntouched = 0;
   }
   __syncwarp();
   // the per-step scratch starts clear; set up once the warp has work (a
   // grid has more warps than most searches have items)
   bool ready = false;
   auto setup = [&] {
-    for (uint32_t i = lane; i < n; i += 32) {
-      W.cnt[i] = 0;
-      W.cellcnt[i] = 0;
-      W.fill[i] = 0;
-    }
-    for (uint32_t w = lane; w < W.nw; w += 32) {
-      W.act[w] = 0;
-      W.tcb[w] = 0;
-    }
-    for (uint32_t w = lane; w < W.nsw; w += 32) {
-      W.acts[w] = 0;
-      W.tcbs[w] = 0;
-    }
-    __syncwarp();
+    sp_clear_scratch();
     ready = true;
   };
   const uint64_t deadline = A.budget_ns ? H->t0 + A.budget_ns : 0;

@@ -143,7 +143,6 @@ __global__ void __launch_bounds__(kSpThreads, 5)
     sp_batch_kernel(BatchArgs A, const int* list, const int* count, int* next, int* fail_list,
                     int* fail_count, uint32_t n_max, uint64_t m2_max, uint32_t pool, uint32_t cap,
                     uint64_t slot_bytes, uint64_t smem_per_warp) {
-  extern __shared__ __align__(16) uint8_t sp_dyn[];
   const int warp = (int)(threadIdx.x >> 5);
   const uint32_t lane = lane_id();
   uint8_t* slot = A.work + ((uint64_t)blockIdx.x * kSpWarps + (uint64_t)warp) * slot_bytes;
