@@ -18,9 +18,10 @@
 //     exactly like the upper-triangle compare (sequential.cpp:114-124);
 //   * the target cell of a level is not stored: when the search is back at
 //     that level the partition is the same, so its members are the cell at
-//     the stored start position; orbit representatives live in a small
-//     stack of per-level arrays that are only allocated when orbits are
-//     first computed at a level.
+//     the stored start position; orbit representatives live in a stack with
+//     an entry per member, pushed when orbits first change at a level.  (With
+//     an array of n per level, trees of more than 32 levels outgrew the first
+//     pass and were searched twice: 45 of 48 trees of 257 to 1,000 vertices.)
 //
 // All state lives in a per-warp slot of device memory; the warp's pointers
 // and scalars live in shared memory.  Each phase is one non-inlined function.
@@ -47,28 +48,30 @@ constexpr uint32_t kNone = 0xffffffffu;
 struct SpTc {
   uint32_t first, len, counter;
   int32_t last;   // last_num_aut_at_level
-  int32_t rslot;  // slot of this level's representatives, -1 = all v are reps
+  uint32_t rslot;  // this level's representatives in W.reps, kNone = all v are reps
   uint32_t pad;
 };
 
 // Byte layout of one slot for graphs with at most n vertices and m2 CSR
-// entries, `pool` per-level representative arrays and `cap` ring slots.
+// entries, representatives of `pool` target cells of n vertices (a target
+// cell takes as many entries as it has vertices, so sparse searches reach far
+// deeper), `cap` ring slots, and the fix state of `fixcap` entries of a shared
+// store.
 struct SpLayout {
   uint64_t u32n[13];  // offsets of the n-sized u32 arrays
   uint64_t elem, pos, cnt;
   uint64_t fcode, ccode, pool_owner;
   uint64_t stb, sts, act, acts, itm, nsb;
   uint64_t fcert, bcert, ccert;
-  uint64_t tc, reps, auts, fixst;
-  uint32_t fixcap;
+  uint64_t tc, reps, auts, fixm, fixst;
+  uint32_t fixcap, reps_cap;
   uint64_t bytes;
   uint32_t nw, nsw;
   uint32_t stride;  // elements per representative array / ring entry
 };
 
 __host__ __device__ inline SpLayout sp_layout(uint32_t n, uint64_t m2, uint32_t pool,
-                                              uint32_t cap, uint32_t fixcap = 0xffffffffu) {
-  if (fixcap == 0xffffffffu) fixcap = cap;
+                                              uint32_t cap, uint32_t fixcap = 0) {
   SpLayout L{};
   uint64_t o = 0;
   auto take = [&](uint64_t bytes) {
@@ -85,7 +88,7 @@ __host__ __device__ inline SpLayout sp_layout(uint32_t n, uint64_t m2, uint32_t 
   L.cnt = take(2 * N1);
   L.fcode = take(4 * (N1 + 1));
   L.ccode = take(4 * (N1 + 1));
-  L.pool_owner = take(4 * ((uint64_t)pool + 1));
+  L.pool_owner = take(4 * N1);
   L.nw = (n + 63) / 64 + 1;
   L.nsw = (L.nw + 63) / 64 + 1;
   L.stb = take(8ull * L.nw);
@@ -98,8 +101,13 @@ __host__ __device__ inline SpLayout sp_layout(uint32_t n, uint64_t m2, uint32_t 
   L.bcert = take(4 * (m2 + 1));
   L.ccert = take(4 * (m2 + 1));
   L.tc = take(sizeof(SpTc) * N1);
-  L.reps = take(4ull * pool * N1);
+  // the target cells of a path, each a part of the one before or of the rest,
+  // have at most n + (n - 1) + ... vertices
+  const uint64_t all = N1 * (N1 + 1) / 2;
+  L.reps_cap = (uint32_t)(pool * N1 < all ? pool * N1 : all);
+  L.reps = take(4ull * L.reps_cap);
   L.auts = take(2ull * cap * N1);
+  L.fixm = take(4ull * ((cap + 31) / 32) * N1);
   L.fixcap = fixcap;
   L.fixst = take(8ull * fixcap);
   L.bytes = o;
@@ -143,14 +151,18 @@ struct SpWarp {
                     // position of seq it moves or kNone}, valid for the path
   uint64_t *stb, *sts, *act, *acts;  // cell starts (position n too) and active cells
   uint32_t *itm, *nsb;  // marks of the hash: touched fragments, fragment starts
-  uint32_t *fcert, *bcert, *ccert, *reps;
+  uint32_t *fcert, *bcert, *ccert;
+  uint32_t* reps;   // stack of target cells' {vertex, representative << 16}
+  uint32_t* fixm;   // per vertex: a bit per ring entry that fixes it
+  uint32_t fixw;    // words of a vertex's row in fixm
   SpTc* tc;
   uint16_t* auts;
   const int32_t* rp;
   const int32_t* col;
   uint32_t n, nw, nsw, stride;  // stride: elements per pool / ring entry
   uint32_t ncells, nact;
-  uint32_t pool_top, pool_cap, aut_cap, max_aut;
+  uint32_t pool_top, pool_frames, pool_cap, aut_cap, max_aut;
+  uint32_t scr[32];  // a word per lane: the union-find of a small target cell
   uint32_t utop;  // entries of slog
   uint32_t fixcap;  // store entries whose fix state is kept (later ones are checked in full)
 };
@@ -1097,13 +1109,32 @@ __device__ __forceinline__ uint32_t sp_first_nonsingleton() {
 __device__ __forceinline__ uint32_t sp_next_rep(const SpTc& t) {
   SpWarp& W = sp_w();
   const uint32_t lane = lane_id();
-  const uint32_t* reps = t.rslot >= 0 ? W.reps + (uint64_t)t.rslot * W.stride : nullptr;
   uint32_t best = kNone;
-  for (uint32_t q = t.first + lane; q < t.first + t.len; q += 32) {
-    const uint32_t v = W.elem[q];
-    if (v >= t.counter && v < best && (!reps || reps[v] == v)) best = v;
+  if (t.rslot == kNone) {
+    for (uint32_t q = t.first + lane; q < t.first + t.len; q += 32) {
+      const uint32_t v = W.elem[q];
+      if (v >= t.counter) best = min(best, v);
+    }
+  } else {
+    for (uint32_t i = lane; i < t.len; i += 32) {
+      const uint32_t x = W.reps[t.rslot + i], v = x & 0xffffu;
+      if (v >= t.counter && (x >> 16) == v) best = min(best, v);
+    }
   }
   return __reduce_min_sync(GCL_FULL, best);
+}
+
+// The representatives of levels Lv and deeper are dropped (after a backtrack
+// to level Lv; their target-cell headers are still in place).
+__device__ __forceinline__ void sp_pool_pop(uint32_t Lv) {
+  SpWarp& W = sp_w();
+  __syncwarp();
+  if (lane_id() == 0) {
+    uint32_t f = W.pool_frames;
+    while (f > 0 && W.pool_owner[f - 1] >= (int32_t)Lv) W.pool_top = W.tc[W.pool_owner[--f]].rslot;
+    W.pool_frames = f;
+  }
+  __syncwarp();
 }
 
 __device__ __forceinline__ uint32_t sp_find(volatile uint32_t* d, uint32_t x, uint32_t n) {
@@ -1149,111 +1180,224 @@ __device__ __forceinline__ bool sp_dsu_apply(const uint16_t* pm, const T* member
   }
 }
 
+// The orbits of a target cell of at most 32 vertices, a lane per vertex: a
+// component is named by its least lane.
+struct SpCellOrbits {
+  uint32_t v, comp;  // the lane's vertex (kNone past the cell) and its component
+};
+
+// Merge the orbits of one automorphism, whose image of the lane's vertex lies
+// at index j of the cell (j == lane past it).
+__device__ __forceinline__ void sp_cell_merge(SpCellOrbits& o, uint32_t j) {
+  SpWarp& W = sp_w();
+  const uint32_t lane = lane_id();
+  while (true) {  // every round with an open edge removes a component
+    const uint32_t cj = __shfl_sync(GCL_FULL, o.comp, (int)j);
+    const bool d = cj != o.comp;
+    if (!__any_sync(GCL_FULL, d)) return;
+    W.scr[lane] = lane;
+    __syncwarp();
+    if (d) atomicMin(&W.scr[max(o.comp, cj)], min(o.comp, cj));
+    __syncwarp();
+    bool moved;
+    do {  // to the root (links go to smaller lanes)
+      const uint32_t r = W.scr[o.comp];
+      moved = r != o.comp;
+      o.comp = r;
+    } while (__any_sync(GCL_FULL, moved));
+    __syncwarp();
+  }
+}
+
 // subgroup_fixing_sequence + compute_orbits_fast (perm_group.cpp:5-116).
 // The reference unites v with aut[v] over all vertices; an automorphism that
 // fixes the sequence maps the node's partition onto itself, cell by cell, so
 // the orbits that meet the target cell lie inside it and are found by
 // uniting over the cell's members alone (O(cell) per automorphism instead of
 // O(n)); the least vertex of each orbit -- the representative -- is the same.
+//
+// The ring's search (kCg false) keeps a bit per vertex and entry that says
+// whether the entry fixes the vertex, so the entries that fix the sequence and
+// move a member of the cell are the and of the sequence's rows without the and
+// of the cell's: a few independent loads, where testing every entry along the
+// sequence took a chain of dependent ones (10,400 to 13,700 cycles a node, 40
+// to 47% of the time, on trees of 65 to 1,000 vertices).  An entry that moves
+// no member changes nothing.  Cells of up to 32 vertices -- all but the
+// largest -- are merged in registers.
+//
+// Returns kOk, kAutOverflow (no room for the representatives) or kInternal.
 template <bool kCg = false>
-__device__ __forceinline__ bool sp_orbits(int idx, int num_aut, uint32_t seqlen) {
+__device__ __noinline__ int32_t sp_orbits(int idx, int num_aut, uint32_t seqlen) {
   SpWarp& W = sp_w();
   const uint32_t lane = lane_id();
   const uint32_t n = W.n;
   SpTc t = W.tc[idx];
   const int limit = num_aut < (int)W.max_aut ? num_aut : (int)W.max_aut;
   const int from = t.last == -1 ? 0 : t.last;
+  const bool small = t.len <= 32;
   volatile uint32_t* dsu = W.dsu;
-  const uint32_t* reps = t.rslot >= 0 ? W.reps + (uint64_t)t.rslot * W.stride : nullptr;
   const uint16_t* mem = W.elem + t.first;
-  for (uint32_t i = lane; i < t.len; i += 32) {
-    const uint32_t v = mem[i];
-    dsu[v] = reps ? reps[v] : v;
-  }
-  __syncwarp();
   bool any = false;
-  // the store entries that fix the sequence, 32 at a time (one per lane),
-  // each batch merged in one union-find pass over (entry, member) pairs
-  for (int base = from; base < limit; base += 32) {
-    const int a = base + (int)lane;
-    bool fix = a < limit;
-    if (fix) {
-      // extend what is known about entry a along the current sequence: the
-      // prefix it fixes and the first position it moves stay valid until a
-      // backtrack shortens the sequence below them (sp_fix_clamp)
-      const bool kept = (uint32_t)a < W.fixcap;
-      uint2 st = kept ? W.fixst[a] : make_uint2(0u, kNone);
-      if (st.y != kNone && st.y < seqlen) {
-        fix = false;
-      } else {
-        const uint16_t* pa = W.auts + (uint64_t)a * W.stride;
-        uint32_t j = st.x;
-        for (; j < seqlen; ++j) {
-          const uint32_t sv = W.seq[j];
-          if (ldx<kCg>(pa + sv) != sv) break;
+  SpCellOrbits o{kNone, lane};
+  // the cell's orbits so far
+  auto begin = [&] {
+    if (small) {
+      if (lane < t.len) o.v = mem[lane];
+      if (t.rslot != kNone) {
+        // the list is keyed by vertex: its order is that of its last writing
+        uint32_t rep = kNone - lane;
+        if (lane < t.len) {
+          const uint32_t x = W.reps[t.rslot + lane];
+          W.scr[W.pos[x & 0xffffu] - t.first] = x >> 16;
         }
-        fix = j >= seqlen;
-        st.x = j;
-        st.y = fix ? kNone : j;
-        if (kept) W.fixst[a] = st;
+        __syncwarp();
+        if (lane < t.len) rep = W.scr[lane];
+        o.comp = (uint32_t)__ffs((int)__match_any_sync(GCL_FULL, rep)) - 1;
+        __syncwarp();
       }
+      return;
     }
-    const uint32_t fm = __ballot_sync(GCL_FULL, fix);
-    if (!fm) continue;
+    for (uint32_t i = lane; i < t.len; i += 32) {
+      const uint32_t x = t.rslot != kNone ? W.reps[t.rslot + i] : mem[i] * 0x10001u;
+      dsu[x & 0xffffu] = x >> 16;
+    }
+    __syncwarp();
+  };
+  // the entries base + i, i a bit of m: kInternal if one does not map the cell
+  // onto itself
+  auto merge = [&](uint32_t base, uint32_t m) -> int32_t {
+    if (!any) begin();
     any = true;
-    const uint32_t nf = (uint32_t)__popc(fm);
-    // the cell must map onto itself (a failed check is an internal error)
-    bool out = false;
-    for (uint32_t x = lane; x < nf * t.len; x += 32) {
-      const uint32_t which = (uint32_t)__fns(fm, 0, (int)(x / t.len) + 1);
-      const uint16_t* pm = W.auts + (uint64_t)(base + (int)which) * W.stride;
-      const uint32_t q = W.pos[ldx<kCg>(pm + mem[x % t.len])];
-      out |= q < t.first || q >= t.first + t.len;
+    if (small) {
+      while (m) {
+        // up to four entries' images at once, so their loads overlap
+        uint32_t j[4], cnt = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          j[k] = lane;
+          if (!m) continue;
+          const uint16_t* pm = W.auts + (uint64_t)(base + (uint32_t)__ffs((int)m) - 1) * W.stride;
+          m &= m - 1;
+          ++cnt;
+          if (lane < t.len) j[k] = ldx<kCg>(pm + o.v);
+        }
+        bool out = false;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if ((uint32_t)k < cnt && lane < t.len) {
+            j[k] = (uint32_t)W.pos[j[k]] - t.first;
+            out |= j[k] >= t.len;
+          }
+        if (__any_sync(GCL_FULL, out)) return kInternal;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if ((uint32_t)k < cnt) sp_cell_merge(o, j[k]);
+      }
+      return kOk;
     }
-    if (__any_sync(GCL_FULL, out)) return false;
-    for (uint32_t round = 0;; ++round) {
-      if (round > t.len + 1) return false;
-      bool changed = false;
-      for (uint32_t x = lane; x < nf * t.len; x += 32) {
-        const uint32_t which = (uint32_t)__fns(fm, 0, (int)(x / t.len) + 1);
-        const uint16_t* pm = W.auts + (uint64_t)(base + (int)which) * W.stride;
-        const uint32_t v = mem[x % t.len];
-        const uint32_t img = ldx<kCg>(pm + v);
-        if (img == v) continue;
-        const uint32_t ra = sp_find(dsu, v, n), rb = sp_find(dsu, img, n);
-        if (ra != rb) {
-          atomicMin((uint32_t*)&dsu[max(ra, rb)], min(ra, rb));
-          changed = true;
+    for (; m; m &= m - 1) {
+      const uint16_t* pm = W.auts + (uint64_t)(base + (uint32_t)__ffs((int)m) - 1) * W.stride;
+      bool out = false;
+      for (uint32_t i = lane; i < t.len; i += 32) {
+        const uint32_t q = W.pos[ldx<kCg>(pm + mem[i])];
+        out |= q < t.first || q >= t.first + t.len;
+      }
+      if (__any_sync(GCL_FULL, out)) return kInternal;
+      if (!sp_dsu_apply<kCg>(pm, mem, t.len, n)) return kInternal;
+    }
+    return kOk;
+  };
+  if constexpr (kCg) {
+    // the store entries that fix the sequence, one per lane at a time
+    for (int base = from; base < limit; base += 32) {
+      const int a = base + (int)lane;
+      bool fix = a < limit;
+      if (fix) {
+        // extend what is known about entry a along the current sequence: the
+        // prefix it fixes and the first position it moves stay valid until a
+        // backtrack shortens the sequence below them (sp_fix_clamp)
+        const bool kept = (uint32_t)a < W.fixcap;
+        uint2 st = kept ? W.fixst[a] : make_uint2(0u, kNone);
+        if (st.y != kNone && st.y < seqlen) {
+          fix = false;
+        } else {
+          const uint16_t* pa = W.auts + (uint64_t)a * W.stride;
+          uint32_t j = st.x;
+          for (; j < seqlen; ++j) {
+            const uint32_t sv = W.seq[j];
+            if (ldx<kCg>(pa + sv) != sv) break;
+          }
+          fix = j >= seqlen;
+          st.x = j;
+          st.y = fix ? kNone : j;
+          if (kept) W.fixst[a] = st;
         }
       }
-      __syncwarp();
-      for (uint32_t i = lane; i < t.len; i += 32) {
-        const uint32_t v = mem[i];
-        atomicMin((uint32_t*)&dsu[v], sp_find(dsu, v, n));
+      const uint32_t fm = __ballot_sync(GCL_FULL, fix);
+      if (!fm) continue;
+      const int32_t st = merge((uint32_t)base, fm);
+      if (st != kOk) return st;
+    }
+  } else if (from < limit) {
+    // the entries' words [w0, w1], up to 32 at a time: `per` lanes (a power of
+    // two) take a row's words, the other lanes further rows
+    const uint32_t w0 = (uint32_t)from / 32, w1 = (uint32_t)(limit - 1) / 32;
+    for (uint32_t wb = w0; wb <= w1; wb += 32) {
+      const uint32_t nwd = min(32u, w1 - wb + 1);
+      const uint32_t per = nwd <= 1 ? 1u : 1u << (32 - __clz((int)nwd - 1));
+      const uint32_t wl = lane & (per - 1), row = lane / per, rows = 32 / per;
+      uint32_t fs = 0xffffffffu, fc = 0xffffffffu;
+      if (wl < nwd) {
+        const uint32_t* F = W.fixm + wb + wl;
+        const uint64_t fw = W.fixw;
+#pragma unroll 4
+        for (uint32_t j = row; j < seqlen; j += rows) fs &= F[W.seq[j] * fw];
+#pragma unroll 4
+        for (uint32_t i = row; i < t.len; i += rows) fc &= F[mem[i] * fw];
       }
-      __syncwarp();
-      if (!__any_sync(GCL_FULL, changed)) break;
+      for (uint32_t d = per; d < 32; d <<= 1) {
+        fs &= __shfl_xor_sync(GCL_FULL, fs, (int)d);
+        fc &= __shfl_xor_sync(GCL_FULL, fc, (int)d);
+      }
+      uint32_t sel = 0;
+      if (lane < nwd) {
+        const int b = (int)(wb + lane) * 32;  // entries b .. b + 31, those in [from, limit)
+        sel = fs & ~fc;
+        if (b < from) sel &= 0xffffffffu << (from - b);
+        if (limit - b < 32) sel &= (1u << (limit - b)) - 1u;
+      }
+      for (uint32_t m = __ballot_sync(GCL_FULL, sel != 0); m; m &= m - 1) {
+        const int src = __ffs((int)m) - 1;
+        const int32_t st = merge((wb + (uint32_t)src) * 32, __shfl_sync(GCL_FULL, sel, src));
+        if (st != kOk) return st;
+      }
     }
   }
-  if (!any) return true;
-  if (t.rslot < 0) {
-    if (W.pool_top >= W.pool_cap) return false;  // caller reports overflow
-    t.rslot = (int32_t)W.pool_top;
+  if (!any) return kOk;
+  if (t.rslot == kNone) {
+    if (W.pool_top + t.len > W.pool_cap) return kAutOverflow;
+    t.rslot = W.pool_top;
     __syncwarp();
     if (lane == 0) {
-      W.pool_owner[W.pool_top] = idx;
-      W.pool_top += 1;
+      W.pool_owner[W.pool_frames++] = idx;
+      W.pool_top += t.len;
       W.tc[idx].rslot = t.rslot;
     }
     __syncwarp();
   }
-  uint32_t* rw = W.reps + (uint64_t)t.rslot * W.stride;
-  for (uint32_t i = lane; i < t.len; i += 32) {
-    const uint32_t v = mem[i];
-    rw[v] = sp_find(dsu, v, n);
+  uint32_t* rw = W.reps + t.rslot;
+  if (small) {
+    const uint32_t g = __match_any_sync(GCL_FULL, o.comp);
+    const uint32_t r = __reduce_min_sync(g, o.v);
+    if (lane < t.len) rw[lane] = o.v | (r << 16);
+  } else {
+    for (uint32_t i = lane; i < t.len; i += 32) {
+      const uint32_t v = mem[i];
+      rw[i] = v | (sp_find(dsu, v, n) << 16);
+    }
   }
   __syncwarp();
-  return true;
+  return kOk;
 }
 
 // After a backtrack to sequence length s: positions >= s of the sequence
@@ -1272,11 +1416,19 @@ __device__ __forceinline__ void sp_fix_clamp(uint32_t s, uint32_t count) {
   __syncwarp();
 }
 
-// aut[label[j]] = elem[j] (sequential.cpp:505-520, 544-555)
-__device__ __forceinline__ void sp_store_aut(const uint32_t* label, uint16_t* dst) {
+// Ring entry si := aut[label[j]] = elem[j] (sequential.cpp:505-520, 544-555),
+// with its bit of every vertex it fixes.
+__device__ __forceinline__ void sp_store_aut(const uint32_t* label, uint32_t si) {
   SpWarp& W = sp_w();
   const uint32_t lane = lane_id();
-  for (uint32_t j = lane; j < W.n; j += 32) dst[label[j]] = (uint16_t)W.elem[j];
+  uint16_t* dst = W.auts + (uint64_t)si * W.stride;
+  const uint32_t bit = 1u << (si & 31u);
+  for (uint32_t j = lane; j < W.n; j += 32) {
+    const uint32_t v = label[j], img = W.elem[j];
+    dst[v] = (uint16_t)img;
+    uint32_t* f = W.fixm + (uint64_t)v * W.fixw + si / 32;
+    *f = v == img ? *f | bit : *f & ~bit;
+  }
   __syncwarp();
 }
 
@@ -1415,20 +1567,6 @@ __device__ __noinline__ bool sp_check_input(int64_t m) {
   return !__any_sync(GCL_FULL, bad);
 }
 
-struct SpArgs {
-  BatchArgs A;
-  const int* list;   // graph ids to process
-  const int* count;  // number of ids (device)
-  int* next;         // work counter
-  int* fail_list;    // graphs needing the rerun pass
-  int* fail_count;
-  uint32_t n_max;
-  uint64_t m2_max;
-  uint32_t pool;
-  uint32_t cap;
-  uint64_t slot_bytes;
-};
-
 struct SpResult {
   int32_t status;
   int num_aut;
@@ -1439,8 +1577,7 @@ struct SpResult {
 // the per-step arrays fit there).  Lane 0 writes; the caller syncs the warp.
 __device__ __noinline__ void sp_bind(uint8_t* slot, const SpLayout& Lo, uint32_t n,
                                      const int32_t* rp, const int32_t* col, uint8_t* smem,
-                                     uint64_t smem_bytes, uint32_t pool, uint32_t cap,
-                                     uint32_t max_aut) {
+                                     uint64_t smem_bytes, uint32_t cap, uint32_t max_aut) {
   SpWarp& W = sp_w();
   if (lane_id() != 0) return;
   W.elem = (uint16_t*)(slot + Lo.elem);
@@ -1462,6 +1599,8 @@ __device__ __noinline__ void sp_bind(uint8_t* slot, const SpLayout& Lo, uint32_t
   W.blabel = base[10];
   W.dsu = base[11];
   W.pathcode = (int32_t*)base[12];
+  W.fixm = (uint32_t*)(slot + Lo.fixm);
+  W.fixw = (cap + 31) / 32;
   W.fixst = (uint2*)(slot + Lo.fixst);
   W.fixcap = Lo.fixcap;
   W.utop = 0;
@@ -1502,14 +1641,15 @@ __device__ __noinline__ void sp_bind(uint8_t* slot, const SpLayout& Lo, uint32_t
     W.nsb = (uint32_t*)(smem + G.nsb);
   }
   W.pool_top = 0;
-  W.pool_cap = pool;
+  W.pool_frames = 0;
+  W.pool_cap = Lo.reps_cap;
   W.aut_cap = cap;
   W.max_aut = max_aut;
 }
 
 __device__ __noinline__ SpResult sp_search(const BatchArgs& A, int g, uint8_t* slot,
-                                           const SpLayout& Lo, uint32_t pool, uint32_t cap,
-                                           uint8_t* smem, uint64_t smem_bytes) {
+                                           const SpLayout& Lo, uint32_t cap, uint8_t* smem,
+                                           uint64_t smem_bytes) {
   SpWarp& W = sp_w();
   const uint32_t lane = lane_id();
   const int64_t vo = A.voff[g];
@@ -1518,7 +1658,7 @@ __device__ __noinline__ SpResult sp_search(const BatchArgs& A, int g, uint8_t* s
   const int64_t m = A.eoff[g + 1] - eo;
   SpResult res{kOk, 0, 1};
   if (n == 0) return res;
-  sp_bind(slot, Lo, n, A.rowptr + vo + g, A.col + eo, smem, smem_bytes, pool, cap, A.max_aut);
+  sp_bind(slot, Lo, n, A.rowptr + vo + g, A.col + eo, smem, smem_bytes, cap, A.max_aut);
   __syncwarp();
   if (!sp_check_input(m)) {
     res.status = kBadInput;
@@ -1595,7 +1735,7 @@ __device__ __noinline__ SpResult sp_search(const BatchArgs& A, int g, uint8_t* s
           h.len = sp_cell_end(W, t) - t;
           h.counter = 0;
           h.last = 0;
-          h.rslot = -1;
+          h.rslot = kNone;
           h.pad = 0;
           W.tc[tcl] = h;
         }
@@ -1618,7 +1758,7 @@ __device__ __noinline__ SpResult sp_search(const BatchArgs& A, int g, uint8_t* s
             h.len = sp_cell_end(W, t) - t;
             h.counter = 0;
             h.last = 0;
-            h.rslot = -1;
+            h.rslot = kNone;
             h.pad = 0;
             W.tc[tcl] = h;
           }
@@ -1631,10 +1771,8 @@ __device__ __noinline__ SpResult sp_search(const BatchArgs& A, int g, uint8_t* s
           classify = false;
         } else {
           if (num_aut > 0 && num_aut > W.tc[idx].last) {
-            if (!sp_orbits(idx, num_aut, seqlen)) {
-              status = W.pool_top >= W.pool_cap ? kAutOverflow : kInternal;
-              break;
-            }
+            status = sp_orbits(idx, num_aut, seqlen);
+            if (status != kOk) break;
             __syncwarp();
             if (lane == 0) W.tc[idx].last = num_aut;
             __syncwarp();
@@ -1722,9 +1860,7 @@ __device__ __noinline__ SpResult sp_search(const BatchArgs& A, int g, uint8_t* s
           status = kAutOverflow;
           break;
         }
-        sp_store_aut(dec == 1 ? W.flabel : W.blabel, W.auts + (uint64_t)si * W.stride);
-        if (lane == 0 && si < W.fixcap) W.fixst[si] = make_uint2(0u, kNone);
-        __syncwarp();
+        sp_store_aut(dec == 1 ? W.flabel : W.blabel, si);
         ++num_aut;
         const int gg = dec == 1 ? sp_gca(W.fseq, first_seqlen, seqlen)
                                 : sp_gca(W.bseq, best_seqlen, seqlen);
@@ -1762,12 +1898,7 @@ __device__ __noinline__ SpResult sp_search(const BatchArgs& A, int g, uint8_t* s
       seqlen = Lv - 1;
       tcl = (int)Lv;
       level = Lv;
-      sp_fix_clamp(seqlen, (uint32_t)min(num_aut, (int)W.max_aut));
-      // representative arrays of levels deeper than Lv are free again
-      __syncwarp();
-      if (lane == 0)
-        while (W.pool_top > 0 && W.pool_owner[W.pool_top - 1] >= (int32_t)Lv) W.pool_top -= 1;
-      __syncwarp();
+      sp_pool_pop(Lv);
     }
   }
   res.status = status;

@@ -181,7 +181,6 @@ struct WideArgs {
   uint8_t* slots;  // per-warp workspace
   SpLayout Lo;
   uint64_t slot_bytes;
-  uint32_t pool;
   uint32_t gate;  // level gate: 1 on (a level's items wait for the deeper ones), 0 off, 2 auto
   uint32_t probe;  // under the gate: a level's first item runs before the rest of the level
   uint64_t smem_per_warp;
@@ -264,7 +263,7 @@ __global__ void __launch_bounds__(32) wide_first_kernel(WideArgs A) {
     H->nodes = 1;
     H->t0 = global_ns();
   }
-  sp_bind(A.slots, A.Lo, n, A.rp, A.col, nullptr, 0, A.pool, 0, 1);
+  sp_bind(A.slots, A.Lo, n, A.rp, A.col, nullptr, 0, 0, 1);
   __syncwarp();
   if (!sp_check_input(A.m)) {
     wide_fail(H, kBadInput);
@@ -953,7 +952,7 @@ __device__ __noinline__ int32_t wide_gift_node(const WidePtrs& P, const WideArgs
       h.len = len;
       h.counter = n;
       h.last = 0;
-      h.rslot = -1;
+      h.rslot = kNone;
       h.pad = 0;
       W.tc[lvl - 1] = h;
       W.seq[lvl - 1] = u;
@@ -1028,7 +1027,7 @@ __global__ void __launch_bounds__(kSpThreads) wide_items_kernel(WideArgs A) {
   const uint32_t n = A.n, D = H->D, nitems = H->nitems, cap = A.WL.cap;
   uint8_t* slot = A.slots + ((uint64_t)blockIdx.x * kSpWarps + (uint64_t)warp) * A.slot_bytes;
   uint8_t* smem = A.smem_per_warp ? sp_dyn + (uint64_t)warp * A.smem_per_warp : nullptr;
-  sp_bind(slot, A.Lo, n, A.rp, A.col, smem, A.smem_per_warp, A.pool, 0, cap);
+  sp_bind(slot, A.Lo, n, A.rp, A.col, smem, A.smem_per_warp, 0, cap);
   __syncwarp();
   if (lane == 0) {
     // the first path is shared and read-only; automorphisms go to the store
@@ -1179,10 +1178,11 @@ __global__ void __launch_bounds__(kSpThreads) wide_items_kernel(WideArgs A) {
       h.len = tl;
       h.counter = n;  // this warp takes no other child of the parent
       h.last = 0;
-      h.rslot = -1;
+      h.rslot = kNone;
       h.pad = 0;
       W.tc[k] = h;
       W.pool_top = 0;
+      W.pool_frames = 0;
     }
     __syncwarp();
     // private best: refresh when the shared one has changed
@@ -1338,7 +1338,7 @@ __global__ void __launch_bounds__(kSpThreads) wide_items_kernel(WideArgs A) {
               h.len = sp_cell_end(W, t) - t;
               h.counter = 0;
               h.last = 0;
-              h.rslot = -1;
+              h.rslot = kNone;
               h.pad = 0;
               W.tc[tcl] = h;
             }
@@ -1356,12 +1356,9 @@ __global__ void __launch_bounds__(kSpThreads) wide_items_kernel(WideArgs A) {
             }
             if (known > (uint32_t)W.tc[idx].last) {
               const unsigned long long tc = cnt.now();
-              const bool orb_ok = sp_orbits<true>(idx, (int)known, seqlen);
+              status = sp_orbits<true>(idx, (int)known, seqlen);
               cnt.add(kCntOrbitCycles, cnt.now() - tc);
-              if (!orb_ok) {
-                status = W.pool_top >= W.pool_cap ? kAutOverflow : kInternal;
-                break;
-              }
+              if (status != kOk) break;
               __syncwarp();
               if (lane == 0) W.tc[idx].last = (int32_t)known;
               __syncwarp();
@@ -1418,10 +1415,7 @@ __global__ void __launch_bounds__(kSpThreads) wide_items_kernel(WideArgs A) {
         tcl = (int)Lv;
         level = Lv;
         sp_fix_clamp(seqlen, fix_init);
-        __syncwarp();
-        if (lane == 0)
-          while (W.pool_top > 0 && W.pool_owner[W.pool_top - 1] >= (int32_t)Lv) W.pool_top -= 1;
-        __syncwarp();
+        sp_pool_pop(Lv);
         if (recompare) wide_recompare(level, best.canon_level, &eqlevcanon, &comp_canon);
       }
     }

@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kSpThreads, 5)
       if (lane == 0) A.status[g] = kTooLarge;
       continue;
     }
-    const SpResult r = sp_search(A, g, slot, Lo, pool, cap, smem, smem_per_warp);
+    const SpResult r = sp_search(A, g, slot, Lo, cap, smem, smem_per_warp);
     if (lane == 0) {
       A.status[g] = r.status;
       if (A.out_stats) {
@@ -925,7 +925,6 @@ int gcl_canon_wide_device_async(gcl_context* c, const int32_t* d_rowptr, const i
   WA.slots = (uint8_t*)c->wide_slots.p;
   WA.Lo = Lo;
   WA.slot_bytes = Lo.bytes;
-  WA.pool = pool;
   WA.gate = (uint32_t)c->wide_gate;
   WA.probe = c->wide_probe ? 1u : 0u;
   WA.smem_per_warp = smw;
