@@ -61,7 +61,7 @@ struct SpLayout {
   uint64_t u32n[13];  // offsets of the n-sized u32 arrays
   uint64_t elem, pos, cnt;
   uint64_t fcode, ccode, pool_owner;
-  uint64_t stb, sts, act, acts, itm, nsb;
+  uint64_t stb, sts, act, itm, nsb;
   uint64_t fcert, bcert, ccert;
   uint64_t tc, reps, auts, fixm, fixst;
   uint32_t fixcap, reps_cap;
@@ -69,6 +69,11 @@ struct SpLayout {
   uint32_t nw, nsw;
   uint32_t stride;  // elements per representative array / ring entry
 };
+
+// 32-bit words of a bitmap over n positions that is read four words at a time
+__host__ __device__ inline uint32_t sp_pad_words(uint32_t n) {
+  return ((n + 31) / 32 + 3) & ~3u;
+}
 
 __host__ __device__ inline SpLayout sp_layout(uint32_t n, uint64_t m2, uint32_t pool,
                                               uint32_t cap, uint32_t fixcap = 0) {
@@ -93,10 +98,10 @@ __host__ __device__ inline SpLayout sp_layout(uint32_t n, uint64_t m2, uint32_t 
   L.nsw = (L.nw + 63) / 64 + 1;
   L.stb = take(8ull * L.nw);
   L.sts = take(8ull * L.nsw);
-  L.act = take(8ull * L.nw);
-  L.acts = take(8ull * L.nsw);
-  L.itm = take(8ull * L.nw);
-  L.nsb = take(8ull * L.nw);
+  const uint64_t wp = sp_pad_words(n);
+  L.act = take(4 * wp);
+  L.itm = take(4 * wp);
+  L.nsb = take(4 * wp);
   L.fcert = take(4 * (m2 + 1));
   L.bcert = take(4 * (m2 + 1));
   L.ccert = take(4 * (m2 + 1));
@@ -115,11 +120,11 @@ __host__ __device__ inline SpLayout sp_layout(uint32_t n, uint64_t m2, uint32_t 
 }
 
 // Shared-memory staging: the arrays every refinement step touches (elem, pos,
-// neighbour counts by position, the start and active bitmaps with their
-// summaries, the marks of the hash) live in the warp's shared-memory region
+// neighbour counts by position, the start bitmap with its summary, the active
+// cells, the marks of the hash) live in the warp's shared-memory region
 // when they fit.  elem lies at offset 0.
 struct SpStage {
-  uint32_t pos, cnt, stb, sts, act, acts, itm, nsb, bytes;
+  uint32_t pos, cnt, stb, sts, act, itm, nsb, bytes;
 };
 __host__ __device__ inline SpStage sp_stage(uint32_t n) {
   const uint32_t nw = (n + 63) / 64 + 1, nsw = (nw + 63) / 64 + 1;
@@ -129,11 +134,10 @@ __host__ __device__ inline SpStage sp_stage(uint32_t n) {
   G.cnt = 2 * a;
   G.stb = 3 * a;
   G.sts = G.stb + 8 * nw;
-  G.act = G.sts + 8 * nsw;
-  G.acts = G.act + 8 * nw;
-  G.itm = G.acts + 8 * nsw;
-  G.nsb = G.itm + 8 * nw;
-  G.bytes = (G.nsb + 8 * nw + 15) & ~15u;
+  G.act = (G.sts + 8 * nsw + 15) & ~15u;
+  G.itm = G.act + 4 * sp_pad_words(n);
+  G.nsb = G.itm + 4 * sp_pad_words(n);
+  G.bytes = G.nsb + 4 * sp_pad_words(n);
   return G;
 }
 __host__ __device__ inline uint64_t sp_smem_bytes(uint32_t n) { return sp_stage(n).bytes; }
@@ -149,8 +153,9 @@ struct SpWarp {
   uint32_t *umark;  // per level: start-log size when the level's child was made
   uint2* fixst;     // per stored automorphism: {prefix of seq it fixes, first
                     // position of seq it moves or kNone}, valid for the path
-  uint64_t *stb, *sts, *act, *acts;  // cell starts (position n too) and active cells
-  uint32_t *itm, *nsb;  // marks of the hash: touched fragments, fragment starts
+  uint64_t *stb, *sts;         // cell starts (position n too) and their summary
+  uint32_t *act, *itm, *nsb;   // active cells; marks of the hash: touched fragments,
+                               // fragment starts (sp_pad_words words each)
   uint32_t *fcert, *bcert, *ccert;
   uint32_t* reps;   // stack of target cells' {vertex, representative << 16}
   uint32_t* fixm;   // per vertex: a bit per ring entry that fixes it
@@ -163,6 +168,7 @@ struct SpWarp {
   uint32_t ncells, nact;
   uint32_t pool_top, pool_frames, pool_cap, aut_cap, max_aut;
   uint32_t scr[32];  // a word per lane: the union-find of a small target cell
+  alignas(16) uint16_t list[256];  // items of a hash
   uint32_t utop;  // entries of slog
   uint32_t fixcap;  // store entries whose fix state is kept (later ones are checked in full)
 };
@@ -184,7 +190,7 @@ __device__ __forceinline__ bool bm_test(const uint64_t* B, uint32_t p) {
   return (B[p >> 6] >> (p & 63)) & 1ull;
 }
 // smallest set position >= p, or n
-__device__ uint32_t bm_next(const uint64_t* B, const uint64_t* Sm, uint32_t p, uint32_t n,
+__device__ __noinline__ uint32_t bm_next(const uint64_t* B, const uint64_t* Sm, uint32_t p, uint32_t n,
                             uint32_t nw, uint32_t nsw) {
   if (p >= n) return n;
   uint32_t w = p >> 6;
@@ -203,7 +209,7 @@ __device__ uint32_t bm_next(const uint64_t* B, const uint64_t* Sm, uint32_t p, u
   return min(n, w2 * 64 + ctz64(B[w2]));
 }
 // largest set position <= p, or kNone
-__device__ uint32_t bm_prev(const uint64_t* B, const uint64_t* Sm, uint32_t p) {
+__device__ __noinline__ uint32_t bm_prev(const uint64_t* B, const uint64_t* Sm, uint32_t p) {
   uint32_t w = p >> 6;
   const uint64_t x = B[w] & low_mask((p & 63) + 1);
   if (x) return w * 64 + msb64(x);
@@ -223,16 +229,6 @@ __device__ __forceinline__ void bm_set1(uint64_t* B, uint64_t* Sm, uint32_t p) {
   B[p >> 6] |= bit64(p & 63);
   Sm[p >> 12] |= bit64((p >> 6) & 63);
 }
-__device__ __forceinline__ void bm_clear1(uint64_t* B, uint64_t* Sm, uint32_t p) {
-  const uint64_t v = B[p >> 6] & ~bit64(p & 63);
-  B[p >> 6] = v;
-  if (!v) Sm[p >> 12] &= ~bit64((p >> 6) & 63);
-}
-__device__ __forceinline__ void bm_set_atomic(uint64_t* B, uint64_t* Sm, uint32_t p) {
-  atomicOr((unsigned long long*)&B[p >> 6], (unsigned long long)bit64(p & 63));
-  atomicOr((unsigned long long*)&Sm[p >> 12], (unsigned long long)bit64((p >> 6) & 63));
-}
-
 // warp: rebuild a summary from its bitmap
 __device__ void bm_resummarize(const uint64_t* B, uint64_t* Sm, uint32_t nw, uint32_t nsw) {
   const uint32_t lane = lane_id();
@@ -283,8 +279,8 @@ __device__ __forceinline__ void add_start(SpWarp& W, uint32_t p) {
 template <bool kS>
 struct SpRef {
   uint16_t *elem, *pos, *cnt;
-  uint64_t *stb, *sts, *act, *acts;
-  uint32_t *itm, *nsb;
+  uint64_t *stb, *sts;
+  uint32_t *st, *act, *itm, *nsb;  // st: stb as 32-bit words
   __device__ __forceinline__ explicit SpRef(const SpWarp& W) {
     if constexpr (kS) {
       const SpStage G = sp_stage(W.n);
@@ -294,8 +290,7 @@ struct SpRef {
       cnt = (uint16_t*)(b + G.cnt);
       stb = (uint64_t*)(b + G.stb);
       sts = (uint64_t*)(b + G.sts);
-      act = (uint64_t*)(b + G.act);
-      acts = (uint64_t*)(b + G.acts);
+      act = (uint32_t*)(b + G.act);
       itm = (uint32_t*)(b + G.itm);
       nsb = (uint32_t*)(b + G.nsb);
     } else {
@@ -305,10 +300,37 @@ struct SpRef {
       stb = W.stb;
       sts = W.sts;
       act = W.act;
-      acts = W.acts;
       itm = W.itm;
       nsb = W.nsb;
     }
+    st = (uint32_t*)stb;
+  }
+  // whether the vertex at position p is alone in its cell: p and p + 1 are
+  // starts (position n is marked as one)
+  __device__ __forceinline__ bool alone(uint32_t p) const {
+    const uint32_t w = p >> 5;
+    return (__funnelshift_r(st[w], st[w + 1], p & 31u) & 3u) == 3u;
+  }
+  __device__ __forceinline__ bool active(uint32_t c) const {
+    return (act[c >> 5] >> (c & 31u)) & 1u;
+  }
+  // the cell [c, e) of position p.  Cells are short once a refinement is under
+  // way: the words beside p's are tried before the summary.
+  __device__ __forceinline__ uint32_t start_of(uint32_t p) const {
+    uint32_t w = p >> 5, x = st[w] & (0xffffffffu >> (31u - (p & 31u)));
+    for (int far = 0; !x; ++far) {
+      if (far == 4) return bm_prev(stb, sts, w * 32 - 1);
+      x = st[--w];
+    }
+    return w * 32 + 31u - (uint32_t)__clz((int)x);
+  }
+  __device__ __forceinline__ uint32_t end_of(uint32_t p, uint32_t n) const {
+    uint32_t w = p >> 5, x = st[w] & (0xfffffffeu << (p & 31u));
+    for (int far = 0; !x; ++far) {
+      if (far == 4) return bm_next(stb, sts, (w + 1) * 32, n, (n + 63) / 64 + 1, ((n + 63) / 64 + 64) / 64 + 1);
+      x = st[++w];
+    }
+    return w * 32 + (uint32_t)__ffs((int)x) - 1u;
   }
 };
 
@@ -343,24 +365,23 @@ __device__ __forceinline__ uint32_t nth_bit(uint32_t x, uint32_t j) {
 // marked in `itm`).  The fragment starts are the old non-singleton cells' and
 // the marked positions, or, when `listed`, the bits of `nsb`.
 //
-// A lane takes kW words of 32 positions.  Few items are folded one after the
-// other, two instructions each.  Many are folded one bit of the running value
-// at a time over all positions at once: bit j of the value before item i is bit
-// j of the initial value xor the parity of the flips of the items before it
-// (a prefix parity within the word, a ballot across the lanes), and that gives
-// the carries into bit j + 1.  A position's own bits are constants of its word,
-// so no list of cells is ever built.  Listing the cells and taking 15 ballots
-// per 32 of them took 61,700 of a step's 67,600 cycles on a 64 x 64 torus
-// (about 1,200 cells); with this fold the search of that torus takes 71 ms
-// instead of 270.
-// ---------------------------------------------------------------------------
+// A lane takes kW words of 32 positions.  Up to 256 items are compacted into a
+// list and folded one after the other, two instructions each.  More are folded
+// one bit of the running value at a time over all positions at once: bit j of
+// the value before item i is bit j of the initial value xor the parity of the
+// flips of the items before it (a prefix parity within the word, a ballot
+// across the lanes), and that gives the carries into bit j + 1.  A position's
+// own bits are constants of its word, so no list of cells is built.  Listing
+// the cells and taking 15 ballots per 32 of them took 61,700 of a step's 67,600
+// cycles on a 64 x 64 torus (about 1,200 cells); with the bit-wise fold the
+// search of that torus took 71 ms instead of 270.
 template <bool kS, int kW>
 __device__ __noinline__ uint32_t sp_fold(uint32_t lc, bool listed) {
   constexpr uint32_t C = 065435u;
-  // items above which the bit-wise fold is the faster one: about 20 cycles per
-  // item against about 2,000 (one word per lane) or 3,500 (four)
-  constexpr uint32_t kDense = kW == 1 ? 96 : 176;
-  const SpWarp& W = sp_w();
+  // a list item takes about 14 cycles, the bit-wise fold 3,000 (one word per
+  // lane) to 5,000 (four) in all: the line lies at the list's size
+  constexpr uint32_t kList = 256;
+  SpWarp& W = sp_w();
   const SpRef<kS> R(W);
   const uint32_t lane = lane_id(), n = W.n, nwd = (n + 31) / 32, lt = lanemask_lt();
   for (uint32_t base = 0; base < nwd; base += 32 * kW) {
@@ -377,7 +398,8 @@ __device__ __noinline__ uint32_t sp_fold(uint32_t lc, bool listed) {
         K += (uint32_t)__popc(vw[w]);
       }
     }
-    bool dense = __reduce_add_sync(GCL_FULL, K) > kDense;
+    const uint32_t total = __reduce_add_sync(GCL_FULL, K);
+    bool dense = total > kList;
     uint32_t kb[6][kW];
     if (dense) {  // the counts, one bit per word (larger counts take the other way)
       bool big = false;
@@ -395,23 +417,54 @@ __device__ __noinline__ uint32_t sp_fold(uint32_t lc, bool listed) {
       dense = !__any_sync(GCL_FULL, big);
     }
     if (!dense) {
-      uint32_t some = 0;
+      // the items in position order, 256 at a time (one round unless a large
+      // count turned the bit-wise fold away)
+      uint32_t at = K;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(GCL_FULL, at, o);
+        if (lane >= (uint32_t)o) at += y;
+      }
+      at -= K;
+      for (uint32_t done = 0; done < total; done += kList) {
+        const uint32_t m = min(kList, total - done);
+        uint32_t i = at - done;  // index in this round's list (wraps below it)
 #pragma unroll
-      for (int w = 0; w < kW; ++w) some |= vw[w];
-      for (uint32_t any = __ballot_sync(GCL_FULL, some != 0); any; any &= any - 1) {
-        const int src = __ffs((int)any) - 1;
-#pragma unroll
-        for (int w = 0; w < kW; ++w) {
-          const uint32_t m = __shfl_sync(GCL_FULL, mw[w], src);
-          uint32_t x = __shfl_sync(GCL_FULL, vw[w], src);
-          const uint32_t pb = (base + (uint32_t)src * kW + w) * 32;
-          for (; x; x &= x - 1) {
-            const uint32_t b = (uint32_t)__ffs((int)x) - 1;
-            uint32_t v = pb + b;
-            if ((m >> b) & 1u) v += R.cnt[v];
-            lc = (lc ^ C) + v;
+        for (int w = 0; w < kW; ++w)
+          for (uint32_t x = vw[w]; x; x &= x - 1, ++i) {
+            if (i >= kList) continue;
+            const uint32_t b = (uint32_t)__ffs((int)x) - 1, p = (w0 + w) * 32 + b;
+            // the low 15 bits of an item are all that counts
+            W.list[i] = (uint16_t)(p + ((mw[w] >> b) & 1u ? R.cnt[p] : 0u));
           }
+        __syncwarp();
+        const uint4* l4 = (const uint4*)W.list;
+        auto two = [&](uint32_t x) {  // bits above 14 never come down
+          lc = (lc ^ C) + x;
+          lc = (lc ^ C) + (x >> 16);
+        };
+        for (uint32_t q = 0; q < m / 8; ++q) {
+          const uint4 x = l4[q];
+          two(x.x);
+          two(x.y);
+          two(x.z);
+          two(x.w);
         }
+        if (m & 7u) {
+          const uint4 x = l4[m / 8];
+          uint32_t a = x.x, b = x.y;
+          if (m & 4u) {
+            two(a);
+            two(b);
+            a = x.z;
+            b = x.w;
+          }
+          if (m & 2u) {
+            two(a);
+            a = b;
+          }
+          if (m & 1u) lc = (lc ^ C) + a;
+        }
+        __syncwarp();
       }
       continue;
     }
@@ -473,7 +526,7 @@ __device__ __noinline__ SpStep sp_refine_general(uint32_t s, uint32_t e, uint32_
                                                  uint32_t hint, uint32_t utop) {
   SpWarp& W = sp_w();
   const SpRef<kS> R(W);
-  const uint32_t lane = lane_id(), n = W.n, nw = W.nw, nsw = W.nsw, lt = lanemask_lt();
+  const uint32_t lane = lane_id(), n = W.n, lt = lanemask_lt();
   const uint32_t nwd = (n + 31) / 32;
   const bool single = e - s == 1;
   const uint32_t flip = single ? 1u : 0u;  // a neighbour's key is 0, a non-neighbour's 1
@@ -509,7 +562,7 @@ __device__ __noinline__ SpStep sp_refine_general(uint32_t s, uint32_t e, uint32_
       bm_or(R.stb, R.sts, f);
       or_bit32(R.nsb, f);
     }
-    if (frag && active) bm_or(R.act, R.acts, f);
+    if (frag && active) or_bit32(R.act, f);
     utop += (uint32_t)__popc(m);
     if (!single) {
       const uint32_t h = __reduce_max_sync(GCL_FULL, fresh && size == 1 ? f + 1 : 0u);
@@ -529,7 +582,7 @@ __device__ __noinline__ SpStep sp_refine_general(uint32_t s, uint32_t e, uint32_
     uint32_t pend = 0;
     for (uint32_t x = wi < nwd ? R.nsb[wi] : 0u; x; x &= x - 1) {
       const uint32_t b = (uint32_t)__ffs((int)x) - 1, c = wi * 32 + b;
-      const uint32_t ce = bm_next(R.stb, R.sts, c + 1, n, nw, nsw);
+      const uint32_t ce = R.end_of(c, n);
       bool differ = ce - c > 32;  // large cells are tested by the whole warp
       if (!differ) {
         const uint32_t a = R.cnt[c];
@@ -543,8 +596,8 @@ __device__ __noinline__ SpStep sp_refine_general(uint32_t s, uint32_t e, uint32_
       const int src = __ffs((int)any) - 1;
       for (uint32_t m = __shfl_sync(GCL_FULL, pend, src); m; m &= m - 1) {
         const uint32_t c = (base + (uint32_t)src) * 32 + (uint32_t)__ffs((int)m) - 1;
-        const uint32_t ce = bm_next(R.stb, R.sts, c + 1, n, nw, nsw), L = ce - c;
-        const bool was = bm_test(R.act, c);
+        const uint32_t ce = R.end_of(c, n), L = ce - c;
+        const bool was = R.active(c);
         if (L <= 32) {
           const bool in = lane < L;
           const uint32_t v = in ? R.elem[c + lane] : 0u, a = in ? R.cnt[c + lane] : 0u;
@@ -676,7 +729,7 @@ __device__ __noinline__ int sp_refine_t() {
   SpWarp& W = sp_w();
   const SpRef<kS> R(W);
   const uint32_t lane = lane_id(), lt = lanemask_lt();
-  const uint32_t n = W.n, nw = W.nw, nsw = W.nsw;
+  const uint32_t n = W.n, nwd = (n + 31) / 32;
   constexpr uint32_t C = 065435u;
   uint32_t ncells = W.ncells, nact = W.nact, utop = W.utop;
   uint32_t lc = ncells, hint = 0, iters = 0;
@@ -684,27 +737,58 @@ __device__ __noinline__ int sp_refine_t() {
   const int32_t* const rp = W.rp;
   const int32_t* const col = W.col;
   uint32_t* const slog = W.slog;
-  // whether the vertex at position p is not alone in its cell (position n is
-  // marked as a start)
-  auto shared_cell = [&](uint32_t p) {
-    const uint32_t* s = (const uint32_t*)R.stb;
-    return !((s[p >> 5] >> (p & 31u)) & (s[(p + 1) >> 5] >> ((p + 1) & 31u)) & 1u);
+  // the splitter: the first active position from the hint on, else from 0
+  auto next_active = [&]() -> uint32_t {
+    if (nwd <= 32) {  // a word per lane
+      const uint32_t w = lane < nwd ? R.act[lane] : 0u, hw = hint >> 5;
+      const uint32_t ge = lane > hw ? w : lane == hw ? w & (0xffffffffu << (hint & 31u)) : 0u;
+      uint32_t m = __ballot_sync(GCL_FULL, ge != 0), x = ge;
+      if (!m) {
+        m = __ballot_sync(GCL_FULL, w != 0);
+        x = w;
+      }
+      if (!m) return kNone;
+      const uint32_t src = (uint32_t)__ffs((int)m) - 1;
+      return src * 32 + (uint32_t)__ffs((int)__shfl_sync(GCL_FULL, x, (int)src)) - 1;
+    }
+    const uint32_t near = R.act[hint >> 5] >> (hint & 31u);
+    if (near) return hint + (uint32_t)__ffs((int)near) - 1;
+    // four words per lane from the word after the hint's, then from word 0
+    const uint32_t from = (hint >> 5) + 1, wp = sp_pad_words(n);
+    for (int wrap = 0; wrap < 2; ++wrap)
+      for (uint32_t base = wrap ? 0 : from & ~127u; base < wp; base += 128) {
+        const uint32_t w0 = base + lane * 4;
+        uint4 x = make_uint4(0, 0, 0, 0);
+        if (w0 < wp) x = *(const uint4*)(R.act + w0);
+        if (!wrap && base < from) {
+          if (w0 < from) x.x = 0;
+          if (w0 + 1 < from) x.y = 0;
+          if (w0 + 2 < from) x.z = 0;
+          if (w0 + 3 < from) x.w = 0;
+        }
+        const uint32_t m = __ballot_sync(GCL_FULL, (x.x | x.y | x.z | x.w) != 0);
+        if (!m) continue;
+        const uint32_t p = x.x   ? (uint32_t)__ffs((int)x.x)
+                           : x.y ? 32 + (uint32_t)__ffs((int)x.y)
+                           : x.z ? 64 + (uint32_t)__ffs((int)x.z)
+                                 : 96 + (uint32_t)__ffs((int)x.w);
+        return __shfl_sync(GCL_FULL, w0 * 32 + p - 1, __ffs((int)m) - 1);
+      }
+    return kNone;
   };
   while (ncells < n && nact > 0) {
     if (++iters > 4 * n + 64) {  // every step removes an active cell or splits one
       ok = 0;
       break;
     }
-    // splitter: hint if active, else the next active after it, else wrap
-    uint32_t s = bm_next(R.act, R.acts, hint, n, nw, nsw);
-    if (s >= n) s = bm_next(R.act, R.acts, 0, n, nw, nsw);
+    const uint32_t s = next_active();
     if (s >= n) {
       ok = 0;
       break;
     }
-    const uint32_t e = bm_next(R.stb, R.sts, s + 1, n, nw, nsw);
+    const uint32_t e = (R.st[(s + 1) >> 5] >> ((s + 1) & 31u)) & 1u ? s + 1 : R.end_of(s, n);
     __syncwarp();
-    if (lane == 0) bm_clear1(R.act, R.acts, s);
+    if (lane == 0) atomicAnd(R.act + (s >> 5), ~(1u << (s & 31u)));
     nact -= 1;
     const uint32_t len = e - s;
     lc = (lc ^ C) + (s + e - 1);
@@ -719,13 +803,13 @@ __device__ __noinline__ int sp_refine_t() {
         if ((int32_t)lane < sd) {
           u = (uint32_t)col[sb + (int32_t)lane];
           p = R.pos[u];
-          on = shared_cell(p);
+          on = !R.alone(p);
         }
         __syncwarp();
         if (!__any_sync(GCL_FULL, on)) continue;
         if (on) {
-          c = bm_prev(R.stb, R.sts, p);
-          L = bm_next(R.stb, R.sts, p + 1, n, nw, nsw) - c;
+          c = R.start_of(p);
+          L = R.end_of(p, n) - c;
         }
         const uint32_t grp = __match_any_sync(GCL_FULL, c);
         const uint32_t k = (uint32_t)__popc(grp);
@@ -749,7 +833,7 @@ __device__ __noinline__ int sp_refine_t() {
         }
         if (mv) x = R.elem[h];
         const bool lead = spl && lane == (uint32_t)(__ffs((int)grp) - 1);
-        const bool was = lead && bm_test(R.act, c);
+        const bool was = lead && R.active(c);
         const uint32_t leaders = __ballot_sync(GCL_FULL, lead);
         const uint32_t made = (uint32_t)__popc(leaders);
         __syncwarp();
@@ -767,7 +851,7 @@ __device__ __noinline__ int sp_refine_t() {
           key = (c << 6) | k;
           slog[utop + (uint32_t)__popc(leaders & lt)] = pp;
           bm_or(R.stb, R.sts, pp);
-          bm_or(R.act, R.acts, rest ? pp : c);
+          or_bit32(R.act, rest ? pp : c);
         }
         utop += made;
         ncells += made;
@@ -823,15 +907,15 @@ __device__ __noinline__ int sp_refine_t() {
         if (lane < D) {
           u = (uint32_t)col[bs + (int32_t)(lane - es)];
           p = R.pos[u];
-          if (!shared_cell(p)) u = kNone;  // singleton cells never split (:257-259)
+          if (R.alone(p)) u = kNone;  // singleton cells never split (:257-259)
         }
         // lanes on the same neighbour: the group's size is its count
         const uint32_t gu = __match_any_sync(GCL_FULL, u);
         const uint32_t cnt = (uint32_t)__popc(gu);
         const bool lead = u != kNone && lane == (uint32_t)(__ffs((int)gu) - 1);
         if (lead) {
-          c = bm_prev(R.stb, R.sts, p);
-          L = bm_next(R.stb, R.sts, p + 1, n, nw, nsw) - c;
+          c = R.start_of(p);
+          L = R.end_of(p, n) - c;
         }
         const uint32_t gc = __match_any_sync(GCL_FULL, c);
         const uint32_t k = (uint32_t)__popc(gc);  // touched vertices of the cell
@@ -873,7 +957,7 @@ __device__ __noinline__ int sp_refine_t() {
                              (uint32_t)__popc(outs & lt));
             x = R.elem[h];
           }
-          const bool was = split && bm_test(R.act, c);
+          const bool was = split && R.active(c);
           // the first largest fragment is the untouched one (it comes first)
           const bool rest = L - k >= (best >> 6);
           const bool fresh = frag && f != c;
@@ -888,8 +972,8 @@ __device__ __noinline__ int sp_refine_t() {
             R.elem[f + eq] = (uint16_t)u;
             R.pos[u] = (uint16_t)(f + eq);
           }
-          if (frag && (was ? f != c : rest || rank != best)) bm_or(R.act, R.acts, f);
-          if (cell_lead && split && L > k && !was && !rest) bm_or(R.act, R.acts, c);
+          if (frag && (was ? f != c : rest || rank != best)) or_bit32(R.act, f);
+          if (cell_lead && split && L > k && !was && !rest) or_bit32(R.act, c);
           if (fresh) slog[utop + (uint32_t)__popc(fm & lt)] = f;
           const uint32_t hv = __reduce_max_sync(GCL_FULL, fresh && size == 1 ? f + 1 : 0u);
           if (hv) hint = hv - 1;
@@ -924,8 +1008,8 @@ __device__ __noinline__ int sp_refine_t() {
   }
   // clear what is left of the active set
   __syncwarp();
-  for (uint32_t w = lane; w < nw; w += 32) R.act[w] = 0;
-  for (uint32_t w = lane; w < nsw; w += 32) R.acts[w] = 0;
+  if (nact)
+    for (uint32_t w = lane; w < sp_pad_words(n); w += 32) R.act[w] = 0;
   if (lane == 0) {
     W.ncells = ncells;
     W.utop = utop;
@@ -956,7 +1040,7 @@ __device__ __forceinline__ bool sp_individualize(uint32_t level, uint32_t v, uin
     W.pos[v] = t;
     add_start(W, t + 1);
     W.ncells += 1;
-    bm_set1(W.act, W.acts, t);
+    or_bit32(W.act, t);
     W.nact = 1;
   }
   __syncwarp();
@@ -991,21 +1075,62 @@ __device__ __forceinline__ bool sp_backtrack(uint32_t Lv) {
 }
 
 // ---- leaves ----------------------------------------------------------------
+// A certificate row of at most kD entries by one lane, in registers.
+template <int kD>
+__device__ __forceinline__ void sp_cert_row(const SpWarp& W, uint32_t* cert, int32_t b, int32_t d) {
+  uint32_t x[kD];
+#pragma unroll
+  for (int i = 0; i < kD; ++i) x[i] = i < d ? (uint32_t)W.col[b + i] : 0u;
+#pragma unroll
+  for (int i = 0; i < kD; ++i) x[i] = i < d ? W.pos[x[i]] : kNone;
+#pragma unroll
+  for (int i = 0; i < kD; ++i) {
+    int32_t r = 0;
+#pragma unroll
+    for (int k = 0; k < kD; ++k) r += x[k] < x[i];
+    if (i < d) cert[b + r] = x[i];
+  }
+}
+
 // Certificate of a discrete partition: for every vertex, the canonical
-// positions of its neighbours in ascending order, stored at its CSR offset.
+// positions of its neighbours in ascending order, stored at its CSR offset --
+// each written once, at its rank in the row (sorting the row in place read back
+// every entry from device memory: 40,400 cycles for a tree of 1,000 vertices).
 __device__ __forceinline__ void sp_leaf_cert(uint32_t* cert) {
   SpWarp& W = sp_w();
   const uint32_t lane = lane_id();
-  for (uint32_t v = lane; v < W.n; v += 32) {
-    const int32_t b = W.rp[v], e = W.rp[v + 1];
-    for (int32_t i = b; i < e; ++i) {
-      const uint32_t x = W.pos[W.col[i]];
-      int32_t j = i - 1;
-      while (j >= b && cert[j] > x) {  // insertion sort (rows are short)
-        cert[j + 1] = cert[j];
-        --j;
+  for (uint32_t v0 = 0; v0 < W.n; v0 += 32) {
+    const uint32_t v = v0 + lane;
+    int32_t b = 0, d = 0;
+    if (v < W.n) {
+      b = W.rp[v];
+      d = W.rp[v + 1] - b;
+    }
+    // a row per lane; what the widest row of up to 16 entries needs decides
+    // how many compares every row takes
+    const int32_t ds = d <= 16 ? d : 0, top = __reduce_max_sync(GCL_FULL, ds);
+    if (top <= 4)
+      sp_cert_row<4>(W, cert, b, ds);
+    else if (top <= 8)
+      sp_cert_row<8>(W, cert, b, ds);
+    else
+      sp_cert_row<16>(W, cert, b, ds);
+    // longer rows: the warp takes a row at a time, an entry per lane
+    for (uint32_t m = __ballot_sync(GCL_FULL, d > 16); m; m &= m - 1) {
+      const int src = __ffs((int)m) - 1;
+      const int32_t rb = __shfl_sync(GCL_FULL, b, src), rd = __shfl_sync(GCL_FULL, d, src);
+      for (int32_t i0 = 0; i0 < rd; i0 += 32) {
+        const int32_t i = i0 + (int32_t)lane;
+        const uint32_t x = i < rd ? W.pos[W.col[rb + i]] : kNone;
+        int32_t r = 0;
+        for (int32_t k0 = 0; k0 < rd; k0 += 32) {
+          const int32_t kk = k0 + (int32_t)lane;
+          const uint32_t y = k0 == i0 ? x : kk < rd ? W.pos[W.col[rb + kk]] : kNone;
+          const int32_t cnt = min(32, rd - k0);
+          for (int32_t k = 0; k < cnt; ++k) r += __shfl_sync(GCL_FULL, y, k) < x;
+        }
+        if (i < rd) cert[rb + r] = x;
       }
-      cert[j + 1] = x;
     }
   }
   __syncwarp();
@@ -1186,18 +1311,25 @@ struct SpCellOrbits {
   uint32_t v, comp;  // the lane's vertex (kNone past the cell) and its component
 };
 
-// Merge the orbits of one automorphism, whose image of the lane's vertex lies
-// at index j of the cell (j == lane past it).
-__device__ __forceinline__ void sp_cell_merge(SpCellOrbits& o, uint32_t j) {
+// Merge the orbits of up to four automorphisms, whose images of the lane's
+// vertex lie at indexes j of the cell (j == lane where there is none).
+__device__ __forceinline__ void sp_cell_merge(SpCellOrbits& o, const uint32_t (&j)[4]) {
   SpWarp& W = sp_w();
   const uint32_t lane = lane_id();
   while (true) {  // every round with an open edge removes a component
-    const uint32_t cj = __shfl_sync(GCL_FULL, o.comp, (int)j);
-    const bool d = cj != o.comp;
+    uint32_t cj[4];
+    bool d = false;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      cj[k] = __shfl_sync(GCL_FULL, o.comp, (int)j[k]);
+      d |= cj[k] != o.comp;
+    }
     if (!__any_sync(GCL_FULL, d)) return;
     W.scr[lane] = lane;
     __syncwarp();
-    if (d) atomicMin(&W.scr[max(o.comp, cj)], min(o.comp, cj));
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (cj[k] != o.comp) atomicMin(&W.scr[max(o.comp, cj[k])], min(o.comp, cj[k]));
     __syncwarp();
     bool moved;
     do {  // to the root (links go to smaller lanes)
@@ -1271,27 +1403,23 @@ __device__ __noinline__ int32_t sp_orbits(int idx, int num_aut, uint32_t seqlen)
     if (small) {
       while (m) {
         // up to four entries' images at once, so their loads overlap
-        uint32_t j[4], cnt = 0;
+        uint32_t j[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          j[k] = lane;
+          j[k] = lane < t.len ? o.v : kNone;
           if (!m) continue;
           const uint16_t* pm = W.auts + (uint64_t)(base + (uint32_t)__ffs((int)m) - 1) * W.stride;
           m &= m - 1;
-          ++cnt;
           if (lane < t.len) j[k] = ldx<kCg>(pm + o.v);
         }
         bool out = false;
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if ((uint32_t)k < cnt && lane < t.len) {
-            j[k] = (uint32_t)W.pos[j[k]] - t.first;
-            out |= j[k] >= t.len;
-          }
+        for (int k = 0; k < 4; ++k) {
+          j[k] = j[k] == kNone ? lane : j[k] == o.v ? lane : (uint32_t)W.pos[j[k]] - t.first;
+          out |= lane < t.len && j[k] >= t.len;
+        }
         if (__any_sync(GCL_FULL, out)) return kInternal;
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if ((uint32_t)k < cnt) sp_cell_merge(o, j[k]);
+        sp_cell_merge(o, j);
       }
       return kOk;
     }
@@ -1437,9 +1565,7 @@ __device__ __forceinline__ void sp_clear_scratch() {
   SpWarp& W = sp_w();
   const uint32_t lane = lane_id();
   for (uint32_t i = lane; i < W.n; i += 32) W.cnt[i] = 0;
-  for (uint32_t w = lane; w < 2 * W.nw; w += 32) W.itm[w] = 0;
-  for (uint32_t w = lane; w < W.nw; w += 32) W.act[w] = 0;
-  for (uint32_t w = lane; w < W.nsw; w += 32) W.acts[w] = 0;
+  for (uint32_t w = lane; w < sp_pad_words(W.n); w += 32) W.itm[w] = W.act[w] = 0;
   __syncwarp();
 }
 
@@ -1506,9 +1632,8 @@ __device__ __noinline__ void sp_init_partition(const int32_t* color) {
   for (uint32_t w = lane; w < W.nw; w += 32) cells += popc64(W.stb[w]);
   cells = __reduce_add_sync(GCL_FULL, cells);
   // every cell starts active (sequential.cpp:628, refinement with no subsequence)
-  for (uint32_t w = lane; w < W.nw; w += 32) W.act[w] = W.stb[w];
+  for (uint32_t w = lane; w < (n + 31) / 32; w += 32) W.act[w] = ((const uint32_t*)W.stb)[w];
   __syncwarp();
-  bm_resummarize(W.act, W.acts, W.nw, W.nsw);
   if (lane == 0) or_bit32((uint32_t*)W.stb, n);
   __syncwarp();
   bm_resummarize(W.stb, W.sts, W.nw, W.nsw);
@@ -1609,8 +1734,7 @@ __device__ __noinline__ void sp_bind(uint8_t* slot, const SpLayout& Lo, uint32_t
   W.pool_owner = (int32_t*)(slot + Lo.pool_owner);
   W.stb = (uint64_t*)(slot + Lo.stb);
   W.sts = (uint64_t*)(slot + Lo.sts);
-  W.act = (uint64_t*)(slot + Lo.act);
-  W.acts = (uint64_t*)(slot + Lo.acts);
+  W.act = (uint32_t*)(slot + Lo.act);
   W.itm = (uint32_t*)(slot + Lo.itm);
   W.nsb = (uint32_t*)(slot + Lo.nsb);
   W.fcert = (uint32_t*)(slot + Lo.fcert);
@@ -1635,8 +1759,7 @@ __device__ __noinline__ void sp_bind(uint8_t* slot, const SpLayout& Lo, uint32_t
     W.cnt = (uint16_t*)(smem + G.cnt);
     W.stb = (uint64_t*)(smem + G.stb);
     W.sts = (uint64_t*)(smem + G.sts);
-    W.act = (uint64_t*)(smem + G.act);
-    W.acts = (uint64_t*)(smem + G.acts);
+    W.act = (uint32_t*)(smem + G.act);
     W.itm = (uint32_t*)(smem + G.itm);
     W.nsb = (uint32_t*)(smem + G.nsb);
   }
