@@ -146,6 +146,9 @@ extern __shared__ __align__(16) uint8_t sp_dyn[];
 struct SpWarp {
   uint16_t *elem, *pos;  // position -> vertex, vertex -> position (n <= 65536)
   uint16_t* cnt;         // position -> neighbours in the splitter, zero between steps
+  // a block whose other warps count for this one (the first path): the
+  // splitter's positions, equal to end them
+  uint32_t helpers, job_s, job_e;
   uint32_t soff;         // the warp's shared-memory region (offset in sp_dyn), or kNone
   uint32_t *slog, *tmp, *lst1, *hist, *pre;
   uint32_t *seq, *fseq, *bseq, *flabel, *blabel, *dsu;
@@ -509,6 +512,41 @@ __device__ __noinline__ uint32_t sp_fold(uint32_t lc, bool listed) {
   return lc;
 }
 
+// The first path runs on one warp of a block whose other warps wait at named
+// barrier 1 for a splitter to count, and meet it again at barrier 2.
+constexpr uint32_t kSpHelpThreads = 256;
+// members from which the two barriers (about 100 cycles) cost less than the
+// 32-wide count they save (some 300 cycles per 32 members)
+constexpr uint32_t kSpHelpMin = 96;
+__device__ __forceinline__ void sp_block_sync(int id) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kSpHelpThreads) : "memory");
+}
+
+// Thread t of nt: the neighbours of the splitter's vertices [s, e), counted at
+// their positions.
+template <bool kS>
+__device__ __forceinline__ void sp_count(const SpWarp& W, uint32_t s, uint32_t e, uint32_t t,
+                                         uint32_t nt) {
+  const SpRef<kS> R(W);
+  auto add = [&](uint32_t u) {
+    const uint32_t p = R.pos[u];
+    atomicAdd((uint32_t*)R.cnt + (p >> 1), 1u << ((p & 1u) * 16u));
+  };
+  if (e - s <= 8) {  // the threads share each row
+    for (uint32_t q = s; q < e; ++q) {
+      const uint32_t w = R.elem[q];
+      const int32_t f = W.rp[w + 1];
+      for (int32_t i = W.rp[w] + (int32_t)t; i < f; i += (int32_t)nt) add((uint32_t)W.col[i]);
+    }
+    return;
+  }
+  for (uint32_t q = s + t; q < e; q += nt) {
+    const uint32_t w = R.elem[q];
+    const int32_t f = W.rp[w + 1];
+    for (int32_t i = W.rp[w]; i < f; ++i) add((uint32_t)W.col[i]);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // A step whose splitter has more than 32 edges.  Neighbour counts are kept by
 // position, so a cell's counts are contiguous: a lane tests whole small cells
@@ -531,22 +569,17 @@ __device__ __noinline__ SpStep sp_refine_general(uint32_t s, uint32_t e, uint32_
   const bool single = e - s == 1;
   const uint32_t flip = single ? 1u : 0u;  // a neighbour's key is 0, a non-neighbour's 1
   const uint32_t utop0 = utop;
-  auto add = [&](uint32_t u) {
-    const uint32_t p = R.pos[u];
-    atomicAdd((uint32_t*)R.cnt + (p >> 1), 1u << ((p & 1u) * 16u));
-  };
-  if (e - s <= 8) {
-    for (uint32_t q = s; q < e; ++q) {
-      const uint32_t w = R.elem[q];
-      const int32_t f = W.rp[w + 1];
-      for (int32_t i = W.rp[w] + (int32_t)lane; i < f; i += 32) add((uint32_t)W.col[i]);
+  if (W.helpers && e - s >= kSpHelpMin) {
+    if (lane == 0) {
+      W.job_s = s;
+      W.job_e = e;
     }
+    __syncwarp();
+    sp_block_sync(1);
+    sp_count<kS>(W, s, e, lane, kSpHelpThreads);
+    sp_block_sync(2);
   } else {
-    for (uint32_t q = s + lane; q < e; q += 32) {
-      const uint32_t w = R.elem[q];
-      const int32_t f = W.rp[w + 1];
-      for (int32_t i = W.rp[w]; i < f; ++i) add((uint32_t)W.col[i]);
-    }
+    sp_count<kS>(W, s, e, lane, 32);
   }
   for (uint32_t wi = lane; wi < nwd; wi += 32) R.nsb[wi] = sp_nonsingle_word(R.stb, n, wi);
   __syncwarp();
@@ -1096,10 +1129,11 @@ __device__ __forceinline__ void sp_cert_row(const SpWarp& W, uint32_t* cert, int
 // positions of its neighbours in ascending order, stored at its CSR offset --
 // each written once, at its rank in the row (sorting the row in place read back
 // every entry from device memory: 40,400 cycles for a tree of 1,000 vertices).
-__device__ __forceinline__ void sp_leaf_cert(uint32_t* cert) {
-  SpWarp& W = sp_w();
+// Warp `warp` of `warps` takes every warps-th group of 32 rows.
+__device__ __forceinline__ void sp_leaf_cert_part(const SpWarp& W, uint32_t* cert, uint32_t warp,
+                                                  uint32_t warps) {
   const uint32_t lane = lane_id();
-  for (uint32_t v0 = 0; v0 < W.n; v0 += 32) {
+  for (uint32_t v0 = warp * 32; v0 < W.n; v0 += warps * 32) {
     const uint32_t v = v0 + lane;
     int32_t b = 0, d = 0;
     if (v < W.n) {
@@ -1133,6 +1167,10 @@ __device__ __forceinline__ void sp_leaf_cert(uint32_t* cert) {
       }
     }
   }
+}
+
+__device__ __forceinline__ void sp_leaf_cert(uint32_t* cert) {
+  sp_leaf_cert_part(sp_w(), cert, 0, 1);
   __syncwarp();
 }
 
@@ -1644,39 +1682,35 @@ __device__ __noinline__ void sp_init_partition(const int32_t* color) {
   __syncwarp();
 }
 
-// Input checks: indices in range, rows strictly ascending (so no duplicate
-// edge), no loop, and both directions of every edge stored.
-__device__ __noinline__ bool sp_check_input(int64_t m) {
-  SpWarp& W = sp_w();
-  const uint32_t lane = lane_id();
-  const uint32_t n = W.n;
-  bool bad = W.rp[0] != 0 || (int64_t)W.rp[n] != m;
-  for (uint32_t v = lane; v < n && !bad; v += 32) {
-    const int32_t b = W.rp[v], e = W.rp[v + 1];
-    if (b < 0 || e < b || (int64_t)e > m) {
-      bad = true;
-      break;
-    }
+// Input checks, thread t of nt: offsets and indices in range, rows strictly
+// ascending (so no duplicate edge), no loop ...
+__device__ __forceinline__ bool sp_check_rows(const int32_t* rp, const int32_t* col, uint32_t n,
+                                              int64_t m, uint32_t t, uint32_t nt) {
+  if (rp[0] != 0 || (int64_t)rp[n] != m) return false;
+  for (uint32_t v = t; v < n; v += nt) {
+    const int32_t b = rp[v], e = rp[v + 1];
+    if (b < 0 || e < b || (int64_t)e > m) return false;
     int32_t prev = -1;
     for (int32_t i = b; i < e; ++i) {
-      const int32_t u = W.col[i];
-      if (u <= prev || (uint32_t)u >= n || (uint32_t)u == v) {
-        bad = true;
-        break;
-      }
+      const int32_t u = col[i];
+      if (u <= prev || (uint32_t)u >= n || (uint32_t)u == v) return false;
       prev = u;
     }
   }
-  if (__any_sync(GCL_FULL, bad)) return false;
-  for (uint32_t v = lane; v < n && !bad; v += 32) {
-    const int32_t b = W.rp[v], e = W.rp[v + 1];
-    for (int32_t i = b; i < e && !bad; ++i) {
-      const uint32_t u = (uint32_t)W.col[i];
-      int32_t lo = W.rp[u], hi = W.rp[u + 1] - 1;
+  return true;
+}
+// ... and, the rows being right, both directions of every edge stored.
+__device__ __forceinline__ bool sp_check_mates(const int32_t* rp, const int32_t* col, uint32_t n,
+                                               uint32_t t, uint32_t nt) {
+  for (uint32_t v = t; v < n; v += nt) {
+    const int32_t b = rp[v], e = rp[v + 1];
+    for (int32_t i = b; i < e; ++i) {
+      const uint32_t u = (uint32_t)col[i];
+      int32_t lo = rp[u], hi = rp[u + 1] - 1;
       bool found = false;
       while (lo <= hi) {
         const int32_t mid = (lo + hi) >> 1;
-        const uint32_t x = (uint32_t)W.col[mid];
+        const uint32_t x = (uint32_t)col[mid];
         if (x == v) {
           found = true;
           break;
@@ -1686,10 +1720,16 @@ __device__ __noinline__ bool sp_check_input(int64_t m) {
         else
           hi = mid - 1;
       }
-      if (!found) bad = true;
+      if (!found) return false;
     }
   }
-  return !__any_sync(GCL_FULL, bad);
+  return true;
+}
+
+__device__ __noinline__ bool sp_check_input(int64_t m) {
+  const SpWarp& W = sp_w();
+  if (!__all_sync(GCL_FULL, sp_check_rows(W.rp, W.col, W.n, m, lane_id(), 32))) return false;
+  return __all_sync(GCL_FULL, sp_check_mates(W.rp, W.col, W.n, lane_id(), 32));
 }
 
 struct SpResult {
@@ -1749,6 +1789,7 @@ __device__ __noinline__ void sp_bind(uint8_t* slot, const SpLayout& Lo, uint32_t
   W.nw = (n + 63) / 64 + 1;
   W.nsw = (W.nw + 63) / 64 + 1;
   W.stride = Lo.stride;
+  W.helpers = 0;
   W.soff = kNone;
   if (smem && sp_smem_bytes(n) <= smem_bytes) {
     // stage the per-step arrays in this warp's shared memory

@@ -67,7 +67,7 @@ struct WideHdr {
   unsigned long long nodes;
   unsigned long long t0;  // start time (globaltimer ns)
   // how long a level's other items wait for its first item (the probe)
-  // before they start anyway: twice the first path's duration
+  // before they start anyway: three times the first path's duration
   unsigned long long probe_ns;
   // opt-in counters of the items kernel (GCL_OPT_COUNTERS; zeroed by the
   // host before a counted search, untouched otherwise)
@@ -184,6 +184,8 @@ struct WideArgs {
   uint32_t gate;  // level gate: 1 on (a level's items wait for the deeper ones), 0 off, 2 auto
   uint32_t probe;  // under the gate: a level's first item runs before the rest of the level
   uint64_t smem_per_warp;
+  uint64_t smem_first;   // shared memory of the first path's state, 0 = device memory
+  uint32_t items_min, items_max;  // the items kernel runs for searches of this many items
   uint64_t budget_ns;
   uint8_t* out_dense;    // n*n, or null
   uint64_t* out_rows;    // n * ceil(n/64) words, or null
@@ -234,15 +236,70 @@ __device__ __forceinline__ void wide_fail(WideHdr* H, int32_t status) {
 }
 
 // ---------------------------------------------------------------------------
-// 1. First path (one warp).
+// 1. First path: one warp refines and individualizes, with its state in shared
+//    memory when it fits (it has the SM to itself); the block's other warps
+//    take shares of the input check, of large splitters' counts and of the
+//    first leaf's certificate and copies.
+//
+//    Bound by that one warp's chain of steps.  With one warp alone and the
+//    state in device memory a 256-vertex random graph took 550-690 us and one
+//    of 20,000 vertices 91 ms, of which the input check 8 ms and the leaf 5 ms;
+//    now about 120 us and 50 ms.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(32) wide_first_kernel(WideArgs A) {
-  const uint32_t lane = lane_id();
+struct FirstPath {
+  int32_t status;
+  uint32_t level, seqlen;
+  unsigned long long nodes;
+};
+
+// warp 0: the nodes from the root to the first leaf
+__device__ __noinline__ FirstPath wide_first_path(const WideArgs& A, const WidePtrs& P) {
+  SpWarp& W = sp_w();
+  const uint32_t lane = lane_id(), n = A.n;
+  FirstPath r{kInternal, 1, 0, 1};
+  sp_init_partition(A.color);
+  int code = sp_refine();
+  if (code < 0) return r;
+  if (lane == 0) P.fcode[0] = code;
+  __syncwarp();
+  while (W.ncells < n) {
+    const uint32_t t = r.level <= n ? sp_first_nonsingleton() : kNone;
+    if (t == kNone) return r;
+    const uint32_t len = sp_cell_end(W, t) - t;
+    uint32_t v = kNone;
+    for (uint32_t q = t + lane; q < t + len; q += 32) v = min(v, (uint32_t)W.elem[q]);
+    v = __reduce_min_sync(GCL_FULL, v);  // first representative: the least member
+    __syncwarp();
+    if (lane == 0) {
+      P.tcfirst[r.level - 1] = t;
+      P.tclen[r.level - 1] = len;
+      W.seq[r.seqlen] = v;
+    }
+    __syncwarp();
+    ++r.seqlen;
+    ++r.nodes;
+    if (!sp_individualize(r.level, v, t)) return r;
+    code = sp_refine();
+    if (code < 0) return r;
+    ++r.level;
+    __syncwarp();
+    for (uint32_t i = W.umark[r.level - 1] + lane; i < W.utop; i += 32)
+      P.linlev[W.slog[i]] = r.level;
+    if (lane == 0) P.fcode[r.level - 1] = code;
+    __syncwarp();
+  }
+  r.status = kOk;
+  return r;
+}
+
+__global__ void __launch_bounds__(kSpHelpThreads) wide_first_kernel(WideArgs A) {
+  __shared__ FirstPath path;
+  const uint32_t t = threadIdx.x, warp = t >> 5, lane = lane_id();
   const WidePtrs P = wide_ptrs(A);
   WideHdr* H = P.H;
-  SpWarp& W = sp_w();
+  SpWarp& W = g_sp[0];
   const uint32_t n = A.n;
-  if (lane == 0) {
+  if (t == 0) {
     H->D = 0;
     H->nitems = 0;
     H->next_item = 0;
@@ -263,78 +320,63 @@ __global__ void __launch_bounds__(32) wide_first_kernel(WideArgs A) {
     H->nodes = 1;
     H->t0 = global_ns();
   }
-  sp_bind(A.slots, A.Lo, n, A.rp, A.col, nullptr, 0, 0, 1);
-  __syncwarp();
-  if (!sp_check_input(A.m)) {
-    wide_fail(H, kBadInput);
-    return;
+  if (warp == 0) {
+    sp_bind(A.slots, A.Lo, n, A.rp, A.col, A.smem_first ? sp_dyn : nullptr, A.smem_first, 0, 1);
+    __syncwarp();
+    if (lane == 0) W.helpers = 1;
   }
-  sp_init_partition(A.color);
   // level of the node whose refinement (or individualization) made each
   // position a cell start; the root's are level 1
-  for (uint32_t i = lane; i < n; i += 32) P.linlev[i] = 1;
-  int code = sp_refine();
-  if (code < 0) {
-    wide_fail(H, kInternal);
+  for (uint32_t i = t; i < n; i += kSpHelpThreads) P.linlev[i] = 1;
+  bool ok = __syncthreads_and(sp_check_rows(A.rp, A.col, n, A.m, t, kSpHelpThreads)) != 0;
+  if (ok) ok = __syncthreads_and(sp_check_mates(A.rp, A.col, n, t, kSpHelpThreads)) != 0;
+  if (!ok) {
+    if (warp == 0) wide_fail(H, kBadInput);
     return;
   }
-  uint32_t level = 1, seqlen = 0;
-  unsigned long long nodes = 1;
-  if (lane == 0) P.fcode[0] = code;
-  __syncwarp();
-  while (W.ncells < n) {
-    const uint32_t t = level <= n ? sp_first_nonsingleton() : kNone;
-    if (t == kNone) {
-      wide_fail(H, kInternal);
-      return;
-    }
-    const uint32_t len = sp_cell_end(W, t) - t;
-    uint32_t v = kNone;
-    for (uint32_t q = t + lane; q < t + len; q += 32) v = min(v, W.elem[q]);
-    v = __reduce_min_sync(GCL_FULL, v);  // first representative: the least member
-    __syncwarp();
+  if (warp == 0) {
+    const FirstPath r = wide_first_path(A, P);
     if (lane == 0) {
-      P.tcfirst[level - 1] = t;
-      P.tclen[level - 1] = len;
-      W.seq[seqlen] = v;
+      path = r;
+      W.job_s = W.job_e = 0;  // ends the helpers
     }
     __syncwarp();
-    ++seqlen;
-    ++nodes;
-    if (!sp_individualize(level, v, t)) {
-      wide_fail(H, kInternal);
-      return;
+    sp_block_sync(1);
+  } else {
+    while (true) {
+      sp_block_sync(1);
+      const uint32_t s = W.job_s, e = W.job_e;
+      if (s == e) break;
+      if (W.soff != kNone)
+        sp_count<true>(W, s, e, t, kSpHelpThreads);
+      else
+        sp_count<false>(W, s, e, t, kSpHelpThreads);
+      sp_block_sync(2);
     }
-    code = sp_refine();
-    if (code < 0) {
-      wide_fail(H, kInternal);
-      return;
-    }
-    ++level;
-    __syncwarp();
-    for (uint32_t i = W.umark[level - 1] + lane; i < W.utop; i += 32)
-      P.linlev[W.slog[i]] = level;
-    if (lane == 0) P.fcode[level - 1] = code;
-    __syncwarp();
+  }
+  __syncthreads();
+  if (path.status != kOk) {
+    if (warp == 0) wide_fail(H, path.status);
+    return;
   }
   // the first leaf: certificate, labeling, partition, and the initial best
-  const uint32_t D = level;
-  sp_leaf_cert(P.fcert);
-  for (uint32_t i = lane; i < n; i += 32) {
+  const uint32_t D = path.level, seqlen = path.seqlen;
+  sp_leaf_cert_part(W, P.fcert, warp, kSpHelpThreads / 32);
+  for (uint32_t i = t; i < n; i += kSpHelpThreads) {
     const uint32_t e = W.elem[i];
     P.flabel[i] = e;
     P.blabel[i] = e;
     P.lelem[i] = e;
   }
-  for (uint32_t i = lane; i < seqlen; i += 32) {
+  for (uint32_t i = t; i < seqlen; i += kSpHelpThreads) {
     P.fseq[i] = W.seq[i];
     P.bseq[i] = W.seq[i];
   }
-  for (uint32_t w = lane; w < W.nw; w += 32) P.lstb[w] = W.stb[w];
-  for (int64_t i = lane; i < A.m; i += 32) P.bcert[i] = P.fcert[i];
-  for (uint32_t i = lane; i < D; i += 32) P.bcode[i] = P.fcode[i];
-  __syncwarp();
-  if (lane == 0) {
+  for (uint32_t w = t; w < W.nw; w += kSpHelpThreads) P.lstb[w] = W.stb[w];
+  for (uint32_t i = t; i < D; i += kSpHelpThreads) P.bcode[i] = P.fcode[i];
+  __syncthreads();  // the certificate is whole
+  for (int64_t i = t; i < A.m; i += kSpHelpThreads) P.bcert[i] = P.fcert[i];
+  if (t == 0) {
     P.fcode[D] = kSentinel;
     P.bcode[D] = kSentinel;
     // items of node level L = D-1 .. 1: its target cell minus the first-path
@@ -349,11 +391,11 @@ __global__ void __launch_bounds__(32) wide_first_kernel(WideArgs A) {
     H->D = D;
     H->best_level = D;
     H->best_seqlen = seqlen;
-    H->nodes = nodes;
+    H->nodes = path.nodes;
     // automatic gate: off when the levels hold fewer than 4 items each on
     // average (trees), where it would run the items one after another
     H->gate = A.gate == 2 ? (run >= 4u * (D - 1u) ? 1u : 0u) : (A.gate != 0 ? 1u : 0u);
-    H->probe_ns = max(2ull * (global_ns() - H->t0), 20000ull);
+    H->probe_ns = max(3ull * (global_ns() - H->t0), 20000ull);
     __threadfence();
     H->nitems = run;
   }
@@ -1020,12 +1062,12 @@ __global__ void __launch_bounds__(kSpThreads) wide_items_kernel(WideArgs A) {
   const uint32_t lane = lane_id();
   const WidePtrs P = wide_ptrs(A);
   WideHdr* H = P.H;
-  if (H->status != kOk || H->nitems == 0) return;
+  if (H->status != kOk || H->nitems < A.items_min || H->nitems > A.items_max) return;
   WideCnt<kCount> cnt;
   const unsigned long long t_start = cnt.now();
   SpWarp& W = sp_w();
   const uint32_t n = A.n, D = H->D, nitems = H->nitems, cap = A.WL.cap;
-  uint8_t* slot = A.slots + ((uint64_t)blockIdx.x * kSpWarps + (uint64_t)warp) * A.slot_bytes;
+  uint8_t* slot = A.slots + ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (uint64_t)warp) * A.slot_bytes;
   uint8_t* smem = A.smem_per_warp ? sp_dyn + (uint64_t)warp * A.smem_per_warp : nullptr;
   sp_bind(slot, A.Lo, n, A.rp, A.col, smem, A.smem_per_warp, 0, cap);
   __syncwarp();
@@ -1121,7 +1163,7 @@ __global__ void __launch_bounds__(kSpThreads) wide_items_kernel(WideArgs A) {
         const unsigned long long tc = cnt.now();
         int32_t gs = wide_gate(H, P.cum[lo], deadline);
         // with the probe, the level's other items also wait for its first
-        // item, up to twice the first path's duration: the automorphisms
+        // item, up to three times the first path's duration: the automorphisms
         // that one finds prune them (it is done when `done` passes the
         // deeper levels' items, since no other item of the level can finish
         // before it)
