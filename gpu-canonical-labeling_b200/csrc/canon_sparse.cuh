@@ -317,16 +317,8 @@ struct SpRef {
   __device__ __forceinline__ bool active(uint32_t c) const {
     return (act[c >> 5] >> (c & 31u)) & 1u;
   }
-  // the cell [c, e) of position p.  Cells are short once a refinement is under
-  // way: the words beside p's are tried before the summary.
-  __device__ __forceinline__ uint32_t start_of(uint32_t p) const {
-    uint32_t w = p >> 5, x = st[w] & (0xffffffffu >> (31u - (p & 31u)));
-    for (int far = 0; !x; ++far) {
-      if (far == 4) return bm_prev(stb, sts, w * 32 - 1);
-      x = st[--w];
-    }
-    return w * 32 + 31u - (uint32_t)__clz((int)x);
-  }
+  // the end of the cell of position p.  Cells are short once a refinement is
+  // under way: the words beside p's are tried before the summary.
   __device__ __forceinline__ uint32_t end_of(uint32_t p, uint32_t n) const {
     uint32_t w = p >> 5, x = st[w] & (0xfffffffeu << (p & 31u));
     for (int far = 0; !x; ++far) {
@@ -334,6 +326,26 @@ struct SpRef {
       x = st[++w];
     }
     return w * 32 + (uint32_t)__ffs((int)x) - 1u;
+  }
+  // the start c and length of the cell of position p
+  __device__ __forceinline__ void cell_of(uint32_t p, uint32_t n, uint32_t* c, uint32_t* len) const {
+    const uint32_t w = p >> 5, x = st[w], sh = p & 31u;
+    const uint32_t lo = x & (0xffffffffu >> (31u - sh)), hi = x & (0xfffffffeu << sh);
+    uint32_t a = 0, e = 0;
+    if (lo) {
+      a = w * 32 + 31u - (uint32_t)__clz((int)lo);
+    } else {
+      uint32_t v = w, y = 0;
+      for (int far = 0; far < 4 && !y; ++far) y = st[--v];  // position 0 is a start
+      a = y ? v * 32 + 31u - (uint32_t)__clz((int)y) : bm_prev(stb, sts, v * 32 - 1);
+    }
+    if (hi) {
+      e = w * 32 + (uint32_t)__ffs((int)hi) - 1u;
+    } else {
+      e = end_of(w * 32 + 31u, n);
+    }
+    *c = a;
+    *len = e - a;
   }
 };
 
@@ -681,22 +693,25 @@ __device__ __noinline__ SpStep sp_refine_general(uint32_t s, uint32_t e, uint32_
           continue;
         }
         const uint32_t range = mx - mn + 1;
-        for (uint32_t i = lane; i < range; i += 32) W.hist[i] = 0;
+        // counts and offsets by key: in shared memory for up to 64 keys
+        uint32_t* const hist = range <= 64 ? (uint32_t*)W.list : W.hist;
+        uint32_t* const pre = range <= 64 ? (uint32_t*)W.list + 64 : W.pre;
+        for (uint32_t i = lane; i < range; i += 32) hist[i] = 0;
         __syncwarp();
         for (uint32_t i = lane; i < L; i += 32)
-          atomicAdd(&W.hist[(uint32_t)(R.cnt[c + i] - mn) ^ flip], 1u);
+          atomicAdd(&hist[(uint32_t)(R.cnt[c + i] - mn) ^ flip], 1u);
         __syncwarp();
         // fragment starts (relative) and the first largest fragment
         uint32_t run = 0, best = 0, bestf = 0;
         for (uint32_t i0 = 0; i0 < range; i0 += 32) {
-          const uint32_t i = i0 + lane, h = i < range ? W.hist[i] : 0u;
+          const uint32_t i = i0 + lane, h = i < range ? hist[i] : 0u;
           uint32_t incl = h;
           for (int o = 1; o < 32; o <<= 1) {
             const uint32_t y = __shfl_up_sync(GCL_FULL, incl, o);
             if (lane >= (uint32_t)o) incl += y;
           }
           const uint32_t f = run + incl - h;
-          if (i < range) W.pre[i] = f;
+          if (i < range) pre[i] = f;
           const uint32_t mxh = __reduce_max_sync(GCL_FULL, h);
           if (mxh > best) {
             best = mxh;
@@ -706,18 +721,18 @@ __device__ __noinline__ SpStep sp_refine_general(uint32_t s, uint32_t e, uint32_
         }
         __syncwarp();
         if (single) {
-          split_single(c, W.hist[0], W.hist[1], was);
+          split_single(c, hist[0], hist[1], was);
         } else {
           for (uint32_t i0 = 0; i0 < range; i0 += 32) {
-            const uint32_t i = i0 + lane, h = i < range ? W.hist[i] : 0u;
-            const uint32_t f = i < range ? W.pre[i] : 0u;
+            const uint32_t i = i0 + lane, h = i < range ? hist[i] : 0u;
+            const uint32_t f = i < range ? pre[i] : 0u;
             fragment(h != 0, c, c + f, h, mn + i, was ? f != 0 : f != bestf);
           }
         }
         __syncwarp();
         for (uint32_t i = lane; i < L; i += 32) {
           const uint32_t a = R.cnt[c + i];
-          W.tmp[atomicAdd(&W.pre[(a - mn) ^ flip], 1u)] = (a << 16) | R.elem[c + i];
+          W.tmp[atomicAdd(&pre[(a - mn) ^ flip], 1u)] = (a << 16) | R.elem[c + i];
         }
         __syncwarp();
         for (uint32_t i = lane; i < L; i += 32) {
@@ -772,6 +787,8 @@ __device__ __noinline__ int sp_refine_t() {
   uint32_t* const slog = W.slog;
   // the splitter: the first active position from the hint on, else from 0
   auto next_active = [&]() -> uint32_t {
+    const uint32_t near = R.act[hint >> 5] >> (hint & 31u);
+    if (near) return hint + (uint32_t)__ffs((int)near) - 1;
     if (nwd <= 32) {  // a word per lane
       const uint32_t w = lane < nwd ? R.act[lane] : 0u, hw = hint >> 5;
       const uint32_t ge = lane > hw ? w : lane == hw ? w & (0xffffffffu << (hint & 31u)) : 0u;
@@ -784,8 +801,6 @@ __device__ __noinline__ int sp_refine_t() {
       const uint32_t src = (uint32_t)__ffs((int)m) - 1;
       return src * 32 + (uint32_t)__ffs((int)__shfl_sync(GCL_FULL, x, (int)src)) - 1;
     }
-    const uint32_t near = R.act[hint >> 5] >> (hint & 31u);
-    if (near) return hint + (uint32_t)__ffs((int)near) - 1;
     // four words per lane from the word after the hint's, then from word 0
     const uint32_t from = (hint >> 5) + 1, wp = sp_pad_words(n);
     for (int wrap = 0; wrap < 2; ++wrap)
@@ -819,15 +834,14 @@ __device__ __noinline__ int sp_refine_t() {
       ok = 0;
       break;
     }
-    const uint32_t e = (R.st[(s + 1) >> 5] >> ((s + 1) & 31u)) & 1u ? s + 1 : R.end_of(s, n);
+    const uint32_t w = R.elem[s];
+    const bool one = R.alone(s);
+    const int32_t sb = rp[w], sd = rp[w + 1] - sb;
     __syncwarp();
     if (lane == 0) atomicAnd(R.act + (s >> 5), ~(1u << (s & 31u)));
     nact -= 1;
-    const uint32_t len = e - s;
-    lc = (lc ^ C) + (s + e - 1);
-    if (len == 1) {
-      const uint32_t w = R.elem[s];
-      const int32_t sb = rp[w], sd = rp[w + 1] - sb;
+    if (one) {
+      lc = (lc ^ C) + (2 * s);  // split1 + split2
       if (sd <= 32) {
         // Singleton splitter: a cell splits into [neighbours, non-neighbours]
         // when only some of its vertices are neighbours (:296-309, 399-435).
@@ -840,10 +854,7 @@ __device__ __noinline__ int sp_refine_t() {
         }
         __syncwarp();
         if (!__any_sync(GCL_FULL, on)) continue;
-        if (on) {
-          c = R.start_of(p);
-          L = R.end_of(p, n) - c;
-        }
+        if (on) R.cell_of(p, n, &c, &L);
         const uint32_t grp = __match_any_sync(GCL_FULL, c);
         const uint32_t k = (uint32_t)__popc(grp);
         const bool spl = on && k < L;
@@ -864,9 +875,9 @@ __device__ __noinline__ int sp_refine_t() {
         } else {
           mv = spl && p != c;
         }
+        const bool lead = spl && (grp & lt) == 0;
+        const bool was = R.active(lead ? c : 0);
         if (mv) x = R.elem[h];
-        const bool lead = spl && lane == (uint32_t)(__ffs((int)grp) - 1);
-        const bool was = lead && R.active(c);
         const uint32_t leaders = __ballot_sync(GCL_FULL, lead);
         const uint32_t made = (uint32_t)__popc(leaders);
         __syncwarp();
@@ -876,12 +887,13 @@ __device__ __noinline__ int sp_refine_t() {
           R.elem[p] = (uint16_t)x;
           R.pos[x] = (uint16_t)p;
         }
-        uint32_t hv = 0, key = kNone;
+        // key: start, neighbours and whether the split sets the hint to its
+        // first (1) or second (2) fragment
+        uint32_t key = kNone;
         if (lead) {
           const uint32_t pp = c + k, nn = L - k;
           const bool rest = was || k >= nn;
-          hv = rest ? (nn == 1 ? pp + 1 : 0u) : (k == 1 ? c + 1 : 0u);
-          key = (c << 6) | k;
+          key = (c << 8) | (k << 2) | (rest ? (nn == 1 ? 2u : 0u) : (k == 1 ? 1u : 0u));
           slog[utop + (uint32_t)__popc(leaders & lt)] = pp;
           bm_or(R.stb, R.sts, pp);
           or_bit32(R.act, rest ? pp : c);
@@ -891,23 +903,26 @@ __device__ __noinline__ int sp_refine_t() {
         nact += made;
         // hash (cell.first + neighbors_size - 1) in position order; the hint
         // is the last split cell's that sets one
-        if (made == 1) {
-          key = __shfl_sync(GCL_FULL, key, __ffs((int)leaders) - 1);
-          hv = __shfl_sync(GCL_FULL, hv, __ffs((int)leaders) - 1);
-          lc = (lc ^ C) + ((key >> 6) + (key & 63u) - 1);
-        } else {
-          for (uint32_t i = 0; i < made; ++i) {
-            const uint32_t m = __reduce_min_sync(GCL_FULL, key);
-            if (key == m) key = kNone;
-            lc = (lc ^ C) + ((m >> 6) + (m & 63u) - 1);
+        for (uint32_t i = 0; i < made; ++i) {
+          uint32_t x;
+          if (made == 1) {
+            x = __shfl_sync(GCL_FULL, key, __ffs((int)leaders) - 1);
+          } else {
+            x = __reduce_min_sync(GCL_FULL, key);
+            if (key == x) key = kNone;
           }
-          hv = __reduce_max_sync(GCL_FULL, hv);
+          const uint32_t cc = x >> 8, pp = cc + ((x >> 2) & 63u);
+          lc = (lc ^ C) + (pp - 1);
+          if (x & 2u) hint = pp;
+          if (x & 1u) hint = cc;
         }
-        if (hv) hint = hv - 1;
         __syncwarp();
         continue;
       }
-    } else {
+    }
+    const uint32_t e = one ? s + 1 : R.end_of(s, n), len = e - s;
+    if (!one) {
+      lc = (lc ^ C) + (s + e - 1);
       lc = (lc ^ C) + len;
     }
     if (len > 1 && len <= 32) {
@@ -945,11 +960,8 @@ __device__ __noinline__ int sp_refine_t() {
         // lanes on the same neighbour: the group's size is its count
         const uint32_t gu = __match_any_sync(GCL_FULL, u);
         const uint32_t cnt = (uint32_t)__popc(gu);
-        const bool lead = u != kNone && lane == (uint32_t)(__ffs((int)gu) - 1);
-        if (lead) {
-          c = R.start_of(p);
-          L = R.end_of(p, n) - c;
-        }
+        const bool lead = u != kNone && (gu & lt) == 0;
+        if (lead) R.cell_of(p, n, &c, &L);
         const uint32_t gc = __match_any_sync(GCL_FULL, c);
         const uint32_t k = (uint32_t)__popc(gc);  // touched vertices of the cell
         // rank by count within the cell: a radix pass over ballots
@@ -968,7 +980,7 @@ __device__ __noinline__ int sp_refine_t() {
         const uint32_t eq = (uint32_t)__popc(peers & lt), size = (uint32_t)__popc(peers);
         const bool uniform = lead && k == L && size == k;  // one common count: no split
         const bool split = lead && !uniform;
-        const bool cell_lead = lead && lane == (uint32_t)(__ffs((int)gc) - 1);
+        const bool cell_lead = lead && (gc & lt) == 0;
         const uint32_t R0 = c + (L - k), f = R0 + less;
         uint32_t h = 0, x = 0, made = 0;
         if (__any_sync(GCL_FULL, split)) {
