@@ -245,10 +245,10 @@ __device__ void bm_resummarize(const uint64_t* B, uint64_t* Sm, uint32_t nw, uin
 }
 
 __device__ __forceinline__ uint32_t sp_cell_end(const SpWarp& W, uint32_t c) {
-  return bm_next(W.stb, W.sts, c + 1, W.n, W.nw, W.nsw);
-}
-__device__ __forceinline__ uint32_t sp_cell_of(const SpWarp& W, uint32_t p) {
-  return bm_prev(W.stb, W.sts, p);
+  const uint32_t* st = (const uint32_t*)W.stb;
+  const uint32_t w = c >> 5, x = st[w] & (0xfffffffeu << (c & 31u));
+  if (x) return w * 32 + (uint32_t)__ffs((int)x) - 1;
+  return bm_next(W.stb, W.sts, (w + 1) * 32, W.n, W.nw, W.nsw);
 }
 __device__ __forceinline__ uint32_t lanemask_lt() {
   uint32_t m;
@@ -1073,8 +1073,8 @@ __device__ __forceinline__ int sp_refine() {
 __device__ __forceinline__ bool sp_individualize(uint32_t level, uint32_t v, uint32_t t) {
   SpWarp& W = sp_w();
   const uint32_t lane = lane_id();
-  const uint32_t e = sp_cell_end(W, t);
-  if (e - t <= 1) return false;
+  const uint32_t* st = (const uint32_t*)W.stb;
+  if ((st[(t + 1) >> 5] >> ((t + 1) & 31u)) & 1u) return false;  // a singleton
   __syncwarp();
   if (lane == 0) {
     W.umark[level] = W.utop;  // backtracking to `level` undoes from here
@@ -1189,23 +1189,38 @@ __device__ __forceinline__ void sp_leaf_cert(uint32_t* cert) {
 // Compare the certificate rows of the current leaf (vertex order elem[])
 // with a stored leaf (vertex order label[], rows in cert2) in canonical
 // row order.  upper: compare_adj_upper (entries right of the diagonal,
-// sequential.cpp:114-124); otherwise full-row equality.  Returns -1/0/+1.
+// sequential.cpp:114-124), -1/0/+1; otherwise 0 when every row is equal.
 template <bool kCg = false>
 __device__ __forceinline__ int sp_cmp_leaf(const uint32_t* cur, const uint32_t* label,
                                         const uint32_t* cert2, bool upper) {
   SpWarp& W = sp_w();
   const uint32_t lane = lane_id();
   const uint32_t n = W.n;
+  if (!upper) {  // equal rows or not: every entry's load is independent
+    for (uint32_t i0 = 0; i0 < n; i0 += 32) {
+      const uint32_t i = i0 + lane;
+      bool differ = false;
+      if (i < n) {
+        const uint32_t va = W.elem[i], vb = ldx<kCg>(label + i);
+        const int32_t a = W.rp[va], b = W.rp[vb], d = W.rp[va + 1] - a;
+        differ = W.rp[vb + 1] - b != d;
+        if (!differ) {
+#pragma unroll 4
+          for (int32_t k = 0; k < d; ++k) differ |= cur[a + k] != ldx<kCg>(cert2 + b + k);
+        }
+      }
+      if (__any_sync(GCL_FULL, differ)) return 1;
+    }
+    return 0;
+  }
   for (uint32_t i0 = 0; i0 < n; i0 += 32) {
     const uint32_t i = i0 + lane;
     int r = 0;
     if (i < n) {
       const uint32_t va = W.elem[i], vb = ldx<kCg>(label + i);
       int32_t a = W.rp[va], ae = W.rp[va + 1], b = W.rp[vb], be = W.rp[vb + 1];
-      if (upper) {
-        while (a < ae && cur[a] <= i) ++a;
-        while (b < be && ldx<kCg>(cert2 + b) <= i) ++b;
-      }
+      while (a < ae && cur[a] <= i) ++a;
+      while (b < be && ldx<kCg>(cert2 + b) <= i) ++b;
       while (true) {
         const bool ea = a >= ae, eb = b >= be;
         if (ea && eb) break;
@@ -1259,22 +1274,13 @@ __device__ __forceinline__ int sp_gca(const uint32_t* a, uint32_t na, uint32_t s
 __device__ __forceinline__ uint32_t sp_first_nonsingleton() {
   SpWarp& W = sp_w();
   const uint32_t lane = lane_id();
-  const uint32_t n = W.n, nw = (n + 63) / 64;
-  for (uint32_t w0 = 0; w0 < nw; w0 += 32) {
-    const uint32_t w = w0 + lane;
-    uint64_t ns = 0;
-    if (w < nw) {
-      const uint64_t b = W.stb[w];
-      ns = b & ~((b >> 1) | (W.stb[w + 1] << 63));  // starts whose successor is none
-      if (n - w * 64 < 64) ns &= low_mask(n - w * 64);  // position n is marked as a start
-    }
-    const uint32_t bal = __ballot_sync(GCL_FULL, ns != 0);
-    if (bal) {
-      const int src = __ffs(bal) - 1;
-      const uint32_t p = (uint32_t)src + w0;
-      const uint64_t x = bcast64(ns, src);
-      return p * 64 + ctz64(x);
-    }
+  const uint32_t n = W.n, nwd = (n + 31) / 32;
+  for (uint32_t w0 = 0; w0 < nwd; w0 += 32) {
+    const uint32_t x = w0 + lane < nwd ? sp_nonsingle_word(W.stb, n, w0 + lane) : 0u;
+    const uint32_t m = __ballot_sync(GCL_FULL, x != 0);
+    if (!m) continue;
+    const uint32_t src = (uint32_t)__ffs((int)m) - 1;
+    return (w0 + src) * 32 + (uint32_t)__ffs((int)__shfl_sync(GCL_FULL, x, (int)src)) - 1;
   }
   return kNone;
 }
@@ -1303,11 +1309,15 @@ __device__ __forceinline__ uint32_t sp_next_rep(const SpTc& t) {
 // to level Lv; their target-cell headers are still in place).
 __device__ __forceinline__ void sp_pool_pop(uint32_t Lv) {
   SpWarp& W = sp_w();
+  const uint32_t lane = lane_id(), f = W.pool_frames;
+  uint32_t keep = 0;  // frames of levels above Lv (owners ascend)
+  for (uint32_t i0 = 0; i0 < f; i0 += 32)
+    keep += (uint32_t)__popc(
+        __ballot_sync(GCL_FULL, i0 + lane < f && W.pool_owner[i0 + lane] < (int32_t)Lv));
   __syncwarp();
-  if (lane_id() == 0) {
-    uint32_t f = W.pool_frames;
-    while (f > 0 && W.pool_owner[f - 1] >= (int32_t)Lv) W.pool_top = W.tc[W.pool_owner[--f]].rslot;
-    W.pool_frames = f;
+  if (lane == 0 && keep < f) {
+    W.pool_top = W.tc[W.pool_owner[keep]].rslot;
+    W.pool_frames = keep;
   }
   __syncwarp();
 }
@@ -1522,8 +1532,8 @@ __device__ __noinline__ int32_t sp_orbits(int idx, int num_aut, uint32_t seqlen)
     const uint32_t w0 = (uint32_t)from / 32, w1 = (uint32_t)(limit - 1) / 32;
     for (uint32_t wb = w0; wb <= w1; wb += 32) {
       const uint32_t nwd = min(32u, w1 - wb + 1);
-      const uint32_t per = nwd <= 1 ? 1u : 1u << (32 - __clz((int)nwd - 1));
-      const uint32_t wl = lane & (per - 1), row = lane / per, rows = 32 / per;
+      const uint32_t lg = nwd <= 1 ? 0u : 32u - (uint32_t)__clz((int)nwd - 1), per = 1u << lg;
+      const uint32_t wl = lane & (per - 1), row = lane >> lg, rows = 32u >> lg;
       uint32_t fs = 0xffffffffu, fc = 0xffffffffu;
       if (wl < nwd) {
         const uint32_t* F = W.fixm + wb + wl;
@@ -1565,9 +1575,13 @@ __device__ __noinline__ int32_t sp_orbits(int idx, int num_aut, uint32_t seqlen)
   }
   uint32_t* rw = W.reps + t.rslot;
   if (small) {
-    const uint32_t g = __match_any_sync(GCL_FULL, o.comp);
-    const uint32_t r = __reduce_min_sync(g, o.v);
-    if (lane < t.len) rw[lane] = o.v | (r << 16);
+    // the least vertex of each component (a reduction per component, one after
+    // the other, took 3,200 of the 7,400 cycles of a call)
+    W.scr[lane] = kNone;
+    __syncwarp();
+    if (lane < t.len) atomicMin(&W.scr[o.comp], o.v);
+    __syncwarp();
+    if (lane < t.len) rw[lane] = o.v | (W.scr[o.comp] << 16);
   } else {
     for (uint32_t i = lane; i < t.len; i += 32) {
       const uint32_t v = mem[i];
