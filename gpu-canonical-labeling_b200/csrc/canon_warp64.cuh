@@ -83,9 +83,9 @@ struct __align__(16) W64Smem {
   uint32_t dsu[kW64MaxN];
   uint16_t firstcode[kW64Levels];
   uint16_t canoncode[kW64Levels];
-  uint8_t cs[kW64MaxN];     // vertex -> start position of its cell
-  uint8_t inlev[kW64MaxN];  // cell start position -> in_level
-  uint8_t fk[kW64MaxN];     // fragment start position -> its neighbour count
+  uint64_t lst[kW64Levels];  // cell starts of the path's node of each level
+  alignas(16) uint16_t item[kW64MaxN];  // hash items of a refinement step
+  uint8_t cs[kW64MaxN];      // vertex -> start position of its cell
   uint8_t seq[kW64MaxN];
   uint8_t first_seq[kW64MaxN];
   uint8_t best_seq[kW64MaxN];
@@ -152,22 +152,27 @@ struct W64Refined {
   int ok;
 };
 
-static __device__ __forceinline__ W64Refined w64_refine(int n, uint64_t starts, uint32_t level,
-                                                     uint64_t active) {
+// What bounds it: issue slots while a batch's roots are refined, and one warp's
+// chain of steps in the longest searches, so both count instructions.  The cells
+// a singleton splits (one or two on sparse graphs) are taken one after the other
+// with every value uniform -- no reductions or shuffles; a non-singleton step
+// works by vertex, each fragment's least vertex writing its hash item, instead
+// of by position; no in_level is kept (see w64_backtrack).
+static __device__ __forceinline__ W64Refined w64_refine(int n, uint64_t starts, uint64_t active) {
   W64Smem& S = w64_smem();
+  constexpr uint32_t C = 065435u;
   const uint32_t lane = lane_id();
   const uint64_t full = low_mask((uint32_t)n);
   const uint32_t v0 = lane, v1 = lane + 32;
   const bool ok0 = v0 < (uint32_t)n, ok1 = v1 < (uint32_t)n;
   const uint64_t adj0 = ok0 ? S.adj[v0] : 0ull, adj1 = ok1 ? S.adj[v1] : 0ull;
-  const uint32_t lvl1 = level + 1;
   const uint64_t lastbit = bit64((uint32_t)n - 1);
   uint64_t sing = S.sing;
   uint32_t lc = popc64(starts), hint = 0, iters = 0;
   int ok = 1;
   // registers: the member masks of the cells starting at positions lane and
   // lane + 32 (valid where `starts` has the bit), and the cells of vertices
-  // lane and lane + 32
+  // lane and lane + 32 (in shared memory again when the refinement ends)
   uint64_t cmr0 = S.cmask[v0], cmr1 = S.cmask[v1];
   uint32_t csr0 = ok0 ? S.cs[v0] : 0u, csr1 = ok1 ? S.cs[v1] : 0u;
   while (starts != full && active) {
@@ -176,235 +181,178 @@ static __device__ __forceinline__ W64Refined w64_refine(int n, uint64_t starts, 
       break;
     }
     // splitter: hint if active, else the next active after it, else wrap
-    uint32_t s;
-    if ((active >> hint) & 1ull) {
-      s = hint;
-    } else {
-      const uint64_t a = active & ge_mask(hint + 1);
-      s = ctz64(a ? a : active);
-    }
+    const uint64_t ah = active & (~0ull << hint);
+    const uint32_t s = ctz64(ah ? ah : active);
     active &= ~bit64(s);
-    const uint64_t nx = starts & ge_mask(s + 1);
-    const uint32_t e = nx ? ctz64(nx) : (uint32_t)n;
-    lc = mash(lc, s + e - 1);  // split1 + split2
-    if (e - s == 1) {
+    const uint64_t ends = (starts >> 1) | lastbit;  // last positions of the cells
+    if ((ends >> s) & 1ull) {
+      lc = (lc ^ C) + 2 * s;  // split1 + split2
       // Singleton splitter {w}: a cell splits into [neighbours, non-neighbours]
-      // when N(w) meets it partially.  Only neighbours outside singleton
-      // cells can be in such a cell, so most steps end here.
+      // when N(w) meets it partially (:296-465).  Only neighbours outside
+      // singleton cells can be in such a cell, so most steps end here.
       const uint64_t N = S.adj[S.pv[s]];
-      const uint64_t X = N & ~sing;
-      if (!X) continue;
-      // a cell splits when N meets it partially: the lanes test the cells
-      // starting at their two positions
+      if (!(N & ~sing)) continue;
       const bool sp0 = ((starts >> v0) & 1ull) && (cmr0 & N) && (cmr0 & ~N);
       const bool sp1 = ((starts >> v1) & 1ull) && (cmr1 & N) && (cmr1 & ~N);
-      const uint64_t splitc = ballot2(sp0, sp1);
-      if (!splitc) continue;
-      // The split cells, each by the lane owning its start (:296-465): the
-      // neighbours keep the start c, the rest start at p = c + |C & N|.
-      // Cells are disjoint ranges, and whether c was active does not depend
-      // on the cells before it, so they split independently; only the hash
-      // and the hint follow position order (below).
-      uint64_t addA = 0, addS = 0, addG = 0;  // active, starts, singleton additions
-      uint32_t hv0 = 0xffu, hv1 = 0xffu, nbp = 0;
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        if (!(k ? sp1 : sp0)) continue;
-        const uint32_t c = k ? v1 : v0;
-        const uint64_t C = k ? cmr1 : cmr0, CN = C & N, CR = C & ~N;
-        const uint32_t nb = popc64(CN), nn = popc64(CR), p = c + nb;
-        uint32_t hv = 0xffu;
-        if (((active >> c) & 1ull) || nb >= nn) {
-          addA |= bit64(p);
-          if (nn == 1) hv = p;
-        } else {
-          addA |= bit64(c);
-          if (nb == 1) hv = c;
-        }
-        addS |= bit64(p);
-        if (nb == 1) addG |= CN;
-        if (nn == 1) addG |= CR;
-        S.cmask[c] = CN;
-        S.cmask[p] = CR;
-        S.inlev[p] = S.inlev[c];
-        S.inlev[c] = (uint8_t)lvl1;
-        if (nb == 1) S.pv[c] = (uint8_t)ctz64(CN);
-        if (nn == 1) S.pv[p] = (uint8_t)ctz64(CR);
-        if (k) {
-          cmr1 = CN;
-          hv1 = hv;
-          nbp |= nb << 8;
-        } else {
-          cmr0 = CN;
-          hv0 = hv;
-          nbp |= nb;
-        }
-      }
-      // hash: cell.first + neighbors_size - 1 per split cell, in position order
-      for (uint64_t t = splitc; t; t &= t - 1) {
+      uint64_t t = ballot2(sp0, sp1);
+      if (!t) continue;
+      // the split cells in position order: the neighbours keep the start c,
+      // the rest start at p
+      uint64_t fresh = 0;
+      do {
         const uint32_t c = ctz64(t);
-        const uint32_t w = __shfl_sync(GCL_FULL, nbp, (int)(c & 31u));
-        lc = mash(lc, c + ((c >= 32u ? w >> 8 : w) & 0xffu) - 1u);
-      }
-      // hint: the last split cell in position order that sets one
-      const uint64_t hc = ballot2(hv0 != 0xffu, hv1 != 0xffu);
-      if (hc) {
-        const uint32_t cl = msb64(hc);
-        hint = __shfl_sync(GCL_FULL, cl >= 32u ? hv1 : hv0, (int)(cl & 31u));
-      }
-      active |= warp_or64(addA);
-      const uint64_t NSt = warp_or64(addS);
-      starts |= NSt;
-      sing |= warp_or64(addG);
-      // vertices of split cells outside N move to the second fragment
-      {
-        const uint32_t w0 = __shfl_sync(GCL_FULL, nbp, (int)(csr0 & 31u));
-        const uint32_t w1 = __shfl_sync(GCL_FULL, nbp, (int)(csr1 & 31u));
-        if (ok0 && ((splitc >> csr0) & 1ull) && !((N >> v0) & 1ull)) {
-          csr0 += (csr0 >= 32u ? w0 >> 8 : w0) & 0xffu;
-          S.cs[v0] = (uint8_t)csr0;
+        t &= t - 1;
+        const uint64_t cm = S.cmask[c], CN = cm & N, CR = cm & ~N;
+        const uint32_t nb = popc64(CN), nn = popc64(CR), p = c + nb;
+        lc = (lc ^ C) + (p - 1);  // cell.first + neighbors_size - 1
+        if (((active >> c) & 1ull) || nb >= nn) {
+          active |= bit64(p);
+          if (nn == 1) hint = p;
+        } else {
+          active |= bit64(c);
+          if (nb == 1) hint = c;
         }
-        if (ok1 && ((splitc >> csr1) & 1ull) && !((N >> v1) & 1ull)) {
-          csr1 += (csr1 >= 32u ? w1 >> 8 : w1) & 0xffu;
-          S.cs[v1] = (uint8_t)csr1;
+        fresh |= bit64(p);
+        if (nb == 1) sing |= CN;
+        if (nn == 1) sing |= CR;
+        if ((CR >> v0) & 1ull) csr0 = p;
+        if ((CR >> v1) & 1ull) csr1 = p;
+        if (v0 == c) cmr0 = CN;
+        if (v1 == c) cmr1 = CN;
+        if (v0 == p) cmr0 = CR;
+        if (v1 == p) cmr1 = CR;
+        __syncwarp();  // every lane has read the old mask
+        if (lane == 0) {
+          S.cmask[c] = CN;
+          S.cmask[p] = CR;
+          if (nb == 1) S.pv[c] = (uint8_t)ctz64(CN);
+          if (nn == 1) S.pv[p] = (uint8_t)ctz64(CR);
         }
-      }
+      } while (t);
+      starts |= fresh;
       __syncwarp();
-      // the new fragments' member masks, written by their cells' owners
-      if ((NSt >> v0) & 1ull) cmr0 = S.cmask[v0];
-      if ((NSt >> v1) & 1ull) cmr1 = S.cmask[v1];
     } else {
       // Non-singleton splitter: fragments in ascending neighbour count.
-      lc = mash(lc, e - s);
+      const uint32_t len = ctz64(ends >> s) + 1;
+      lc = (lc ^ C) + (2 * s + len - 1);
+      lc = (lc ^ C) + len;
       const uint64_t spl = S.cmask[s];
-      uint32_t cs0 = csr0, cs1 = csr1;
-      uint64_t cm0 = ok0 ? S.cmask[cs0] : 0ull, cm1 = ok1 ? S.cmask[cs1] : 0ull;
+      const uint64_t om0 = ok0 ? S.cmask[csr0] : 0ull, om1 = ok1 ? S.cmask[csr1] : 0ull;
+      uint64_t cm0 = om0, cm1 = om1;
       const uint32_t k0 = ok0 ? popc64(adj0 & spl) : 0u, k1 = ok1 ? popc64(adj1 & spl) : 0u;
       const uint32_t mx = __reduce_max_sync(GCL_FULL, max(k0, k1));
-      uint32_t lt0 = 0, lt1 = 0;
+      uint32_t cs0 = csr0, cs1 = csr1;
       for (int b = mx ? 31 - __clz((int)mx) : -1; b >= 0; --b) {
         const bool b0 = (k0 >> b) & 1u, b1 = (k1 >> b) & 1u;
         const uint64_t M = ballot2(b0, b1);
         if (b0) {
-          lt0 += popc64(cm0 & ~M);
+          cs0 += popc64(cm0 & ~M);
           cm0 &= M;
         } else {
           cm0 &= ~M;
         }
         if (b1) {
-          lt1 += popc64(cm1 & ~M);
+          cs1 += popc64(cm1 & ~M);
           cm1 &= M;
         } else {
           cm1 &= ~M;
         }
       }
-      cs0 += lt0;
-      cs1 += lt1;
-      const uint64_t ns = (ok0 ? bit64(cs0) : 0ull) | (ok1 ? bit64(cs1) : 0ull);
-      const bool s0 = ok0 && popc64(cm0) == 1, s1 = ok1 && popc64(cm1) == 1;
-      sing = ballot2(s0, s1);
-      __syncwarp();  // every lane has read the old cell masks
-      if (ok0) {
-        S.cs[v0] = (uint8_t)cs0;
-        S.cmask[cs0] = cm0;
-        S.fk[cs0] = (uint8_t)k0;
-        if (s0) S.pv[cs0] = (uint8_t)v0;
-      }
-      if (ok1) {
-        S.cs[v1] = (uint8_t)cs1;
-        S.cmask[cs1] = cm1;
-        S.fk[cs1] = (uint8_t)k1;
-        if (s1) S.pv[cs1] = (uint8_t)v1;
-      }
-      const uint64_t NS = warp_or64(ns) & ~starts;
-      __syncwarp();
+      const uint64_t NS =
+          warp_or64((ok0 ? bit64(cs0) : 0ull) | (ok1 ? bit64(cs1) : 0ull)) & ~starts;
+      const bool s0 = ok0 && (cm0 & (cm0 - 1)) == 0, s1 = ok1 && (cm1 & (cm1 - 1)) == 0;
       // hash items in position order: every start of a non-singleton old
-      // cell (common count) and every new fragment start (:253-373)
-      const uint64_t singles = starts & ((starts >> 1) | lastbit);
-      uint64_t t = (starts & ~singles) | NS;
-      while (t) {
-        const uint32_t p = ctz64(t);
-        t &= t - 1;
-        lc = mash(lc, (uint32_t)S.fk[p] + p);
+      // cell (common count) and every new fragment start (:253-373), each
+      // written by the fragment's least vertex
+      const uint64_t T = (starts & ~ends) | NS;
+      if (ok0 && !(cm0 & low_mask(v0)) && ((T >> cs0) & 1ull))
+        S.item[popc64(T & low_mask(cs0))] = (uint16_t)(k0 + cs0);
+      if (ok1 && !(cm1 & low_mask(v1)) && ((T >> cs1) & 1ull))
+        S.item[popc64(T & low_mask(cs1))] = (uint16_t)(k1 + cs1);
+      __syncwarp();  // ... and every lane has read the old cell masks
+      {
+        // bits above 14 never come down: two items per word, no masking
+        const uint4* l4 = (const uint4*)S.item;
+        const uint32_t m = popc64(T);
+        auto two = [&](uint32_t x) {
+          lc = (lc ^ C) + x;
+          lc = (lc ^ C) + (x >> 16);
+        };
+        for (uint32_t q = 0; q < m / 8; ++q) {
+          const uint4 x = l4[q];
+          two(x.x);
+          two(x.y);
+          two(x.z);
+          two(x.w);
+        }
+        if (m & 7u) {
+          const uint4 x = l4[m / 8];
+          uint32_t a = x.x, b = x.y;
+          if (m & 4u) {
+            two(a);
+            two(b);
+            a = x.z;
+            b = x.w;
+          }
+          if (m & 2u) {
+            two(a);
+            a = b;
+          }
+          if (m & 1u) lc = (lc ^ C) + a;
+        }
       }
       if (NS) {
+        sing = ballot2(s0, s1);
         const uint64_t all = starts | NS;
-        // in_level of the fragments of split cells: level+1, the last one
-        // keeps the cell's old in_level (:342, 463-465)
-        uint32_t w0 = 0xffu, w1 = 0xffu;
-        if ((all >> v0) & 1ull) {
-          const uint32_t c = msb64(starts & low_mask(v0 + 1));
-          const uint64_t nc = starts & ge_mask(c + 1);
-          const uint32_t end = nc ? ctz64(nc) : (uint32_t)n;
-          if (NS & low_mask(end) & ge_mask(c + 1))
-            w0 = (v0 == msb64(all & low_mask(end))) ? S.inlev[c] : lvl1;
-        }
-        if ((all >> v1) & 1ull) {
-          const uint32_t c = msb64(starts & low_mask(v1 + 1));
-          const uint64_t nc = starts & ge_mask(c + 1);
-          const uint32_t end = nc ? ctz64(nc) : (uint32_t)n;
-          if (NS & low_mask(end) & ge_mask(c + 1))
-            w1 = (v1 == msb64(all & low_mask(end))) ? S.inlev[c] : lvl1;
-        }
-        // active set (:436-460): every new fragment; for a cell that was not
-        // active, its first fragment in and its first largest fragment out.
-        // hint: the last new singleton fragment in position order.
-        const uint64_t single_all = all & ((all >> 1) | lastbit);
-        const uint64_t hs = NS & single_all;
+        // hint: the last new singleton fragment in position order
+        const uint64_t hs = NS & ((all >> 1) | lastbit);
         if (hs) hint = msb64(hs);
-        // each fragment start of a split cell that was not active offers
-        // (size, -position) for its cell's first largest fragment, one
-        // shared-memory max per cell (S.dsu is free outside the orbits)
-        uint32_t key0 = 0, key1 = 0, cell0 = 0, cell1 = 0;
-        bool fr0 = false, fr1 = false;
-        if ((all >> v0) & 1ull) {
-          cell0 = msb64(starts & low_mask(v0 + 1));
-          const uint64_t nc = starts & ge_mask(cell0 + 1);
-          const uint32_t end = nc ? ctz64(nc) : (uint32_t)n;
-          const uint64_t nf = all & ge_mask(v0 + 1);
-          fr0 = !((active >> cell0) & 1ull) && (NS & low_mask(end) & ge_mask(cell0 + 1)) != 0;
-          key0 = ((min(nf ? ctz64(nf) : (uint32_t)n, end) - v0) << 6) | (63u - v0);
+        // active set (:436-460): every new fragment; for a cell that was not
+        // active, its first fragment in and its first largest fragment out --
+        // each of its vertices offers (size, -start), one shared-memory maximum
+        // per cell (S.dsu is free outside the orbits)
+        const bool fr0 = cm0 != om0 && !((active >> csr0) & 1ull);
+        const bool fr1 = cm1 != om1 && !((active >> csr1) & 1ull);
+        active |= NS;
+        if (__any_sync(GCL_FULL, fr0 || fr1)) {
+          const uint32_t key0 = (popc64(cm0) << 6) | (63u - cs0);
+          const uint32_t key1 = (popc64(cm1) << 6) | (63u - cs1);
+          if (fr0) S.dsu[csr0] = 0;
+          if (fr1) S.dsu[csr1] = 0;
+          __syncwarp();
+          if (fr0) atomicMax(&S.dsu[csr0], key0);
+          if (fr1) atomicMax(&S.dsu[csr1], key1);
+          __syncwarp();
+          const uint64_t in = warp_or64((fr0 ? bit64(csr0) : 0ull) | (fr1 ? bit64(csr1) : 0ull));
+          const uint64_t out = warp_or64((fr0 && S.dsu[csr0] == key0 ? bit64(cs0) : 0ull) |
+                                         (fr1 && S.dsu[csr1] == key1 ? bit64(cs1) : 0ull));
+          active = (active | in) & ~out;
         }
-        if ((all >> v1) & 1ull) {
-          cell1 = msb64(starts & low_mask(v1 + 1));
-          const uint64_t nc = starts & ge_mask(cell1 + 1);
-          const uint32_t end = nc ? ctz64(nc) : (uint32_t)n;
-          const uint64_t nf = all & ge_mask(v1 + 1);
-          fr1 = !((active >> cell1) & 1ull) && (NS & low_mask(end) & ge_mask(cell1 + 1)) != 0;
-          key1 = ((min(nf ? ctz64(nf) : (uint32_t)n, end) - v1) << 6) | (63u - v1);
-        }
-        __syncwarp();
-        if (fr0 && cell0 == v0) S.dsu[cell0] = 0;
-        if (fr1 && cell1 == v1) S.dsu[cell1] = 0;
-        __syncwarp();
-        if (fr0) atomicMax(&S.dsu[cell0], key0);
-        if (fr1) atomicMax(&S.dsu[cell1], key1);
-        __syncwarp();
-        const uint64_t out = ballot2(fr0 && S.dsu[cell0] == key0, fr1 && S.dsu[cell1] == key1);
-        const uint64_t in = ballot2(fr0 && cell0 == v0, fr1 && cell1 == v1);
-        active = (active | NS | in) & ~out;
-        __syncwarp();
-        if (w0 != 0xffu) S.inlev[v0] = (uint8_t)w0;
-        if (w1 != 0xffu) S.inlev[v1] = (uint8_t)w1;
+        if (ok0) S.cmask[cs0] = cm0;
+        if (ok1) S.cmask[cs1] = cm1;
+        if (s0) S.pv[cs0] = (uint8_t)v0;
+        if (s1) S.pv[cs1] = (uint8_t)v1;
         starts = all;
+        csr0 = cs0;
+        csr1 = cs1;
+        __syncwarp();
+        cmr0 = S.cmask[v0];
+        cmr1 = S.cmask[v1];
       }
-      __syncwarp();
-      csr0 = cs0;
-      csr1 = cs1;
-      cmr0 = S.cmask[v0];
-      cmr1 = S.cmask[v1];
+      __syncwarp();  // the items are read before the next step's
     }
   }
-  __syncwarp();
+  if (ok0) S.cs[v0] = (uint8_t)csr0;
+  if (ok1) S.cs[v1] = (uint8_t)csr1;
   if (lane == 0) S.sing = sing;
   __syncwarp();
-  return {starts, cleanup(mash(lc, popc64(starts))), ok};
+  return {starts, cleanup(mash(lc & 077777u, popc64(starts))), ok};
 }
 
 // split_by_and_refine's split (partition_refinement.cpp:486-528): vertex v
 // moves to a singleton cell at t, the rest of the cell starts at t+1.
 // Returns false when the cell is already a singleton (nothing to refine).
-static __device__ __forceinline__ bool w64_individualize(int n, uint32_t level, uint32_t v, uint32_t t) {
+static __device__ __forceinline__ bool w64_individualize(int n, uint32_t v, uint32_t t) {
   W64Smem& S = w64_smem();
   const uint32_t lane = lane_id();
   const uint64_t mem = S.cmask[t];
@@ -417,8 +365,6 @@ static __device__ __forceinline__ bool w64_individualize(int n, uint32_t level, 
     const uint64_t rest = mem & ~bit64(v);
     S.cmask[t] = bit64(v);
     S.cmask[t + 1] = rest;
-    S.inlev[t + 1] = S.inlev[t];
-    S.inlev[t] = (uint8_t)(level + 1);
     S.pv[t] = (uint8_t)v;
     uint64_t sg = S.sing | bit64(v);
     if (popc64(rest) == 1) {
@@ -431,78 +377,49 @@ static __device__ __forceinline__ bool w64_individualize(int n, uint32_t level, 
   return true;
 }
 
-// reconstruct_at_level (partition_refinement.cpp:541-604): every maximal run
-// of cells created after level Lv merges with the cell that follows it, and
-// the merged cell takes that cell's in_level.  Returns the new starts mask
-// (0 if the partition is inconsistent).
+// reconstruct_at_level (partition_refinement.cpp:541-604).  It merges every
+// maximal run of cells created below level Lv with the cell that follows it, and
+// a split gives every fragment but the last the new level, so what is left are
+// the starts of the path's node of level Lv: they are kept per level, and no
+// in_level is.  Cells that lost a start take the masks merged into them.
+// Returns the new starts mask.
 static __device__ __forceinline__ uint64_t w64_backtrack(int n, uint64_t starts, uint32_t Lv) {
   W64Smem& S = w64_smem();
   const uint32_t lane = lane_id();
   const uint32_t q0 = lane, q1 = lane + 32;
-  const bool st0 = q0 < (uint32_t)n && ((starts >> q0) & 1ull);
-  const bool st1 = q1 < (uint32_t)n && ((starts >> q1) & 1ull);
-  const bool big0 = st0 && S.inlev[q0] > Lv, big1 = st1 && S.inlev[q1] > Lv;
-  const uint64_t BIG = ballot2(big0, big1);
-  if (!BIG) return starts;
-  bool sv0 = st0, sv1 = st1;
-  if (st0 && q0 > 0 && ((BIG >> msb64(starts & low_mask(q0))) & 1ull)) sv0 = false;
-  if (st1 && ((BIG >> msb64(starts & low_mask(q1))) & 1ull)) sv1 = false;
-  const uint64_t NST = ballot2(sv0, sv1);
-  uint32_t nl0 = 0, nl1 = 0;
+  const uint64_t to = S.lst[Lv], gone = starts & ~to;
+  if (!gone) return to;
+  // starts merged into the surviving cells of the lane's two positions
+  auto merged = [&](uint32_t q) -> uint64_t {
+    if (!((to >> q) & 1ull)) return 0;
+    const uint64_t above = ge_mask(q + 1), next = to & above;
+    return gone & above & low_mask(next ? ctz64(next) : 64u);
+  };
+  const uint64_t g0 = merged(q0), g1 = merged(q1);
   uint64_t m0 = 0, m1 = 0;
-  bool bad = false, w0 = false, w1 = false;
-  if (sv0 && big0) {
-    const uint64_t j = starts & ~BIG & ge_mask(q0 + 1);
-    if (!j) bad = true;
-    else nl0 = S.inlev[ctz64(j)];
-    const uint64_t nn = NST & ge_mask(q0 + 1);
-    uint64_t r = starts & ge_mask(q0) & low_mask(nn ? ctz64(nn) : (uint32_t)n);
-    while (r) {
-      m0 |= S.cmask[ctz64(r)];
-      r &= r - 1;
-    }
-    w0 = true;
-  }
-  if (sv1 && big1) {
-    const uint64_t j = starts & ~BIG & ge_mask(q1 + 1);
-    if (!j) bad = true;
-    else nl1 = S.inlev[ctz64(j)];
-    const uint64_t nn = NST & ge_mask(q1 + 1);
-    uint64_t r = starts & ge_mask(q1) & low_mask(nn ? ctz64(nn) : (uint32_t)n);
-    while (r) {
-      m1 |= S.cmask[ctz64(r)];
-      r &= r - 1;
-    }
-    w1 = true;
-  }
-  if (__any_sync(GCL_FULL, bad)) return 0;
-  __syncwarp();
-  if (w0) {
-    S.inlev[q0] = (uint8_t)nl0;
-    S.cmask[q0] = m0;
-  }
-  if (w1) {
-    S.inlev[q1] = (uint8_t)nl1;
-    S.cmask[q1] = m1;
-  }
-  uint32_t c0 = 0, c1 = 0;
+  for (uint64_t r = g0; r; r &= r - 1) m0 |= S.cmask[ctz64(r)];
+  for (uint64_t r = g1; r; r &= r - 1) m1 |= S.cmask[ctz64(r)];
+  const uint64_t ones = to & ((to >> 1) | bit64((uint32_t)n - 1));
+  bool a0 = false, a1 = false;
   if (q0 < (uint32_t)n) {
-    c0 = msb64(NST & low_mask((uint32_t)S.cs[q0] + 1));
-    S.cs[q0] = (uint8_t)c0;
+    const uint32_t c = msb64(to & low_mask((uint32_t)S.cs[q0] + 1));
+    S.cs[q0] = (uint8_t)c;
+    a0 = (ones >> c) & 1ull;
   }
   if (q1 < (uint32_t)n) {
-    c1 = msb64(NST & low_mask((uint32_t)S.cs[q1] + 1));
-    S.cs[q1] = (uint8_t)c1;
+    const uint32_t c = msb64(to & low_mask((uint32_t)S.cs[q1] + 1));
+    S.cs[q1] = (uint8_t)c;
+    a1 = (ones >> c) & 1ull;
   }
+  // vertices in singleton cells; their pv entries are unchanged (merging
+  // never creates a singleton)
+  const uint64_t sg = ballot2(a0, a1);
   __syncwarp();
-  // vertices in singleton cells after the merge; their pv entries are
-  // unchanged (merging never creates a singleton)
-  const bool g0 = q0 < (uint32_t)n && popc64(S.cmask[c0]) == 1;
-  const bool g1 = q1 < (uint32_t)n && popc64(S.cmask[c1]) == 1;
-  const uint64_t sg = ballot2(g0, g1);
+  if (g0) S.cmask[q0] |= m0;
+  if (g1) S.cmask[q1] |= m1;
   if (lane == 0) S.sing = sg;
   __syncwarp();
-  return NST;
+  return to;
 }
 
 // Certificate rows of the lane's two vertices in a discrete partition: the
@@ -653,14 +570,12 @@ __device__ __forceinline__ void w64_select_tc(int n, uint64_t starts, int tcl) {
 // outside it and cannot change a member's orbit: only permutations that fix
 // the sequence and move a member take part.
 //
-// The merge works on labels that are parent pointers to smaller vertices of
-// the same component.  Every previous orbit is turned into one more
-// permutation (a cycle through its members), so every edge of the union lies
-// on a permutation cycle.  A round pulls the least label over all
-// permutation images of a vertex (independent shared-memory loads), hooks the
-// vertex's old parent under it (atomicMin), and shortcuts parents twice; a
-// round that improves no label ends it, and then every vertex points at the
-// least vertex of its component.  Returns false when the round bound was hit.
+// A target cell of at most 32 vertices -- all but some cells of graphs above 32
+// -- is merged with a lane per member (i-th member in ascending order, so a
+// component's least lane is its least vertex), up to four permutations at a
+// time; the permutations to merge are found with a lane per stored one.
+// Larger cells use a union-find over all vertices (below).  Returns false when
+// a round bound was hit.
 static __device__ __forceinline__ bool w64_orbits(int n, int idx, int num_aut, uint32_t max_aut,
                                                uint32_t seqlen, uint8_t* reps, const uint8_t* auts,
                                                const uint64_t* fixes) {
@@ -672,22 +587,86 @@ static __device__ __forceinline__ bool w64_orbits(int n, int idx, int num_aut, u
   const uint64_t mem = S.tc[idx].members;
   const uint64_t seqm = warp_or64((lane < seqlen ? bit64(S.seq[lane]) : 0ull) |
                                   (lane + 32 < seqlen ? bit64(S.seq[lane + 32]) : 0ull));
-  // taking part: a bit per shared-memory head entry, and whether any later
-  // (device-memory) entry does
-  uint32_t selh = 0;
-  bool seltail = false;
-  for (int i = from; i < limit; ++i) {
+  // whether stored permutation i takes part
+  auto takes_part = [&](int i) {
     const uint64_t fm = i < kW64AutHead ? S.fix_head[i] : fixes[i];
-    if ((seqm & ~fm) || !(mem & ~fm)) continue;
-    if (i < kW64AutHead)
-      selh |= 1u << i;
-    else
-      seltail = true;
-  }
-  if (!selh && !seltail) return true;  // no member's orbit can change
+    return !(seqm & ~fm) && (mem & ~fm) != 0;
+  };
+  // the permutations base .. base + 31 that take part
+  auto selected = [&](int base) {
+    const int i = base + (int)lane;
+    return __ballot_sync(GCL_FULL, i >= from && i < limit && takes_part(i));
+  };
+  int base = from & ~31;
+  uint32_t sel = 0;
+  for (; base < limit; base += 32)
+    if ((sel = selected(base)) != 0) break;
+  if (!sel) return true;  // no member's orbit can change
   const bool rv = S.tc[idx].reps_valid;
   uint8_t* rp = reps + (uint64_t)idx * 64u;
-  const uint32_t v0 = lane, v1 = lane + 32;
+  const uint32_t v0 = lane, v1 = lane + 32, size = popc64(mem);
+  auto image = [&](int i) -> const uint8_t* {
+    return i < kW64AutHead ? S.aut_head[i] : auts + (uint64_t)i * 64u;
+  };
+  if (size <= 32) {
+    if ((mem >> v0) & 1ull) S.map[popc64(mem & low_mask(v0))] = (uint8_t)v0;
+    if ((mem >> v1) & 1ull) S.map[popc64(mem & low_mask(v1))] = (uint8_t)v1;
+    __syncwarp();
+    const bool in = lane < size;
+    const uint32_t v = in ? S.map[lane] : 0u;
+    uint32_t comp = lane;  // the least lane of the member's component
+    if (in && rv) comp = popc64(mem & low_mask((uint32_t)rp[v]));
+    for (;;) {
+      while (sel) {
+        uint32_t j[4], c[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          j[k] = v;
+          if (!sel) continue;
+          const uint8_t* img = image(base + __ffs((int)sel) - 1);
+          sel &= sel - 1;
+          if (in) j[k] = img[v];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) j[k] = in ? popc64(mem & low_mask(j[k])) : lane;
+        for (int round = 0;; ++round) {
+          bool d = false;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            c[k] = __shfl_sync(GCL_FULL, comp, (int)j[k]);
+            d |= c[k] != comp;
+          }
+          if (!__any_sync(GCL_FULL, d)) break;
+          if (round > kW64MaxN) return false;  // a round removes a component
+          S.dsu[lane] = lane;
+          __syncwarp();
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (c[k] != comp) atomicMin(&S.dsu[max(comp, c[k])], min(comp, c[k]));
+          __syncwarp();
+          bool moved;
+          do {  // to the root: links go to smaller lanes
+            const uint32_t r = S.dsu[comp];
+            moved = r != comp;
+            comp = r;
+          } while (__any_sync(GCL_FULL, moved));
+          __syncwarp();
+        }
+      }
+      for (base += 32; base < limit; base += 32)
+        if ((sel = selected(base)) != 0) break;
+      if (!sel) break;
+    }
+    const uint64_t rm = warp_or64(in && comp == lane ? bit64(v) : 0ull);
+    if (in) rp[v] = S.map[comp];
+    __syncwarp();
+    if (lane == 0) {
+      S.tc[idx].repmask = rm;
+      S.tc[idx].reps_valid = 1;
+    }
+    __syncwarp();
+    return true;
+  }
   const bool ok0 = v0 < (uint32_t)n, ok1 = v1 < (uint32_t)n;
   uint32_t L0 = ok0 && ((mem >> v0) & 1ull) && rv ? (uint32_t)rp[v0] : v0;
   uint32_t L1 = ok1 && ((mem >> v1) & 1ull) && rv ? (uint32_t)rp[v1] : v1;
@@ -739,15 +718,13 @@ static __device__ __forceinline__ bool w64_orbits(int n, int idx, int num_aut, u
     return false;
   };
   if (!compress()) return false;
-#pragma unroll 1
-  for (uint32_t k = 0; k < (uint32_t)kW64AutHead; ++k)
-    if (((selh >> k) & 1u) && !apply(S.aut_head[k])) return false;
-  if (seltail)
-    for (int i = max(from, kW64AutHead); i < limit; ++i) {
-      const uint64_t fm = fixes[i];
-      if ((seqm & ~fm) || !(mem & ~fm)) continue;
-      if (!apply(auts + (uint64_t)i * 64u)) return false;
-    }
+  for (;;) {
+    for (; sel; sel &= sel - 1)
+      if (!apply(image(base + __ffs((int)sel) - 1))) return false;
+    for (base += 32; base < limit; base += 32)
+      if ((sel = selected(base)) != 0) break;
+    if (!sel) break;
+  }
   L0 = fp & 0xffu;
   L1 = (fp >> 8) & 0xffu;
   bool r0 = false, r1 = false;
@@ -783,15 +760,21 @@ static __device__ __noinline__ uint64_t w64_load(int n, const int32_t* rp, const
     if (v >= (uint32_t)n) continue;
     uint64_t a = 0;
     const int32_t b = rp[v], e = rp[v + 1];
-    if (b < 0 || e < b || (int64_t)e > m) bad = true;
-    for (int32_t i = b; i < e && !bad; ++i) {
-      const int32_t u = cl[i];
-      if (u < 0 || u >= n || (uint32_t)u == v || ((a >> u) & 1ull)) {
-        bad = true;
-        break;
+    if (b < 0 || e < b || (int64_t)e > m || e - b >= kW64MaxN) bad = true;
+    // four entries' loads at a time: no early exit waits on each of them
+    if (!bad)
+      for (int32_t i = b; i < e; i += 4) {
+        int32_t u[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) u[j] = cl[min(i + j, e - 1)];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (i + j >= e) continue;
+          if ((uint32_t)u[j] >= (uint32_t)n || (uint32_t)u[j] == v || ((a >> (u[j] & 63)) & 1ull))
+            bad = true;
+          a |= bit64((uint32_t)u[j] & 63u);
+        }
       }
-      a |= bit64((uint32_t)u);
-    }
     S.adj[v] = a;
     if (k)
       a1 = a;
@@ -854,8 +837,6 @@ static __device__ __noinline__ uint64_t w64_load(int n, const int32_t* rp, const
                                 lane + 32 < (uint32_t)n && popc64(same1) == 1);
     if (lane == 0) S.sing = sg;
   }
-  if (lane < (uint32_t)n) S.inlev[lane] = 0;
-  if (lane + 32 < (uint32_t)n) S.inlev[lane + 32] = 0;
   __syncwarp();
   return starts;
 }
@@ -885,7 +866,7 @@ static __device__ __noinline__ W64Root w64_root(const BatchArgs& A, int n, int64
     out.status = kBadInput;
     return out;
   }
-  const W64Refined r = w64_refine(n, starts, 0, starts);
+  const W64Refined r = w64_refine(n, starts, starts);
   if (!r.ok) {
     out.status = kInternal;
     return out;
@@ -916,13 +897,15 @@ static __device__ __noinline__ W64Result w64_search_tree(const BatchArgs& A, int
   int64_t nodes = 1;
   int32_t status = kOk;
 
+  if (lane == 0) S.lst[1] = starts;
+  __syncwarp();
   // the next refinement to run on the first path, given by its initially
   // active cells
   uint64_t pending = 0;
   uint64_t iter = 0;
   while (true) {
     if (pending) {
-      const W64Refined r = w64_refine(n, starts, level, pending);
+      const W64Refined r = w64_refine(n, starts, pending);
       pending = 0;
       if (!r.ok) {
         status = kInternal;
@@ -933,7 +916,10 @@ static __device__ __noinline__ W64Result w64_search_tree(const BatchArgs& A, int
       ++level;
       // the first path records its codes (sequential.cpp:254, 630)
       __syncwarp();
-      if (lane == 0) S.firstcode[level - 1] = (uint16_t)code;
+      if (lane == 0) {
+        S.firstcode[level - 1] = (uint16_t)code;
+        S.lst[level] = starts;
+      }
       __syncwarp();
       continue;
     }
@@ -1030,13 +1016,13 @@ static __device__ __noinline__ W64Result w64_search_tree(const BatchArgs& A, int
         __syncwarp();
         ++seqlen;
         ++nodes;
-        if (w64_individualize(n, level, v, t)) {
+        if (w64_individualize(n, v, t)) {
           starts |= bit64(t + 1);
           if (!first_found) {
             pending = bit64(t);  // refine and record firstcode
             continue;
           }
-          const W64Refined rr = w64_refine(n, starts, level, bit64(t));
+          const W64Refined rr = w64_refine(n, starts, bit64(t));
           if (!rr.ok) {
             status = kInternal;
             break;
@@ -1044,6 +1030,8 @@ static __device__ __noinline__ W64Result w64_search_tree(const BatchArgs& A, int
           starts = rr.starts;
           code = rr.code;
           ++level;
+          if (lane == 0) S.lst[level] = starts;
+          __syncwarp();
         } else if (!first_found) {
           __syncwarp();
           if (lane == 0) S.firstcode[level - 1] = (uint16_t)code;
@@ -1156,12 +1144,11 @@ __device__ __forceinline__ uint64_t w64_deadline(const BatchArgs& A) {
 // The partition after the root refinement, handed from the warp that refined
 // the root to the warp that searches below it: a header (starts, singleton
 // vertices, code, graph id), then per vertex or position the adjacency mask, the cell
-// member mask (at cell starts), the cell start, in_level and the singleton
-// cell's vertex -- what the search reads of the root node.  Slots are whole
+// member mask (at cell starts), the cell start and the singleton cell's vertex -- what the search reads of the root node.  Slots are whole
 // 128-byte lines apart, so a warp never holds a line of a neighbouring slot
 // in its L1 from before that slot was written.
 __host__ __device__ constexpr uint64_t w64_root_slot_bytes() {
-  return (32u + (uint64_t)kW64MaxN * (8u + 8u + 3u) + 127u) & ~127ull;
+  return (32u + (uint64_t)kW64MaxN * (8u + 8u + 2u) + 127u) & ~127ull;
 }
 
 static __device__ __noinline__ void w64_save_root(uint8_t* dst, int g, int n, uint64_t starts,
@@ -1182,8 +1169,7 @@ static __device__ __noinline__ void w64_save_root(uint8_t* dst, int g, int n, ui
     adj[v] = S.adj[v];
     cm[v] = S.cmask[v];
     b[v] = S.cs[v];
-    b[kW64MaxN + v] = S.inlev[v];
-    b[2 * kW64MaxN + v] = S.pv[v];
+    b[kW64MaxN + v] = S.pv[v];
   }
 }
 
@@ -1214,8 +1200,7 @@ static __device__ __noinline__ uint64_t w64_restore_root(const uint8_t* src, int
     S.adj[v] = adj[v];
     S.cmask[v] = cm[v];
     S.cs[v] = b[v];
-    S.inlev[v] = b[kW64MaxN + v];
-    S.pv[v] = b[2 * kW64MaxN + v];
+    S.pv[v] = b[kW64MaxN + v];
   }
   const uint64_t starts = h[0];
   *code = (int)(uint32_t)h[2];
