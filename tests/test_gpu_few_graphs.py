@@ -28,3 +28,17 @@ def test_bad_graph_among_few(pkg, G):
     res = pkg.canon_batch([G.torus(5), bad, G.torus(4)], per_graph_errors=True)
     assert res.status.tolist() == [0, 3, 0]
     assert np.array_equal(res.matrix(2), pkg.canon(G.torus(4)).matrix)
+
+
+def test_packed_and_direct_copies_agree(pkg, G):
+    # 13,000 graphs with dense output pass the size up to which a call's arrays
+    # are packed into one copy; halves of it do not
+    pool = G.small_batch(250, seed=9, n_lo=20, n_hi=60)
+    gs = pool * 52
+    whole = pkg.canon_batch(gs, rows=True)
+    half = pkg.canon_batch(gs[: len(gs) // 4], rows=True)
+    assert whole.arena.out_offsets()[-1] > 16 << 20 and (whole.status == 0).all()
+    assert np.array_equal(whole.dense[: half.ooff[-1]], half.dense[: half.ooff[-1]])
+    assert np.array_equal(whole.rows[: half.roff[-1]], half.rows[: half.roff[-1]])
+    assert np.array_equal(whole.stats[: len(half.stats)], half.stats)
+    assert np.array_equal(whole.dense[-half.ooff[-1]:], half.dense[: half.ooff[-1]])
