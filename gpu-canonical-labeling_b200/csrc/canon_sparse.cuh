@@ -1458,6 +1458,10 @@ __device__ __noinline__ int32_t sp_orbits(int idx, int num_aut, uint32_t seqlen)
   // the entries base + i, i a bit of m: kInternal if one does not map the cell
   // onto itself
   auto merge = [&](uint32_t base, uint32_t m) -> int32_t {
+    if (t.len == 2 && !kCg) {  // an entry of the ring that takes part swaps the two
+      any = true;
+      return kOk;
+    }
     if (!any) begin();
     any = true;
     if (small) {
@@ -1574,7 +1578,10 @@ __device__ __noinline__ int32_t sp_orbits(int idx, int num_aut, uint32_t seqlen)
     __syncwarp();
   }
   uint32_t* rw = W.reps + t.rslot;
-  if (small) {
+  if (t.len == 2 && !kCg) {
+    const uint32_t a = mem[0], b = mem[1], r = min(a, b);
+    if (lane < 2) rw[lane] = (lane ? b : a) | (r << 16);
+  } else if (small) {
     // the least vertex of each component (a reduction per component, one after
     // the other, took 3,200 of the 7,400 cycles of a call)
     W.scr[lane] = kNone;

@@ -45,6 +45,7 @@ constexpr int kW64Levels = kW64MaxN + 2;
 constexpr int kW64Threads = 128;  // 4 warps per block, one graph per warp
 constexpr int kW64Warps = kW64Threads / 32;
 constexpr int kW64AutHead = 8;  // first ring entries kept in shared memory
+constexpr int kW64RepHead = 6;  // first levels' representatives kept in shared memory
 
 enum GraphStatus : int32_t {
   kOk = 0,
@@ -84,6 +85,7 @@ struct __align__(16) W64Smem {
   uint16_t firstcode[kW64Levels];
   uint16_t canoncode[kW64Levels];
   uint64_t lst[kW64Levels];  // cell starts of the path's node of each level
+  uint64_t sqm[kW64Levels];  // vertices of the sequence's first k entries
   alignas(16) uint16_t item[kW64MaxN];  // hash items of a refinement step
   uint8_t cs[kW64MaxN];      // vertex -> start position of its cell
   uint8_t seq[kW64MaxN];
@@ -97,6 +99,7 @@ struct __align__(16) W64Smem {
   // ring entries 0..kW64AutHead-1 and their fixed-point masks; later entries
   // live in the slot workspace
   uint8_t aut_head[kW64AutHead][kW64MaxN];
+  uint8_t rep_head[kW64RepHead][kW64MaxN];  // representatives of the first levels
   uint64_t fix_head[kW64AutHead];
 };
 
@@ -585,8 +588,7 @@ static __device__ __forceinline__ bool w64_orbits(int n, int idx, int num_aut, u
   int from = S.tc[idx].last;
   if (from == -1) from = 0;
   const uint64_t mem = S.tc[idx].members;
-  const uint64_t seqm = warp_or64((lane < seqlen ? bit64(S.seq[lane]) : 0ull) |
-                                  (lane + 32 < seqlen ? bit64(S.seq[lane + 32]) : 0ull));
+  const uint64_t seqm = S.sqm[seqlen];
   // whether stored permutation i takes part
   auto takes_part = [&](int i) {
     const uint64_t fm = i < kW64AutHead ? S.fix_head[i] : fixes[i];
@@ -603,11 +605,32 @@ static __device__ __forceinline__ bool w64_orbits(int n, int idx, int num_aut, u
     if ((sel = selected(base)) != 0) break;
   if (!sel) return true;  // no member's orbit can change
   const bool rv = S.tc[idx].reps_valid;
-  uint8_t* rp = reps + (uint64_t)idx * 64u;
   const uint32_t v0 = lane, v1 = lane + 32, size = popc64(mem);
-  auto image = [&](int i) -> const uint8_t* {
-    return i < kW64AutHead ? S.aut_head[i] : auts + (uint64_t)i * 64u;
+  // (one load or the other, not a load through either address)
+  auto image = [&](int i, uint32_t v) -> uint32_t {
+    return i < kW64AutHead ? S.aut_head[i][v] : auts[(uint64_t)i * 64u + v];
   };
+  auto rep_of = [&](uint32_t v) -> uint32_t {
+    return idx < kW64RepHead ? S.rep_head[idx][v] : reps[(uint64_t)idx * 64u + v];
+  };
+  auto set_rep = [&](uint32_t v, uint32_t r) {
+    if (idx < kW64RepHead)
+      S.rep_head[idx][v] = (uint8_t)r;
+    else
+      reps[(uint64_t)idx * 64u + v] = (uint8_t)r;
+  };
+  if (size == 2) {
+    // the permutations that take part move a member, so they swap the two
+    const uint32_t r = ctz64(mem);
+    if (lane == 0) {
+      set_rep(r, r);
+      set_rep(msb64(mem), r);
+      S.tc[idx].repmask = bit64(r);
+      S.tc[idx].reps_valid = 1;
+    }
+    __syncwarp();
+    return true;
+  }
   if (size <= 32) {
     if ((mem >> v0) & 1ull) S.map[popc64(mem & low_mask(v0))] = (uint8_t)v0;
     if ((mem >> v1) & 1ull) S.map[popc64(mem & low_mask(v1))] = (uint8_t)v1;
@@ -615,7 +638,7 @@ static __device__ __forceinline__ bool w64_orbits(int n, int idx, int num_aut, u
     const bool in = lane < size;
     const uint32_t v = in ? S.map[lane] : 0u;
     uint32_t comp = lane;  // the least lane of the member's component
-    if (in && rv) comp = popc64(mem & low_mask((uint32_t)rp[v]));
+    if (in && rv) comp = popc64(mem & low_mask(rep_of(v)));
     for (;;) {
       while (sel) {
         uint32_t j[4], c[4];
@@ -623,9 +646,9 @@ static __device__ __forceinline__ bool w64_orbits(int n, int idx, int num_aut, u
         for (int k = 0; k < 4; ++k) {
           j[k] = v;
           if (!sel) continue;
-          const uint8_t* img = image(base + __ffs((int)sel) - 1);
+          const int i = base + __ffs((int)sel) - 1;
           sel &= sel - 1;
-          if (in) j[k] = img[v];
+          if (in) j[k] = image(i, v);
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k) j[k] = in ? popc64(mem & low_mask(j[k])) : lane;
@@ -658,7 +681,7 @@ static __device__ __forceinline__ bool w64_orbits(int n, int idx, int num_aut, u
       if (!sel) break;
     }
     const uint64_t rm = warp_or64(in && comp == lane ? bit64(v) : 0ull);
-    if (in) rp[v] = S.map[comp];
+    if (in) set_rep(v, S.map[comp]);
     __syncwarp();
     if (lane == 0) {
       S.tc[idx].repmask = rm;
@@ -668,8 +691,8 @@ static __device__ __forceinline__ bool w64_orbits(int n, int idx, int num_aut, u
     return true;
   }
   const bool ok0 = v0 < (uint32_t)n, ok1 = v1 < (uint32_t)n;
-  uint32_t L0 = ok0 && ((mem >> v0) & 1ull) && rv ? (uint32_t)rp[v0] : v0;
-  uint32_t L1 = ok1 && ((mem >> v1) & 1ull) && rv ? (uint32_t)rp[v1] : v1;
+  uint32_t L0 = ok0 && ((mem >> v0) & 1ull) && rv ? rep_of(v0) : v0;
+  uint32_t L1 = ok1 && ((mem >> v1) & 1ull) && rv ? rep_of(v1) : v1;
   // The orbits are the components of the graph whose edges join every
   // vertex v to its previous orbit's label L(v) and to its image under each
   // selected automorphism; a component is labelled by its least vertex.
@@ -696,8 +719,8 @@ static __device__ __forceinline__ bool w64_orbits(int n, int idx, int num_aut, u
     return false;
   };
   // the edges v -- pi(v) of one automorphism
-  auto apply = [&](const uint8_t* img) -> bool {
-    const uint32_t u0 = ok0 ? (uint32_t)img[v0] : v0, u1 = ok1 ? (uint32_t)img[v1] : v1;
+  auto apply = [&](int i) -> bool {
+    const uint32_t u0 = ok0 ? image(i, v0) : v0, u1 = ok1 ? image(i, v1) : v1;
     for (int round = 0; round <= kW64MaxN; ++round) {  // a hook round removes a root
       const uint32_t x0 = __shfl_sync(GCL_FULL, fp, (int)(u0 & 31u));
       const uint32_t x1 = __shfl_sync(GCL_FULL, fp, (int)(u1 & 31u));
@@ -720,7 +743,7 @@ static __device__ __forceinline__ bool w64_orbits(int n, int idx, int num_aut, u
   if (!compress()) return false;
   for (;;) {
     for (; sel; sel &= sel - 1)
-      if (!apply(image(base + __ffs((int)sel) - 1))) return false;
+      if (!apply(base + __ffs((int)sel) - 1)) return false;
     for (base += 32; base < limit; base += 32)
       if ((sel = selected(base)) != 0) break;
     if (!sel) break;
@@ -729,11 +752,11 @@ static __device__ __forceinline__ bool w64_orbits(int n, int idx, int num_aut, u
   L1 = (fp >> 8) & 0xffu;
   bool r0 = false, r1 = false;
   if (ok0 && ((mem >> v0) & 1ull)) {
-    rp[v0] = (uint8_t)L0;
+    set_rep(v0, L0);
     r0 = L0 == v0;
   }
   if (ok1 && ((mem >> v1) & 1ull)) {
-    rp[v1] = (uint8_t)L1;
+    set_rep(v1, L1);
     r1 = L1 == v1;
   }
   const uint64_t rm = ballot2(r0, r1);
@@ -897,13 +920,19 @@ static __device__ __noinline__ W64Result w64_search_tree(const BatchArgs& A, int
   int64_t nodes = 1;
   int32_t status = kOk;
 
-  if (lane == 0) S.lst[1] = starts;
+  if (lane == 0) {
+    S.lst[1] = starts;
+    S.sqm[0] = 0;
+  }
   __syncwarp();
-  // the next refinement to run on the first path, given by its initially
-  // active cells
+  // the next refinement to run, given by its initially active cells: the one
+  // place of this function where a node is refined, so that the loop stays
+  // small in the instruction cache
   uint64_t pending = 0;
   uint64_t iter = 0;
   while (true) {
+    int bt = -1;  // backtrack target level
+    bool classify = false;
     if (pending) {
       const W64Refined r = w64_refine(n, starts, pending);
       pending = 0;
@@ -914,129 +943,117 @@ static __device__ __noinline__ W64Result w64_search_tree(const BatchArgs& A, int
       starts = r.starts;
       code = r.code;
       ++level;
-      // the first path records its codes (sequential.cpp:254, 630)
-      __syncwarp();
       if (lane == 0) {
-        S.firstcode[level - 1] = (uint16_t)code;
         S.lst[level] = starts;
+        // the first path records its codes (sequential.cpp:254, 630)
+        if (!first_found) S.firstcode[level - 1] = (uint16_t)code;
       }
       __syncwarp();
-      continue;
-    }
-    if (level == 0) break;
-    if ((++iter & 63) == 0 && deadline &&
-        __shfl_sync(GCL_FULL, lane == 0 ? global_ns() : 0ull, 0) > deadline) {
-      status = kTimeout;
-      break;
-    }
-    int bt = -1;       // backtrack target level
-    int descend = -1;  // index of the target cell to branch from
-    bool classify = false;
-    const bool disc = starts == full;
-    if (!first_found) {
-      // first_path_node (sequential.cpp:216-257)
-      if (disc) {
-        // first_terminal (sequential.cpp:259-303)
-        const Rows2 R = w64_leaf_rows(n);
-        w64_store_leaf(n, R, S.first_cert, S.fpos);
-        w64_store_leaf(n, R, S.best_cert, S.bpos);
-        if (lane < seqlen) S.first_seq[lane] = S.best_seq[lane] = S.seq[lane];
-        if (lane + 32 < seqlen) S.first_seq[lane + 32] = S.best_seq[lane + 32] = S.seq[lane + 32];
-        if (lane < level) S.canoncode[lane] = S.firstcode[lane];
-        if (lane + 32 < level) S.canoncode[lane + 32] = S.firstcode[lane + 32];
-        __syncwarp();
-        if (lane == 0) {
-          S.firstcode[level] = (uint16_t)kSentinel;
-          S.canoncode[level] = (uint16_t)kSentinel;
-        }
-        __syncwarp();
-        eqlevfirst = level;
-        first_seqlen = best_seqlen = seqlen;
-        first_found = true;
-        canon_level = eqlevcanon = (int)level;
-        comp_canon = 0;
-        bt = (int)level - 1;
-      } else {
-        if (tcl >= kW64Levels) {
-          status = kInternal;
-          break;
-        }
-        w64_select_tc(n, starts, tcl);
-        ++tcl;
-        descend = tcl - 1;
-      }
-    } else {
-      // other_path_node (sequential.cpp:304-392)
+      if (!first_found) continue;
       classify = true;
-      if (!disc && (eqlevfirst == level || comp_canon >= 0)) {
-        if (tcl < (int)level) {
+    } else {
+      if (level == 0) break;
+      if ((++iter & 63) == 0 && deadline &&
+          __shfl_sync(GCL_FULL, lane == 0 ? global_ns() : 0ull, 0) > deadline) {
+        status = kTimeout;
+        break;
+      }
+      int descend = -1;  // index of the target cell to branch from
+      const bool disc = starts == full;
+      if (!first_found) {
+        // first_path_node (sequential.cpp:216-257)
+        if (disc) {
+          // first_terminal (sequential.cpp:259-303)
+          const Rows2 R = w64_leaf_rows(n);
+          w64_store_leaf(n, R, S.first_cert, S.fpos);
+          w64_store_leaf(n, R, S.best_cert, S.bpos);
+          if (lane < seqlen) S.first_seq[lane] = S.best_seq[lane] = S.seq[lane];
+          if (lane + 32 < seqlen) S.first_seq[lane + 32] = S.best_seq[lane + 32] = S.seq[lane + 32];
+          if (lane < level) S.canoncode[lane] = S.firstcode[lane];
+          if (lane + 32 < level) S.canoncode[lane + 32] = S.firstcode[lane + 32];
+          __syncwarp();
+          if (lane == 0) {
+            S.firstcode[level] = (uint16_t)kSentinel;
+            S.canoncode[level] = (uint16_t)kSentinel;
+          }
+          __syncwarp();
+          eqlevfirst = level;
+          first_seqlen = best_seqlen = seqlen;
+          first_found = true;
+          canon_level = eqlevcanon = (int)level;
+          comp_canon = 0;
+          bt = (int)level - 1;
+        } else {
           if (tcl >= kW64Levels) {
             status = kInternal;
             break;
           }
           w64_select_tc(n, starts, tcl);
           ++tcl;
+          descend = tcl - 1;
         }
-        const int idx = (int)level - 1;
-        if (S.tc[idx].counter >= (uint32_t)n) {
-          bt = (int)level - 1;
-          classify = false;
-        } else {
-          if (num_aut > 0 && num_aut > S.tc[idx].last) {
-            if (!w64_orbits(n, idx, num_aut, A.max_aut, seqlen, reps, auts,
-                            reinterpret_cast<const uint64_t*>(auts + (uint64_t)A.aut_cap * 64u))) {
+      } else {
+        // other_path_node (sequential.cpp:304-392)
+        classify = true;
+        if (!disc && (eqlevfirst == level || comp_canon >= 0)) {
+          if (tcl < (int)level) {
+            if (tcl >= kW64Levels) {
               status = kInternal;
               break;
             }
-            __syncwarp();
-            if (lane == 0) S.tc[idx].last = num_aut;
-            __syncwarp();
+            w64_select_tc(n, starts, tcl);
+            ++tcl;
           }
-          descend = idx;
+          const int idx = (int)level - 1;
+          if (S.tc[idx].counter >= (uint32_t)n) {
+            bt = (int)level - 1;
+            classify = false;
+          } else {
+            if (num_aut > 0 && num_aut > S.tc[idx].last) {
+              if (!w64_orbits(n, idx, num_aut, A.max_aut, seqlen, reps, auts,
+                              reinterpret_cast<const uint64_t*>(auts + (uint64_t)A.aut_cap * 64u))) {
+                status = kInternal;
+                break;
+              }
+              __syncwarp();
+              if (lane == 0) S.tc[idx].last = num_aut;
+              __syncwarp();
+            }
+            descend = idx;
+          }
         }
       }
-    }
-    if (descend >= 0) {
-      // next representative: smallest v >= counter with elems[v] == v
-      const uint64_t r = S.tc[descend].repmask & ge_mask(S.tc[descend].counter);
-      if (!r) {
-        // the counter runs past the last vertex (sequential.cpp:359-365)
-        __syncwarp();
-        if (lane == 0) S.tc[descend].counter = (uint16_t)n;
-        __syncwarp();
-        bt = (int)level - 1;
-        classify = false;
-      } else {
-        const uint32_t v = ctz64(r), t = S.tc[descend].first;
-        __syncwarp();
-        if (lane == 0) {
-          S.tc[descend].counter = (uint16_t)(v + 1);
-          S.seq[seqlen] = (uint8_t)v;
-        }
-        __syncwarp();
-        ++seqlen;
-        ++nodes;
-        if (w64_individualize(n, v, t)) {
-          starts |= bit64(t + 1);
-          if (!first_found) {
-            pending = bit64(t);  // refine and record firstcode
+      if (descend >= 0) {
+        // next representative: smallest v >= counter with elems[v] == v
+        const uint64_t r = S.tc[descend].repmask & ge_mask(S.tc[descend].counter);
+        if (!r) {
+          // the counter runs past the last vertex (sequential.cpp:359-365)
+          __syncwarp();
+          if (lane == 0) S.tc[descend].counter = (uint16_t)n;
+          __syncwarp();
+          bt = (int)level - 1;
+          classify = false;
+        } else {
+          const uint32_t v = ctz64(r), t = S.tc[descend].first;
+          __syncwarp();
+          if (lane == 0) {
+            S.tc[descend].counter = (uint16_t)(v + 1);
+            S.seq[seqlen] = (uint8_t)v;
+            S.sqm[seqlen + 1] = S.sqm[seqlen] | bit64(v);
+          }
+          __syncwarp();
+          ++seqlen;
+          ++nodes;
+          if (w64_individualize(n, v, t)) {
+            starts |= bit64(t + 1);
+            pending = bit64(t);
+            continue;
+          } else if (!first_found) {
+            __syncwarp();
+            if (lane == 0) S.firstcode[level - 1] = (uint16_t)code;
+            __syncwarp();
             continue;
           }
-          const W64Refined rr = w64_refine(n, starts, bit64(t));
-          if (!rr.ok) {
-            status = kInternal;
-            break;
-          }
-          starts = rr.starts;
-          code = rr.code;
-          ++level;
-          if (lane == 0) S.lst[level] = starts;
-          __syncwarp();
-        } else if (!first_found) {
-          __syncwarp();
-          if (lane == 0) S.firstcode[level - 1] = (uint16_t)code;
-          __syncwarp();
-          continue;
         }
       }
     }
