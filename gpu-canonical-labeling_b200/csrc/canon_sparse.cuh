@@ -317,35 +317,34 @@ struct SpRef {
   __device__ __forceinline__ bool active(uint32_t c) const {
     return (act[c >> 5] >> (c & 31u)) & 1u;
   }
-  // the end of the cell of position p.  Cells are short once a refinement is
-  // under way: the words beside p's are tried before the summary.
+  // the end of the cell of position p, and its start and length: in p's word of
+  // 64 starts, else through the summary
   __device__ __forceinline__ uint32_t end_of(uint32_t p, uint32_t n) const {
-    uint32_t w = p >> 5, x = st[w] & (0xfffffffeu << (p & 31u));
-    for (int far = 0; !x; ++far) {
-      if (far == 4) return bm_next(stb, sts, (w + 1) * 32, n, (n + 63) / 64 + 1, ((n + 63) / 64 + 64) / 64 + 1);
-      x = st[++w];
-    }
-    return w * 32 + (uint32_t)__ffs((int)x) - 1u;
+    const uint32_t w = p >> 6;
+    const uint64_t x = stb[w] & (~1ull << (p & 63u));
+    if (x) return w * 64 + ctz64(x);
+    const uint64_t y = sts[w >> 6] & (~1ull << (w & 63u));
+    if (!y) return bm_next(stb, sts, (w + 1) * 64, n, (n + 63) / 64 + 1, ((n + 63) / 64 + 64) / 64 + 1);
+    const uint32_t v = (w & ~63u) + ctz64(y);
+    return v * 64 + ctz64(stb[v]);
   }
-  // the start c and length of the cell of position p
   __device__ __forceinline__ void cell_of(uint32_t p, uint32_t n, uint32_t* c, uint32_t* len) const {
-    const uint32_t w = p >> 5, x = st[w], sh = p & 31u;
-    const uint32_t lo = x & (0xffffffffu >> (31u - sh)), hi = x & (0xfffffffeu << sh);
-    uint32_t a = 0, e = 0;
-    if (lo) {
-      a = w * 32 + 31u - (uint32_t)__clz((int)lo);
+    const uint32_t w = p >> 6;
+    const uint64_t x = stb[w] & (~0ull >> (63u - (p & 63u)));
+    uint32_t a;
+    if (x) {
+      a = w * 64 + msb64(x);
     } else {
-      uint32_t v = w, y = 0;
-      for (int far = 0; far < 4 && !y; ++far) y = st[--v];  // position 0 is a start
-      a = y ? v * 32 + 31u - (uint32_t)__clz((int)y) : bm_prev(stb, sts, v * 32 - 1);
-    }
-    if (hi) {
-      e = w * 32 + (uint32_t)__ffs((int)hi) - 1u;
-    } else {
-      e = end_of(w * 32 + 31u, n);
+      const uint64_t y = sts[w >> 6] & (bit64(w & 63u) - 1);
+      if (y) {
+        const uint32_t v = (w & ~63u) + msb64(y);
+        a = v * 64 + msb64(stb[v]);
+      } else {
+        a = bm_prev(stb, sts, w * 64 - 1);  // position 0 is a start
+      }
     }
     *c = a;
-    *len = e - a;
+    *len = end_of(p, n) - a;
   }
 };
 
@@ -435,9 +434,10 @@ __device__ __noinline__ uint32_t sp_fold(uint32_t lc, bool listed) {
       // the items in position order, 256 at a time (one round unless a large
       // count turned the bit-wise fold away)
       uint32_t at = K;
-      for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t used = (nwd - base + kW - 1) / kW;  // lanes that hold words
+      for (uint32_t o = 1; o < 32 && o < used; o <<= 1) {
         const uint32_t y = __shfl_up_sync(GCL_FULL, at, o);
-        if (lane >= (uint32_t)o) at += y;
+        if (lane >= o) at += y;
       }
       at -= K;
       for (uint32_t done = 0; done < total; done += kList) {
@@ -679,16 +679,78 @@ __device__ __noinline__ SpStep sp_refine_general(uint32_t s, uint32_t e, uint32_
           __syncwarp();
           continue;
         }
+        // a large cell: its touched positions, eight counts per lane at a time
+        if (lane == 0) W.scr[0] = 0;
+        __syncwarp();
         uint32_t mn = 0xffffffffu, mx = 0;
-        for (uint32_t i = lane; i < L; i += 32) {
-          const uint32_t x = R.cnt[c + i];
-          mn = min(mn, x);
-          mx = max(mx, x);
+        for (uint32_t q0 = (c & ~7u) + lane * 8; q0 < ce; q0 += 256) {
+          const uint4 x4 = *(const uint4*)(R.cnt + q0);
+          if (!(x4.x | x4.y | x4.z | x4.w)) continue;
+          const uint32_t xs[4] = {x4.x, x4.y, x4.z, x4.w};
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const uint32_t a = (xs[j / 2] >> (j % 2 * 16)) & 0xffffu, q = q0 + j;
+            if (!a || q < c || q >= ce) continue;
+            mn = min(mn, a);
+            mx = max(mx, a);
+            const uint32_t i = atomicAdd(&W.scr[0], 1u);
+            if (i < 256) W.list[i] = (uint16_t)q;
+          }
         }
+        __syncwarp();
+        const uint32_t touched = W.scr[0];
         mn = __reduce_min_sync(GCL_FULL, mn);
         mx = __reduce_max_sync(GCL_FULL, mx);
+        if (touched < L) mn = 0;
         if (mn == mx) {
           if (mn && !single && lane == 0) or_bit32(R.itm, c);
+          __syncwarp();
+          continue;
+        }
+        if (touched <= 32 && touched < L && !single) {
+          // few touched vertices: they go to the cell's last places, ranked by
+          // count, and swap with the untouched ones found there -- the cost of
+          // the touched ones, not of the cell (a counting sort of the whole
+          // cell took some 100 cycles per 32 vertices)
+          const bool on = lane < touched;
+          const uint32_t p = on ? W.list[lane] : 0u, u = on ? R.elem[p] : 0u;
+          const uint32_t a = on ? R.cnt[p] : 0u;
+          const uint32_t all = touched == 32 ? 0xffffffffu : (1u << touched) - 1u;
+          uint32_t peers = all, less = 0;
+          for (int bit = 31 - __clz((int)mx); bit >= 0; --bit) {
+            const bool one = (a >> bit) & 1u;
+            const uint32_t m1 = __ballot_sync(GCL_FULL, on && one);
+            if (one) {
+              less += (uint32_t)__popc(peers & ~m1);
+              peers &= m1;
+            } else {
+              peers &= ~m1;
+            }
+          }
+          const uint32_t eq = (uint32_t)__popc(peers & lt), size = (uint32_t)__popc(peers);
+          const uint32_t R0 = ce - touched, f = R0 + less;
+          const bool in = on && p >= R0, mv = on && p < R0, frag = on && eq == 0;
+          const uint32_t inner = __reduce_or_sync(GCL_FULL, in ? 1u << (p - R0) : 0u);
+          const uint32_t outs = __ballot_sync(GCL_FULL, mv);
+          const uint32_t h = mv ? R0 + nth_bit(~inner & all, (uint32_t)__popc(outs & lt)) : 0u;
+          const uint32_t x = mv ? R.elem[h] : 0u;
+          const uint32_t rank = frag ? (size << 6) | (63u - less) : 0u;
+          const uint32_t best = __reduce_max_sync(GCL_FULL, rank);
+          const bool rest = L - touched >= (best >> 6);  // the untouched fragment is the largest
+          __syncwarp();
+          if (mv) {
+            R.elem[p] = (uint16_t)x;
+            R.pos[x] = (uint16_t)p;
+            R.cnt[p] = 0;
+          }
+          __syncwarp();
+          if (on) {
+            R.elem[f + eq] = (uint16_t)u;
+            R.pos[u] = (uint16_t)(f + eq);
+            R.cnt[f + eq] = (uint16_t)a;
+          }
+          if (lane == 0 && !was && !rest) or_bit32(R.act, c);
+          fragment(frag, c, f, size, a, was || rest || rank != best);
           __syncwarp();
           continue;
         }
@@ -735,6 +797,7 @@ __device__ __noinline__ SpStep sp_refine_general(uint32_t s, uint32_t e, uint32_
           W.tmp[atomicAdd(&pre[(a - mn) ^ flip], 1u)] = (a << 16) | R.elem[c + i];
         }
         __syncwarp();
+#pragma unroll 4
         for (uint32_t i = lane; i < L; i += 32) {
           const uint32_t x = W.tmp[i], v = x & 0xffffu;
           R.elem[c + i] = (uint16_t)v;
@@ -864,13 +927,17 @@ __device__ __noinline__ int sp_refine_t() {
         uint32_t h = c, x = 0;
         bool mv = false;
         if (__any_sync(GCL_FULL, spl && k > 1)) {
+          // the places taken, collected at the cell's first lane
           const bool in = p < c + k;
-          uint32_t inner = 0;
-          if (spl) inner = __reduce_or_sync(grp, in ? 1u << (p - c) : 0u);
+          const uint32_t first = (uint32_t)__ffs((int)grp) - 1;
+          W.scr[lane] = 0;
+          __syncwarp();
+          if (spl && in) atomicOr(&W.scr[first], 1u << (p - c));
           const uint32_t outs = __ballot_sync(GCL_FULL, spl && !in) & grp;
+          __syncwarp();
           mv = spl && !in;
           if (mv)
-            h = c + nth_bit(~inner & (k >= 32 ? 0xffffffffu : (1u << k) - 1u),
+            h = c + nth_bit(~W.scr[first] & (k >= 32 ? 0xffffffffu : (1u << k) - 1u),
                             (uint32_t)__popc(outs & lt));
         } else {
           mv = spl && p != c;
@@ -990,15 +1057,22 @@ __device__ __noinline__ int sp_refine_t() {
           const bool in = p >= R0;
           const bool frag = split && eq == 0;
           const uint32_t rank = frag ? (size << 6) | (63u - less) : 0u;
-          uint32_t inner = 0, best = 0;
-          if (split) {
-            inner = __reduce_or_sync(gc, in ? 1u << (p - R0) : 0u);
-            best = __reduce_max_sync(gc, rank);
-          }
+          // per cell, at its first lane: the places taken in [R0, c + L) and the
+          // first largest fragment (a reduction per cell, one after the other,
+          // took 1,000 cycles of a step that splits five cells)
+          const uint32_t first = (uint32_t)__ffs((int)gc) - 1;
+          uint32_t* const top_of = (uint32_t*)W.list;
+          W.scr[lane] = 0;
+          top_of[lane] = 0;
+          __syncwarp();
+          if (split && in) atomicOr(&W.scr[first], 1u << (p - R0));
+          if (frag) atomicMax(&top_of[first], rank);
           const uint32_t outs = __ballot_sync(GCL_FULL, split && !in) & gc;
+          __syncwarp();
+          const uint32_t best = top_of[first];
           const bool mv = split && !in;
           if (mv) {
-            h = R0 + nth_bit(~inner & (k >= 32 ? 0xffffffffu : (1u << k) - 1u),
+            h = R0 + nth_bit(~W.scr[first] & (k >= 32 ? 0xffffffffu : (1u << k) - 1u),
                              (uint32_t)__popc(outs & lt));
             x = R.elem[h];
           }
@@ -1252,8 +1326,15 @@ __device__ __forceinline__ int sp_cmp_leaf(const uint32_t* cur, const uint32_t* 
 
 template <typename T>
 __device__ __forceinline__ void sp_copy_u32(uint32_t* dst, const T* src, uint32_t k) {
-  const uint32_t lane = lane_id();
-  for (uint32_t i = lane; i < k; i += 32) dst[i] = src[i];
+  // eight loads in flight at a time
+  for (uint32_t i0 = lane_id(); i0 < k; i0 += 256) {
+    uint32_t x[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = i0 + 32 * j < k ? src[i0 + 32 * j] : 0u;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (i0 + 32 * j < k) dst[i0 + 32 * j] = x[j];
+  }
   __syncwarp();
 }
 

@@ -541,8 +541,22 @@ __device__ __noinline__ uint32_t wide_orbit_min_own(const WidePtrs& P, uint32_t 
   return r;
 }
 
+// f(i, src[i]) for i < k, a warp's eight loads in flight at a time (one by one,
+// each waits some 300 cycles for L2: copying the best leaf of a graph of 160,000
+// CSR entries took 2 ms).
+template <typename F>
+__device__ __forceinline__ void wide_each(const uint32_t* src, uint64_t k, F f) {
+  for (uint64_t i0 = lane_id(); i0 < k; i0 += 256) {
+    uint32_t x[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = i0 + 32 * j < k ? __ldcg(src + i0 + 32 * j) : 0u;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (i0 + 32 * j < k) f(i0 + 32 * j, x[j]);
+  }
+}
+
 // Append aut[label[j]] = elem[j] to the store with its fixed-prefix length.
-template <bool kCgLabel>
 __device__ __noinline__ void wide_store_aut(const WidePtrs& P, const uint32_t* label, uint32_t cap,
                                             uint32_t stride, uint32_t D) {
   SpWarp& W = sp_w();
@@ -552,7 +566,8 @@ __device__ __noinline__ void wide_store_aut(const WidePtrs& P, const uint32_t* l
   slot = __shfl_sync(GCL_FULL, slot, 0);
   if (slot >= cap) return;  // store full: fewer prunes, same result
   uint16_t* pm = P.auts + (uint64_t)slot * stride;
-  for (uint32_t j = lane; j < W.n; j += 32) pm[ldx<kCgLabel>(label + j)] = (uint16_t)W.elem[j];
+  const uint16_t* const elem = W.elem;
+  wide_each(label, W.n, [&](uint64_t j, uint32_t v) { pm[v] = elem[j]; });
   __syncwarp();
   // leading first-path vertices it fixes
   const uint32_t np = D - 1;
@@ -609,9 +624,11 @@ __device__ __noinline__ bool wide_adopt(const WidePtrs& P, int64_t m, WideBest* 
       continue;
     }
     for (uint32_t i = lane; i <= lvl; i += 32) W.ccode[i] = __ldcg(P.bcode + i);
-    for (uint32_t i = lane; i < W.n; i += 32) W.blabel[i] = __ldcg(P.blabel + i);
     for (uint32_t i = lane; i < sl; i += 32) W.bseq[i] = __ldcg(P.bseq + i);
-    for (int64_t i = lane; i < m; i += 32) W.bcert[i] = __ldcg(P.bcert + i);
+    uint32_t* const label = W.blabel;
+    wide_each(P.blabel, W.n, [&](uint64_t i, uint32_t x) { label[i] = x; });
+    uint32_t* const cert = W.bcert;
+    wide_each(P.bcert, (uint64_t)m, [&](uint64_t i, uint32_t x) { cert[i] = x; });
     __threadfence();
     __syncwarp();
     uint32_t v2 = 0;
@@ -929,12 +946,14 @@ __device__ __noinline__ void wide_load_node(const WidePtrs& P, uint32_t L) {
   SpWarp& W = sp_w();
   const uint32_t lane = lane_id();
   const uint32_t n = W.n;
-  for (uint32_t i = lane; i < n; i += 32) {
-    const uint32_t x = P.lelem[i];
-    W.elem[i] = x;
-    W.pos[x] = i;
-  }
+  uint16_t* const elem = W.elem;
+  uint16_t* const pos = W.pos;
+  wide_each(P.lelem, n, [&](uint64_t i, uint32_t x) {
+    elem[i] = (uint16_t)x;
+    pos[x] = (uint16_t)i;
+  });
   uint32_t cells = 0;
+#pragma unroll 4
   for (uint32_t w = 0; w < W.nw; ++w) {
     const uint32_t p0 = w * 64 + lane, p1 = p0 + 32;
     uint64_t b = P.lstb[w] & ballot2(p0 < n && P.linlev[p0] <= L, p1 < n && P.linlev[p1] <= L);
@@ -1313,12 +1332,12 @@ __global__ void __launch_bounds__(kSpThreads) wide_items_kernel(WideArgs A) {
         }
         if (dec == 1) {
           cnt.add(kCntAutsFirst, 1);
-          wide_store_aut<false>(P, W.flabel, cap, A.WL.stride, D);
+          wide_store_aut(P, W.flabel, cap, A.WL.stride, D);
           const int gg = sp_gca(W.fseq, D - 1, seqlen);
           bt = gg >= 0 ? gg : (int)Lv - 1;
         } else if (dec == 2) {
           cnt.add(kCntAutsBest, 1);
-          wide_store_aut<false>(P, W.blabel, cap, A.WL.stride, D);
+          wide_store_aut(P, W.blabel, cap, A.WL.stride, D);
           const int gg = best_local ? sp_gca(W.bseq, best.best_seqlen, seqlen) : -1;
           bt = gg >= 0 ? gg : (int)Lv - 1;
         } else if (dec == 3) {
@@ -1353,7 +1372,7 @@ __global__ void __launch_bounds__(kSpThreads) wide_items_kernel(WideArgs A) {
             // equivalent to, or worse than, the adopted best
             if (res == 2) {
               cnt.add(kCntAutsBest, 1);
-              wide_store_aut<false>(P, W.blabel, cap, A.WL.stride, D);
+              wide_store_aut(P, W.blabel, cap, A.WL.stride, D);
             }
             best_local = false;
             recompare = true;

@@ -69,3 +69,12 @@ def test_stars_and_large_cells(pkg, G, oracle_mod, leaves):
           bipartite(G, 100, 2 * leaves, 0.9, rng), G.torus(9, 11)]
     check(pkg, oracle_mod, gs)
     check(pkg, oracle_mod, gs, GCL_OPT_SMEM_STAGE=0)
+
+
+@pytest.mark.parametrize("n", [130, 300])
+def test_few_touched_vertices_of_large_cells(pkg, G, oracle_mod, n):
+    rng = np.random.default_rng(n)
+    gs = [G.random_regular(n, 3, rng), G.random_regular(n, 5, rng),
+          G.disjoint_union(G.random_regular(n // 2 - (n // 2) % 2, 4, rng), 2)]
+    check(pkg, oracle_mod, gs)
+    check(pkg, oracle_mod, gs, GCL_OPT_SMEM_STAGE=0)
