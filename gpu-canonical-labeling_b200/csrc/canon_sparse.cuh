@@ -346,6 +346,24 @@ struct SpRef {
     *c = a;
     *len = end_of(p, n) - a;
   }
+  // the same for n <= 1,024 without a branch: `some` has a bit per word of 32
+  // positions that holds a start (lanes of one step lie in cells of all sizes,
+  // and the two-way choices above run one after the other)
+  __device__ __forceinline__ void cell_of_1k(uint32_t p, uint32_t n, uint32_t some, uint32_t* c,
+                                             uint32_t* len) const {
+    const uint32_t w = p >> 5, sh = p & 31u, x = st[w];
+    const uint32_t lo = x & (0xffffffffu >> (31u - sh)), hi = x & (0xfffffffeu << sh);
+    const uint32_t below = some & ((1u << w) - 1u), above = some & (0xfffffffeu << w);
+    // words that hold the cell's start (word 0 holds one) and the next one; with
+    // none above, the cell ends at n and p's own word is read in its place
+    const uint32_t wl = lo || !below ? w : 31u - (uint32_t)__clz((int)below);
+    const uint32_t wh = hi || !above ? w : (uint32_t)__ffs((int)above) - 1u;
+    const uint32_t y = lo ? lo : st[wl], z = hi ? hi : st[wh];
+    const uint32_t a = wl * 32 + 31u - (uint32_t)__clz((int)y);
+    const uint32_t e = hi || above ? min(n, wh * 32 + (uint32_t)__ffs((int)z) - 1u) : n;
+    *c = a;
+    *len = e - a;
+  }
 };
 
 __device__ __forceinline__ void or_bit32(uint32_t* B, uint32_t p) {
@@ -917,7 +935,12 @@ __device__ __noinline__ int sp_refine_t() {
         }
         __syncwarp();
         if (!__any_sync(GCL_FULL, on)) continue;
-        if (on) R.cell_of(p, n, &c, &L);
+        if (nwd <= 32) {
+          const uint32_t some = __ballot_sync(GCL_FULL, lane < nwd && R.st[lane] != 0);
+          if (on) R.cell_of_1k(p, n, some, &c, &L);
+        } else if (on) {
+          R.cell_of(p, n, &c, &L);
+        }
         const uint32_t grp = __match_any_sync(GCL_FULL, c);
         const uint32_t k = (uint32_t)__popc(grp);
         const bool spl = on && k < L;
@@ -970,18 +993,23 @@ __device__ __noinline__ int sp_refine_t() {
         nact += made;
         // hash (cell.first + neighbors_size - 1) in position order; the hint
         // is the last split cell's that sets one
-        for (uint32_t i = 0; i < made; ++i) {
-          uint32_t x;
-          if (made == 1) {
-            x = __shfl_sync(GCL_FULL, key, __ffs((int)leaders) - 1);
-          } else {
-            x = __reduce_min_sync(GCL_FULL, key);
-            if (key == x) key = kNone;
-          }
+        auto fold = [&](uint32_t x) {
           const uint32_t cc = x >> 8, pp = cc + ((x >> 2) & 63u);
           lc = (lc ^ C) + (pp - 1);
           if (x & 2u) hint = pp;
           if (x & 1u) hint = cc;
+        };
+        if (made <= 2) {  // one or two cells: no reduction
+          const uint32_t x = __shfl_sync(GCL_FULL, key, __ffs((int)leaders) - 1);
+          const uint32_t y = __shfl_sync(GCL_FULL, key, 31 - __clz((int)leaders));
+          fold(min(x, y));
+          if (made == 2) fold(max(x, y));
+        } else {
+          for (uint32_t i = 0; i < made; ++i) {
+            const uint32_t x = __reduce_min_sync(GCL_FULL, key);
+            if (key == x) key = kNone;
+            fold(x);
+          }
         }
         __syncwarp();
         continue;
@@ -1028,7 +1056,12 @@ __device__ __noinline__ int sp_refine_t() {
         const uint32_t gu = __match_any_sync(GCL_FULL, u);
         const uint32_t cnt = (uint32_t)__popc(gu);
         const bool lead = u != kNone && (gu & lt) == 0;
-        if (lead) R.cell_of(p, n, &c, &L);
+        if (nwd <= 32) {
+          const uint32_t some = __ballot_sync(GCL_FULL, lane < nwd && R.st[lane] != 0);
+          if (lead) R.cell_of_1k(p, n, some, &c, &L);
+        } else if (lead) {
+          R.cell_of(p, n, &c, &L);
+        }
         const uint32_t gc = __match_any_sync(GCL_FULL, c);
         const uint32_t k = (uint32_t)__popc(gc);  // touched vertices of the cell
         // rank by count within the cell: a radix pass over ballots
