@@ -144,6 +144,21 @@ __device__ __forceinline__ uint64_t ballot2(bool a, bool b) {
 }
 __device__ __forceinline__ uint64_t bit64(uint32_t p) { return 1ull << p; }
 
+// The lane's two bits of a 64-bit mask, and whether a mask has none below them:
+// 32-bit shifts, where a 64-bit one by a lane takes several instructions.
+__device__ __forceinline__ bool lane_bit0(uint64_t x) {
+  return ((uint32_t)x >> (threadIdx.x & 31u)) & 1u;
+}
+__device__ __forceinline__ bool lane_bit1(uint64_t x) {
+  return ((uint32_t)(x >> 32) >> (threadIdx.x & 31u)) & 1u;
+}
+__device__ __forceinline__ bool none_below0(uint64_t x) {
+  return ((uint32_t)x & ((1u << (threadIdx.x & 31u)) - 1u)) == 0;
+}
+__device__ __forceinline__ bool none_below1(uint64_t x) {
+  return ((uint32_t)x | ((uint32_t)(x >> 32) & ((1u << (threadIdx.x & 31u)) - 1u))) == 0;
+}
+
 // ---------------------------------------------------------------------------
 // Partition_s_refinement (partition_refinement.cpp:150-485).
 // `active` holds the start positions of the initially active cells.  Returns
@@ -195,8 +210,8 @@ static __device__ __forceinline__ W64Refined w64_refine(int n, uint64_t starts, 
       // singleton cells can be in such a cell, so most steps end here.
       const uint64_t N = S.adj[S.pv[s]];
       if (!(N & ~sing)) continue;
-      const bool sp0 = ((starts >> v0) & 1ull) && (cmr0 & N) && (cmr0 & ~N);
-      const bool sp1 = ((starts >> v1) & 1ull) && (cmr1 & N) && (cmr1 & ~N);
+      const bool sp0 = lane_bit0(starts) && (cmr0 & N) && (cmr0 & ~N);
+      const bool sp1 = lane_bit1(starts) && (cmr1 & N) && (cmr1 & ~N);
       uint64_t t = ballot2(sp0, sp1);
       if (!t) continue;
       // the split cells in position order: the neighbours keep the start c,
@@ -218,8 +233,8 @@ static __device__ __forceinline__ W64Refined w64_refine(int n, uint64_t starts, 
         fresh |= bit64(p);
         if (nb == 1) sing |= CN;
         if (nn == 1) sing |= CR;
-        if ((CR >> v0) & 1ull) csr0 = p;
-        if ((CR >> v1) & 1ull) csr1 = p;
+        if (lane_bit0(CR)) csr0 = p;
+        if (lane_bit1(CR)) csr1 = p;
         if (v0 == c) cmr0 = CN;
         if (v1 == c) cmr1 = CN;
         if (v0 == p) cmr0 = CR;
@@ -268,10 +283,10 @@ static __device__ __forceinline__ W64Refined w64_refine(int n, uint64_t starts, 
       // cell (common count) and every new fragment start (:253-373), each
       // written by the fragment's least vertex
       const uint64_t T = (starts & ~ends) | NS;
-      if (ok0 && !(cm0 & low_mask(v0)) && ((T >> cs0) & 1ull))
-        S.item[popc64(T & low_mask(cs0))] = (uint16_t)(k0 + cs0);
-      if (ok1 && !(cm1 & low_mask(v1)) && ((T >> cs1) & 1ull))
-        S.item[popc64(T & low_mask(cs1))] = (uint16_t)(k1 + cs1);
+      if (ok0 && none_below0(cm0) && ((T >> cs0) & 1ull))
+        S.item[popc64(T & (bit64(cs0) - 1))] = (uint16_t)(k0 + cs0);
+      if (ok1 && none_below1(cm1) && ((T >> cs1) & 1ull))
+        S.item[popc64(T & (bit64(cs1) - 1))] = (uint16_t)(k1 + cs1);
       __syncwarp();  // ... and every lane has read the old cell masks
       {
         // bits above 14 never come down: two items per word, no masking
@@ -362,8 +377,8 @@ static __device__ __forceinline__ bool w64_individualize(int n, uint32_t v, uint
   if (popc64(mem) <= 1) return false;
   const uint32_t v0 = lane, v1 = lane + 32;
   __syncwarp();
-  if (v0 < (uint32_t)n && ((mem >> v0) & 1ull) && v0 != v) S.cs[v0] = (uint8_t)(t + 1);
-  if (v1 < (uint32_t)n && ((mem >> v1) & 1ull) && v1 != v) S.cs[v1] = (uint8_t)(t + 1);
+  if (lane_bit0(mem) && v0 != v) S.cs[v0] = (uint8_t)(t + 1);
+  if (lane_bit1(mem) && v1 != v) S.cs[v1] = (uint8_t)(t + 1);
   if (lane == 0) {
     const uint64_t rest = mem & ~bit64(v);
     S.cmask[t] = bit64(v);
@@ -405,12 +420,12 @@ static __device__ __forceinline__ uint64_t w64_backtrack(int n, uint64_t starts,
   const uint64_t ones = to & ((to >> 1) | bit64((uint32_t)n - 1));
   bool a0 = false, a1 = false;
   if (q0 < (uint32_t)n) {
-    const uint32_t c = msb64(to & low_mask((uint32_t)S.cs[q0] + 1));
+    const uint32_t c = msb64(to & (~0ull >> (63u - S.cs[q0])));
     S.cs[q0] = (uint8_t)c;
     a0 = (ones >> c) & 1ull;
   }
   if (q1 < (uint32_t)n) {
-    const uint32_t c = msb64(to & low_mask((uint32_t)S.cs[q1] + 1));
+    const uint32_t c = msb64(to & (~0ull >> (63u - S.cs[q1])));
     S.cs[q1] = (uint8_t)c;
     a1 = (ones >> c) & 1ull;
   }
@@ -632,13 +647,13 @@ static __device__ __forceinline__ bool w64_orbits(int n, int idx, int num_aut, u
     return true;
   }
   if (size <= 32) {
-    if ((mem >> v0) & 1ull) S.map[popc64(mem & low_mask(v0))] = (uint8_t)v0;
-    if ((mem >> v1) & 1ull) S.map[popc64(mem & low_mask(v1))] = (uint8_t)v1;
+    if (lane_bit0(mem)) S.map[popc64(mem & (bit64(v0) - 1))] = (uint8_t)v0;
+    if (lane_bit1(mem)) S.map[popc64(mem & (bit64(v1) - 1))] = (uint8_t)v1;
     __syncwarp();
     const bool in = lane < size;
     const uint32_t v = in ? S.map[lane] : 0u;
     uint32_t comp = lane;  // the least lane of the member's component
-    if (in && rv) comp = popc64(mem & low_mask(rep_of(v)));
+    if (in && rv) comp = popc64(mem & (bit64(rep_of(v)) - 1));
     for (;;) {
       while (sel) {
         uint32_t j[4], c[4];
@@ -651,7 +666,7 @@ static __device__ __forceinline__ bool w64_orbits(int n, int idx, int num_aut, u
           if (in) j[k] = image(i, v);
         }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) j[k] = in ? popc64(mem & low_mask(j[k])) : lane;
+        for (int k = 0; k < 4; ++k) j[k] = in ? popc64(mem & (bit64(j[k]) - 1)) : lane;
         for (int round = 0;; ++round) {
           bool d = false;
 #pragma unroll
