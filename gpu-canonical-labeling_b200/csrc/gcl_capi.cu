@@ -1,13 +1,14 @@
 // gcl_capi.cu -- the C ABI (include/gcl.h) and its host-side context.
 //
-// Dispatch: every batch first runs the warp-per-graph kernel for n <= 64
-// (canon_warp64.cuh).  Graphs it cannot finish are appended to device-side
-// lists and picked up by later launches on the same stream, so the batched
-// device path never synchronizes with the host:
+// Dispatch: up to 64 graphs of at most 64 vertices run on a block each with the
+// full ring (w64_few_kernel).  Every other batch first runs the warp-per-graph
+// kernel for n <= 64 (canon_warp64.cuh).  Graphs it cannot finish are appended
+// to device-side lists and picked up by later launches on the same stream, so
+// the batched device path never synchronizes with the host:
 //   * an automorphism ring that outgrew its per-slot capacity -> rerun with a
 //     workspace holding the full max_aut ring;
 //   * n > 64 -> the sparse warp-per-graph kernel (canon_sparse.cuh), first
-//     with a small pool of per-level orbit arrays and a short ring, then a
+//     with a small stack of orbit representatives and a short ring, then a
 //     rerun of the graphs that outgrew them with both at full size.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -143,7 +144,7 @@ __global__ void __cluster_dims__(kOrderBlocks, 1, 1) __launch_bounds__(kOrderThr
 
 constexpr int kSpSmemPerBlock = 200 * 1024;  // dynamic shared memory cap of one sparse block
 constexpr int kFirstSmem = 208 * 1024;  // ... and of the first path's block
-constexpr uint32_t kWidePool = 64;  // per-level orbit arrays of a wide-search warp
+constexpr uint32_t kWidePool = 64;  // orbit representatives of a wide-search warp, in target cells of n
 constexpr uint64_t kWideStoreBytes = 1ull << 30;  // automorphism store of a wide search
 constexpr uint64_t kWideStoreEntries = 1ull << 22;  // ... and at most this many entries
 constexpr uint32_t kWideFixCap = 4096;  // entries whose fix state a wide-search warp keeps
@@ -159,8 +160,8 @@ static uint32_t wide_store_cap(uint32_t n, int max_aut) {
       1, std::min<uint64_t>(std::min<uint64_t>((uint64_t)max_aut, kWideStoreBytes / per_aut),
                             kWideStoreEntries));
 }
-// Per-level orbit arrays and automorphism-ring entries of the sparse passes:
-// the first pass (n <= 4096 / larger), then a middle rerun of the graphs
+// Orbit representatives (in target cells of n vertices) and automorphism-ring
+// entries of the sparse passes: the first pass (n <= 4096 / larger), then a middle rerun of the graphs
 // that outgrew them, then a rerun with a full-size pool and ring.  Each
 // tier's slots are smaller than the next one's, so more warps fit in the
 // workspace budget.
@@ -285,10 +286,10 @@ constexpr int kW64QueueWait = 1 << 22;
 // last slot) and searches below it.  A warp never waits on a search, only on
 // a root refinement a running warp has claimed, so the launch needs no
 // co-residency.  Results equal w64_batch_kernel's.
-// Six resident blocks per SM (up to 80 registers per thread): measured on the
-// batched small-graph workload against 8 (64 registers, spills across the
-// inlined phases), 7, 5 and 4 blocks, six gave the shortest launch (0.327
-// against 0.372 ms at eight): its warps run the long searches faster.
+// Six resident blocks per SM (up to 80 registers per thread): on the batched
+// small-graph workload a call takes 255 us with six, 267 with seven (fewer
+// registers), 261 with five and 276 with four: fewer warps run the long
+// searches that end the launch faster, but leave issue slots empty before.
 __global__ void __launch_bounds__(kW64Threads, 6)
     w64_pipe_kernel(BatchArgs A, Deferred* D, int* large_list, int* overflow_list,
                     uint8_t* roots, int* ready) {
@@ -486,7 +487,7 @@ struct gcl_context {
   int wide_gate = 1;             // wide search's level gate: 1 on, 0 off, 2 automatic
   bool wide_share = false;       // wide search: busy warps hand subtrees to idle ones
   bool wide_count = false;       // wide search: the items kernel's counters (GCL_OPT_COUNTERS)
-  uint32_t wide_pool = kWidePool;  // wide search: per-level orbit arrays of a warp
+  uint32_t wide_pool = kWidePool;  // wide search: orbit representatives of a warp (cells of n)
   bool wide_probe = true;          // wide search: a level's first item runs before the rest
   uint64_t handoff_ns = 0;         // gcl_canon_batch: batch-warp budget before the wide search
   bool batch_split = false;        // gcl_canon_batch: large small-graph batches in two halves
@@ -802,7 +803,7 @@ int gcl_canon_batch_device_async(gcl_context* c, int count, const int64_t* d_vof
 
   if (max_n > kW64MaxN) {
     // graphs with n > 64: one sparse pass per size bucket, then a rerun of
-    // the graphs that outgrew the first passes' orbit pool or ring
+    // the graphs that outgrew the first passes' representatives or ring
     const uint64_t m2max = (uint64_t)std::max<int64_t>(max_m2, 1);
     const uint32_t cap1 = std::min<uint32_t>(maut, max_n <= 4096 ? kSpAutCap : kSpAutCapHuge);
     const uint32_t pool1 = max_n <= 4096 ? kSpPool : kSpPoolHuge;
@@ -1804,10 +1805,10 @@ int gcl_group_order(gcl_context* c, const int32_t* rowptr, const int32_t* col,
   const int max_aut = 0x7fffffff;
   int32_t status = 0;
   int64_t st[2] = {0, 0};
-  // A warp whose item goes deeper than its per-level orbit arrays reach
+  // A warp whose item needs more orbit representatives than it has room for
   // ends the search with kAutOverflow (the canonizing calls then rerun the
   // graph sequentially); the group order needs this search's automorphisms,
-  // so it reruns the wide search with an orbit array for every level.
+  // so it reruns the wide search with room for every level.
   for (int attempt = 0; attempt < 2; ++attempt) {
     const uint32_t saved_pool = c->wide_pool;
     if (attempt) c->wide_pool = (uint32_t)n + 2;
