@@ -189,9 +189,6 @@ __device__ __forceinline__ T ldx(const T* p) {
 __device__ __forceinline__ SpWarp& sp_w() { return g_sp[threadIdx.x >> 5]; }
 
 // ---- bitmaps with a summary word per 64 words ----------------------------
-__device__ __forceinline__ bool bm_test(const uint64_t* B, uint32_t p) {
-  return (B[p >> 6] >> (p & 63)) & 1ull;
-}
 // smallest set position >= p, or n
 __device__ __noinline__ uint32_t bm_next(const uint64_t* B, const uint64_t* Sm, uint32_t p, uint32_t n,
                             uint32_t nw, uint32_t nsw) {
