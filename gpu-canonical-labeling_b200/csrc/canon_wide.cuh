@@ -883,14 +883,15 @@ __device__ __noinline__ bool wide_try_donate(const WidePtrs& P, const WideArgs& 
   return false;
 }
 
-// Wait for a handed-over subtree.  1: its slot in *slot (the warp now counts
-// as busy); 0: the search is over (no warp busy and the queue empty); else a
-// status.  The busy count is read before the queue, so a subtree published by
-// a warp that then finished is seen.
+// Wait for a handed-over subtree.  kOk: its slot in *slot (the warp now counts
+// as busy), or kNone when the search is over (no warp busy and the queue empty);
+// else the status that ends the search (any of them: kAutOverflow is 1).  The busy
+// count is read before the queue, so a subtree published by a warp that then
+// finished is seen.
 __device__ __noinline__ int32_t wide_take_gift(const WidePtrs& P, uint64_t deadline,
                                                uint32_t* slot) {
   WideHdr* H = P.H;
-  int32_t st = 0;
+  int32_t st = kOk;
   uint32_t got = kNone;
   if (lane_id() == 0) {
     atomicAdd(&H->hungry, 1u);
@@ -912,7 +913,7 @@ __device__ __noinline__ int32_t wide_take_gift(const WidePtrs& P, uint64_t deadl
         }
         continue;
       }
-      if (busy == 0) break;  // st = 0: nothing left anywhere
+      if (busy == 0) break;  // nothing left anywhere
       if (i >= kWideGateSpinLimit || (deadline && (i & 15u) == 0 && global_ns() > deadline)) {
         st = kTimeout;
         break;
@@ -929,7 +930,6 @@ __device__ __noinline__ int32_t wide_take_gift(const WidePtrs& P, uint64_t deadl
         ++j;
       }
       if (j >= kWideSpinLimit) st = kTimeout;
-      else st = 1;
       __threadfence();
     }
     atomicSub(&H->hungry, 1u);
@@ -1130,11 +1130,11 @@ __global__ void __launch_bounds__(kSpThreads) wide_items_kernel(WideArgs A) {
         unsigned long long tc = cnt.now();
         const int32_t gs = wide_take_gift(P, deadline, &slot);
         cnt.add(kCntGiftWaitCycles, cnt.now() - tc);
-        if (gs == 0) break;
-        if (gs != 1) {
+        if (gs != kOk) {
           status = gs;
           break;
         }
+        if (slot == kNone) break;
         gift = true;
         cnt.add(kCntGiftsTaken, 1);
         tc = cnt.now();
