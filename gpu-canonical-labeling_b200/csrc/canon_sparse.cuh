@@ -1476,6 +1476,34 @@ __device__ __forceinline__ bool sp_dsu_apply(const uint16_t* pm, const T* member
   }
 }
 
+// Join the trees of a and b in the min-root union-find d, which other lanes join
+// trees of at the same time: the larger root is hooked only while it still is one,
+// so nothing is lost and no second pass over the edges is needed.  A failed hook
+// means that another lane's took a root away; false past n of them.  A walk
+// points what it passes at its grandparent: only roots are hooked, so that store
+// meets no hook.
+__device__ __forceinline__ bool sp_unite(volatile uint32_t* d, uint32_t a, uint32_t b,
+                                         uint32_t n) {
+  auto root = [&](uint32_t x) {
+    uint32_t p = d[x];
+    for (uint32_t step = 0; p < x && step <= n; ++step) {
+      const uint32_t g = d[p];
+      if (g < p) d[x] = g;
+      x = p;
+      p = g;
+    }
+    return x;
+  };
+  for (uint32_t step = 0; step <= n; ++step) {
+    a = root(a);
+    b = root(b);
+    if (a == b) return true;
+    const uint32_t hi = max(a, b);
+    if (atomicCAS((uint32_t*)d + hi, hi, min(a, b)) == hi) return true;
+  }
+  return false;
+}
+
 // The orbits of a target cell of at most 32 vertices, a lane per vertex: a
 // component is named by its least lane.
 struct SpCellOrbits {
@@ -1535,6 +1563,11 @@ __device__ __forceinline__ void sp_cell_merge(SpCellOrbits& o, const uint32_t (&
 // entries), 14,000 now: the search 790 ms then and 500 now with its state in
 // device memory, that of a tree of 8,192 vertices 25.2 s and 11.4.
 //
+// Larger cells: the members that a word's entries move are listed and joined a
+// lane each.  An entry of a symmetric group moves two or a few, so joining entry
+// after entry kept two lanes busy: a star of 100 leaves took 400,000 cycles a node
+// (965 ms in the wide search, 1,111 in the batched one), 69,000 now (185 and 194 ms).
+//
 // Returns kOk, kAutOverflow (no room for the representatives) or kInternal.
 template <bool kCg = false>
 __device__ __noinline__ int32_t sp_orbits(int idx, int num_aut, uint32_t seqlen) {
@@ -1547,7 +1580,7 @@ __device__ __noinline__ int32_t sp_orbits(int idx, int num_aut, uint32_t seqlen)
   const bool small = t.len <= 32;
   volatile uint32_t* dsu = W.dsu;
   const uint16_t* mem = W.elem + t.first;
-  bool any = false;
+  bool any = false, begun = false;
   SpCellOrbits o{kNone, lane};
   // the cell's orbits so far
   auto begin = [&] {
@@ -1605,20 +1638,58 @@ __device__ __noinline__ int32_t sp_orbits(int idx, int num_aut, uint32_t seqlen)
       }
       return kOk;
     }
-    for (; m; m &= m - 1) {
-      const uint16_t* pm = W.auts + (uint64_t)(base + (uint32_t)__ffs((int)m) - 1) * W.stride;
-      bool out = false, moves = false;
-      for (uint32_t i = lane; i < t.len; i += 32) {
-        const uint32_t v = mem[i], img = ldx<kCg>(pm + v), q = W.pos[img];
-        moves |= img != v;
-        out |= q < t.first || q >= t.first + t.len;
+    // larger cells: a lane takes every 32nd member through all the entries, and
+    // the members they move are listed and joined 32 at a time
+    if (!begun) begin();
+    begun = true;
+    uint32_t* const edge = (uint32_t*)W.list;  // 128 of {vertex, image << 16}
+    uint32_t edges = 0;
+    bool out = false, moves = false;
+    auto join = [&] {
+      __syncwarp();
+      for (uint32_t x = lane; x < edges; x += 32)
+        out |= !sp_unite(dsu, edge[x] & 0xffffu, edge[x] >> 16, n);
+      __syncwarp();
+      edges = 0;
+    };
+    for (uint32_t i0 = 0; i0 < t.len; i0 += 32) {
+      const bool in = i0 + lane < t.len;
+      const uint32_t v = in ? mem[i0 + lane] : 0u;
+      for (uint32_t r = m; r;) {
+        uint32_t img[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          img[k] = v;
+          if (!r) continue;
+          const uint16_t* pm = W.auts + (uint64_t)(base + (uint32_t)__ffs((int)r) - 1) * W.stride;
+          r &= r - 1;
+          if (in) img[k] = ldx<kCg>(pm + v);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          bool mv = img[k] != v;
+          if (mv && (uint32_t)W.pos[img[k]] - t.first >= t.len) {
+            out = true;
+            mv = false;
+          }
+          const uint32_t b = __ballot_sync(GCL_FULL, mv);
+          if (!b) continue;
+          moves = true;
+          if (edges + (uint32_t)__popc(b) > 128) join();
+          if (mv) edge[edges + (uint32_t)__popc(b & lanemask_lt())] = v | (img[k] << 16);
+          edges += (uint32_t)__popc(b);
+        }
       }
-      if (__any_sync(GCL_FULL, out)) return kInternal;
-      if (!__any_sync(GCL_FULL, moves)) continue;
-      if (!any) begin();
-      any = true;
-      if (!sp_dsu_apply<kCg>(pm, mem, t.len, n)) return kInternal;
     }
+    join();
+    if (__any_sync(GCL_FULL, out)) return kInternal;
+    if (!moves) return kOk;
+    any = true;
+    for (uint32_t i = lane; i < t.len; i += 32) {  // every member to its root
+      const uint32_t v = mem[i];
+      atomicMin(W.dsu + v, sp_find(dsu, v, n));
+    }
+    __syncwarp();
     return kOk;
   };
   if constexpr (kCg) {

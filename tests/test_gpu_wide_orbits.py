@@ -47,3 +47,27 @@ def test_idle_entries_cost_a_test(pkg, G):
     assert c["orbit_cycles"] < 6 * c["refine_cycles"], c
     batch = pkg.canon_batch([g], max_aut=10000, ctx=pkg.Context(0), dense=False, rows=True)
     assert np.array_equal(rows.ravel(), batch.rows[: rows.size])
+
+
+@pytest.mark.parametrize("leaves", [[2, 32, 3], [33, 2, 2], [64, 2, 65], [3, 96, 40, 2], [129, 2]])
+def test_cells_in_a_batch(pkg, G, oracle_mod, leaves):
+    # ... and the ring's search, also where the ring wraps
+    rng = np.random.default_rng(len(leaves))
+    gs = [_broom(G, leaves, rng) for _ in range(2)] + [G.random_relabel(G.torus(9, 8), rng)]
+    for max_aut in (10000, 20):
+        res = pkg.canon_batch(gs, max_aut=max_aut, rows=True)
+        out, ooff, na, nd = oracle_mod.canon_batch(res.arena, max_aut=max_aut)
+        assert (res.status == 0).all()
+        assert np.array_equal(res.dense[: ooff[-1]], out[: ooff[-1]])
+        assert np.array_equal(res.stats[:, 0], na) and np.array_equal(res.stats[:, 1], nd)
+
+
+def test_large_cells_join_their_members_together(pkg, G):
+    """A star: every stored automorphism swaps two of up to 100 members."""
+    g = G.from_edges(101, np.array([(0, i) for i in range(1, 101)]))
+    ctx = pkg.Context(0)
+    ctx.set_option(pkg.api.GCL_OPT_COUNTERS, 1)
+    pkg.api.canon_rows(g, 10000, ctx)
+    c = ctx.wide_counters()
+    assert c["auts_first"] == 99, c
+    assert c["orbit_cycles"] < 160000 * c["nodes"], c
