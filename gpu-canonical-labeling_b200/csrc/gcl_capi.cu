@@ -504,6 +504,7 @@ struct gcl_context {
   // pinned host memory and its device twin for small calls' inputs and outputs
   void* stage = nullptr;
   size_t stage_cap = 0;
+  int stage_short = 0;  // calls since it was allocated that found it too small
   DevBuf stage_dev;
   bool counted = false;          // the last wide search was counted
   // launch shape per size bucket (gcl_autotune / gcl_set_tuning): 0 / -1 = default
@@ -1103,11 +1104,17 @@ T* mapped_alias(const gcl_context* c, const T* p, size_t count) {
 // The inputs and outputs of a call from pageable host memory, packed into pinned
 // memory of the context: one copy in, one copy out.  Every pageable copy costs
 // the caller several us whatever its size, and a batched call makes up to 7 in
-// and 5 out: a call on one 20-vertex graph took 150 us with them and takes 105,
-// one on 4,000 small graphs (3.8 MB) 930 to 1,000 us and 750 to 770.  Larger
-// calls than kStageBytes are copied directly (the pinned memory stays with the
-// context), and so are arrays in pinned memory, which the DMA reads in place.
-constexpr size_t kStageBytes = 16u << 20;
+// and 5 out: a call on one 24-vertex graph takes 90 us with them and 55 packed,
+// one on 4,000 small graphs (3.8 MB) 0.86 ms and 0.68, on 16,000 (15 MB) 2.5 and
+// 2.28.  Larger calls than kStageBytes are copied directly (the pinned memory stays
+// with the context), and so are arrays in pinned memory, which the DMA reads in
+// place.
+//
+// Pinning takes 2.6 ms up to 1 MB and 10 ms for 16 MB, which a context made for
+// one call or one pair does not get back (its first call took 2.7 ms instead of
+// 0.17): the memory is allocated, and grown, at the third call that wants more.
+constexpr size_t kStageBytes = 16u << 20, kStageMin = 1u << 20;
+constexpr int kStageShort = 2;
 
 bool is_pinned(const void* p) {
   if (!p) return false;
@@ -1129,12 +1136,17 @@ class Staging {
   bool open() {
     if (size_ > kStageBytes) return false;
     if (c_->stage_cap < size_) {
-      const size_t want = std::min(std::max<size_t>(size_ * 2, 4096), kStageBytes);
+      if (c_->stage_short < kStageShort) {
+        ++c_->stage_short;
+        return false;
+      }
+      const size_t want = std::min(std::max(size_ * 2, kStageMin), kStageBytes);
       void* p = nullptr;
       if (pinned_alloc(&p, want) != cudaSuccess) return false;
       if (c_->stage) cudaFreeHost(c_->stage);
       c_->stage = p;
       c_->stage_cap = want;
+      c_->stage_short = 0;
     }
     return c_->stage_dev.ensure(c_->stage_cap) == cudaSuccess;
   }
