@@ -67,7 +67,7 @@ struct WideHdr {
   unsigned long long nodes;
   unsigned long long t0;  // start time (globaltimer ns)
   // how long a level's other items wait for its first item (the probe)
-  // before they start anyway: three times the first path's duration
+  // before they start anyway: twice the first path's duration
   unsigned long long probe_ns;
   // opt-in counters of the items kernel (GCL_OPT_COUNTERS; zeroed by the
   // host before a counted search, untouched otherwise)
@@ -395,7 +395,9 @@ __global__ void __launch_bounds__(kSpHelpThreads) wide_first_kernel(WideArgs A) 
     // automatic gate: off when the levels hold fewer than 4 items each on
     // average (trees), where it would run the items one after another
     H->gate = A.gate == 2 ? (run >= 4u * (D - 1u) ? 1u : 0u) : (A.gate != 0 ? 1u : 0u);
-    H->probe_ns = max(3ull * (global_ns() - H->t0), 20000ull);
+    // (three times measured the same on tori up to 140 x 140, unions, cubic graphs
+    // and trees, with the items' state in shared and in device memory)
+    H->probe_ns = max(2ull * (global_ns() - H->t0), 20000ull);
     __threadfence();
     H->nitems = run;
   }
@@ -1182,7 +1184,7 @@ __global__ void __launch_bounds__(kSpThreads) wide_items_kernel(WideArgs A) {
         const unsigned long long tc = cnt.now();
         int32_t gs = wide_gate(H, P.cum[lo], deadline);
         // with the probe, the level's other items also wait for its first
-        // item, up to three times the first path's duration: the automorphisms
+        // item, up to twice the first path's duration: the automorphisms
         // that one finds prune them (it is done when `done` passes the
         // deeper levels' items, since no other item of the level can finish
         // before it)
