@@ -963,13 +963,15 @@ int gcl_canon_wide_device_async(gcl_context* c, const int32_t* d_rowptr, const i
   const WideLayout WL = wide_layout(un, m2, cap, qcap);
   const uint32_t pool = std::min<uint32_t>(c->wide_pool, un + 2);
   const SpLayout Lo = sp_layout(un, m2, pool, 0, std::min<uint32_t>(cap, kWideFixCap));
-  // The items kernel's launch shapes.  With the per-step arrays in shared
-  // memory a warp runs about 4.8 times as fast as from device memory (a
-  // 4096-vertex cubic graph: 4 such warps per SM took 96 ms for 4,095 items, 28
-  // warps from device memory 66 ms), so blocks take as many warps, up to 4, as
-  // fit there.  Where fewer than 4 fit (n above about 7,500) an SM may run
-  // several times as many warps from device memory: both shapes are launched,
-  // and the number of items -- known on the device only -- picks one.
+  // The items kernel's launch shapes.  A warp with its per-step arrays in shared
+  // memory is faster than one from device memory, of which an SM holds 12 (its
+  // registers; a build for 16 was 1 to 3% slower in shared memory and gained
+  // nothing outside).  So blocks take as many warps, up to 4, as fit there: 8 per SM
+  // up to about 4,200 vertices (a cubic graph of 4,096: 53 ms, 68 from device
+  // memory), then 4, where both take the same time (cubic graphs of 5,000 / 6,000 /
+  // 7,800 vertices: 104 / 153 / 302 ms and 102 / 148 / 305).  Where fewer than 4 fit
+  // in a block (n above about 7,800) both shapes are launched, and the number of
+  // items -- known on the device only -- picks one (kItemsPerWarp).
   struct Shape {
     int warps_per_block, grid;
     uint64_t smem_per_warp;
@@ -1031,8 +1033,14 @@ int gcl_canon_wide_device_async(gcl_context* c, const int32_t* d_rowptr, const i
                             sizeof(((WideHdr*)nullptr)->cnt), s));
   wide_first_kernel<<<1, kSpHelpThreads, (size_t)WA.smem_first, s>>>(WA);
   GCL_TRY(cudaGetLastError());
-  // up to 4 items per warp the shared-memory shape wins (4.8 times the speed)
-  const uint32_t split = 4u * (uint32_t)(shape[0].grid * shape[0].warps_per_block);
+  // Items per warp up to which the shared-memory shape takes them.  A cubic
+  // component beside a rigid rest, 9,000 / 12,000 / 20,000 vertices (3 / 2 / 1 such
+  // warps per SM), from shared and from device memory: 4 items per warp 55 / 67 / 83
+  // and 63 / 64 / 80 ms, 8: 93 / 77 / 139 and 97 / 110 / 144, 16: 297 / 206 / 196 and
+  // 264 / 164 / 192; a cubic graph (20 / 40 / 135): 507 / 1,321 / 8,773 and 430 / 931 /
+  // 3,850.
+  constexpr uint32_t kItemsPerWarp = 8;
+  const uint32_t split = kItemsPerWarp * (uint32_t)(shape[0].grid * shape[0].warps_per_block);
   for (int i = 0; i < shapes; ++i) {
     WA.smem_per_warp = shape[i].smem_per_warp;
     WA.items_min = i == 0 ? 1 : split + 1;
