@@ -15,7 +15,6 @@
 // stays usable.  Unset, or not a positive integer: no effect.
 #pragma once
 #include <cuda_runtime.h>
-#include <sys/mman.h>
 
 #include <atomic>
 #include <cstdint>
@@ -109,37 +108,6 @@ inline cudaError_t pinned_alloc(void** p, size_t bytes) {
     (void)cudaGetLastError();
   }
   return e;
-}
-
-// Pinned host memory of a context: one 2 MB page, where the system gives such
-// pages, registered (0.6 ms where cudaHostAlloc takes 1 to 3 for any size up to 1 MB),
-// or `bytes` above that from cudaHostAlloc (5 to 10 ms for 8 and 16 MB; registered
-// pages take 2, but calls of 4 to 10 MB through them took 4% longer).  *p is null on
-// failure.
-constexpr size_t kPinnedPage = 2u << 20;
-inline cudaError_t pinned_region_alloc(void** p, size_t bytes) {
-  if (bytes > kPinnedPage) return pinned_alloc(p, bytes);
-  *p = nullptr;
-  if (alloc_fault_hit()) return cudaErrorMemoryAllocation;
-  void* q = std::aligned_alloc(kPinnedPage, kPinnedPage);
-  if (!q) return cudaErrorMemoryAllocation;
-  (void)madvise(q, kPinnedPage, MADV_HUGEPAGE);
-  const cudaError_t e = cudaHostRegister(q, kPinnedPage, cudaHostRegisterDefault);
-  if (e != cudaSuccess) {
-    (void)cudaGetLastError();
-    std::free(q);
-    return e;
-  }
-  *p = q;
-  return cudaSuccess;
-}
-inline void pinned_region_free(void* p, size_t bytes) {
-  if (bytes > kPinnedPage) {
-    cudaFreeHost(p);
-    return;
-  }
-  cudaHostUnregister(p);
-  std::free(p);
 }
 
 // pinned host allocation mapped into the device's address space

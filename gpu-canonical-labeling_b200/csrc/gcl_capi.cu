@@ -665,7 +665,7 @@ int gcl_destroy(gcl_context* c) {
     cudaStreamDestroy(c->stream);
   }
   for (const auto& h : c->mapped) cudaFreeHost(h.p);
-  if (c->stage) pinned_region_free(c->stage, c->stage_cap);
+  if (c->stage) cudaFreeHost(c->stage);
   delete c;
   return GCL_OK;
 }
@@ -1118,12 +1118,11 @@ T* mapped_alias(const gcl_context* c, const T* p, size_t count) {
 // with the context), and so are arrays in pinned memory, which the DMA reads in
 // place.
 //
-// Pinning 2 MB takes 0.6 ms, 16 MB 10 ms, which a context made for one call does
-// not get back (its first call took 2.7 ms instead of 0.17 on a 24-vertex graph and
-// 12 instead of 1.7 on 10,000 graphs): the memory is allocated, and grown, at the
-// second call that wants more.
-constexpr size_t kStageBytes = 16u << 20;
-constexpr int kStageShort = 1;
+// Pinning takes 2.6 ms up to 1 MB and 10 ms for 16 MB, which a context made for
+// one call or one pair does not get back (its first call took 2.7 ms instead of
+// 0.17): the memory is allocated, and grown, at the third call that wants more.
+constexpr size_t kStageBytes = 16u << 20, kStageMin = 1u << 20;
+constexpr int kStageShort = 2;
 
 bool is_pinned(const void* p) {
   if (!p) return false;
@@ -1149,10 +1148,10 @@ class Staging {
         ++c_->stage_short;
         return false;
       }
-      const size_t want = std::min(std::max(size_ * 2, kPinnedPage), kStageBytes);
+      const size_t want = std::min(std::max(size_ * 2, kStageMin), kStageBytes);
       void* p = nullptr;
-      if (pinned_region_alloc(&p, want) != cudaSuccess) return false;
-      if (c_->stage) pinned_region_free(c_->stage, c_->stage_cap);
+      if (pinned_alloc(&p, want) != cudaSuccess) return false;
+      if (c_->stage) cudaFreeHost(c_->stage);
       c_->stage = p;
       c_->stage_cap = want;
       c_->stage_short = 0;

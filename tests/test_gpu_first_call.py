@@ -1,7 +1,7 @@
-"""A context made for one call: no memory is pinned for it.  With cudaHostAlloc in
-its first call that takes 2.7 ms, without 0.17 to 0.25 on a B200; the line lies at the
-geometric mean.  The second call registers one page (0.7 to 0.8 ms; the line twice
-that).  Later calls, through pinned memory, give the same results."""
+"""A context made for one call or one pair: no memory is pinned for it.  With
+1 MB pinned its first call takes 2.7 ms, without 0.17 to 0.25 on a B200; the line
+lies at the geometric mean.  Later calls, through pinned memory, give the same
+results."""
 import statistics
 import time
 
@@ -26,8 +26,8 @@ def test_first_calls_are_cheap(pkg, G, n):
     g = G.tree_plus_edges(n, np.random.default_rng(n))
     _first_calls(pkg, g, 4)  # the process's first use of the device
     runs = [_first_calls(pkg, g, 2)[0] for _ in range(9)]
-    assert statistics.median(r[0] for r in runs) < 0.8e-3
-    assert statistics.median(r[1] for r in runs) < 1.6e-3
+    for k in range(2):
+        assert statistics.median(r[k] for r in runs) < 0.8e-3
 
 
 @pytest.mark.parametrize("sizes", [[1] * 5, [3, 3, 3, 3000, 3, 3000, 3000, 3, 3000]])
