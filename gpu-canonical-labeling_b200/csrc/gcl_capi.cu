@@ -237,8 +237,8 @@ __global__ void __launch_bounds__(kW64Threads, 8)
 // A few graphs of up to 64 vertices, each on a block of one warp with the full
 // max_aut ring: nothing to order, hand over or rerun, so one launch does what
 // takes five steps of the stream (two clears, the ordering, the pipelined
-// launch and the rerun): a call on one 24-vertex graph took 110 us with them and
-// takes 76 us now.
+// launch and the rerun).  It took a call on one 24-vertex graph from 110 to 76 us;
+// with its arrays packed (Staging) that call takes 55.
 constexpr int kFewGraphs = 64;
 __global__ void __launch_bounds__(32) w64_few_kernel(BatchArgs A) {
   const int g = (int)blockIdx.x;
@@ -1118,11 +1118,12 @@ T* mapped_alias(const gcl_context* c, const T* p, size_t count) {
 // with the context), and so are arrays in pinned memory, which the DMA reads in
 // place.
 //
-// Pinning takes 2.6 ms up to 1 MB and 10 ms for 16 MB, which a context made for
-// one call or one pair does not get back (its first call took 2.7 ms instead of
-// 0.17): the memory is allocated, and grown, at the third call that wants more.
+// Pinning takes 1 to 3 ms up to 1 MB and 10 ms for 16 MB, which a context made for
+// one call does not get back (its first call took 2.7 ms instead of 0.17 on a
+// 24-vertex graph, 12 instead of 1.7 on 10,000 graphs): the memory is allocated, and
+// grown, at the second call that wants more.
 constexpr size_t kStageBytes = 16u << 20, kStageMin = 1u << 20;
-constexpr int kStageShort = 2;
+constexpr int kStageShort = 1;
 
 bool is_pinned(const void* p) {
   if (!p) return false;
