@@ -29,10 +29,10 @@
 // A refinement step is a chain of dependent loads, so what bounds the kernel is
 // the latency of one warp and, for the many-warp search, how many warps' state
 // fits in shared memory.  Positions and vertices are 16-bit (n <= 65536), and a
-// cell's level is not kept (see the log of cell starts): 6.4 bytes per vertex
-// where 32-bit arrays with in_level took 16.4.  With both changes a batch of
-// mixed graphs up to 256 vertices took 430 instead of 478 ms, a 4096-vertex
-// cubic graph 85 instead of 91 ms (12 instead of 3 warps of shared memory).
+// cell's level is not kept (see the log of cell starts): 6.5 bytes per vertex
+// where 32-bit arrays with in_level took 16.4, so a graph of 4,096 vertices fits an
+// SM's shared memory 8 times instead of 3.  When they were made, both changes took
+// a batch of mixed graphs up to 256 vertices from 478 to 430 ms.
 #pragma once
 #include <cstdint>
 
@@ -846,9 +846,9 @@ __device__ __noinline__ SpStep sp_refine_general(uint32_t s, uint32_t e, uint32_
 // that was active gets its new fragments, one that was not all but its first
 // largest.  Singleton neighbours end a step early.  With one lane writing the
 // splits one after the other a singleton step took 1,900-2,500 cycles and a
-// non-singleton one 6,000 beside its hash; a mixed batch up to 256 vertices
-// took 432 ms then and 252 ms now, four copies of a 4-regular graph on 64
-// vertices 219 ms and 133 ms.
+// non-singleton one 6,000 beside its hash; the change took a mixed batch up to 256
+// vertices from 432 to 252 ms and four copies of a 4-regular graph on 64
+// vertices from 219 to 133.
 // ---------------------------------------------------------------------------
 template <bool kS>
 __device__ __noinline__ int sp_refine_t() {

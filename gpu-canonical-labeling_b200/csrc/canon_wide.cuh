@@ -244,7 +244,7 @@ __device__ __forceinline__ void wide_fail(WideHdr* H, int32_t status) {
 //    Bound by that one warp's chain of steps.  With one warp alone and the
 //    state in device memory a 256-vertex random graph took 550-690 us and one
 //    of 20,000 vertices 91 ms, of which the input check 8 ms and the leaf 5 ms;
-//    now about 120 us and 50 ms.
+//    now 127 us and 32 ms.
 // ---------------------------------------------------------------------------
 struct FirstPath {
   int32_t status;

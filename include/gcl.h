@@ -115,7 +115,7 @@ void* gcl_stream(gcl_context* ctx);
  *   queue (up to 65,536 entries, 256 MiB); the receiver rebuilds the parent
  *   from the first leaf.  Same canonical form.  For trees whose work sits in
  *   a few siblings (unions of identical components: 6 copies of a random
- *   4-regular graph on 64 vertices in about 0.8 s on a B200, where the
+ *   4-regular graph on 64 vertices in about 0.4 s on a B200, where the
  *   reference's sequential path takes 20.6 s on one core).  Default 0.
  * GCL_OPT_WIDE_PROBE: 1 (default) makes, under the level gate, the first
  *   item of each level run alone before the rest of that level starts, so
